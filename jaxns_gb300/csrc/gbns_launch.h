@@ -22,6 +22,9 @@ cudaError_t launch_slice_warp(const gbns_batch &b, const float *Lstar, const uin
 // [ib, ie) of a family and DMAX; taken tells whether it launched.
 cudaError_t launch_slice_spec(const gbns_batch &b, int family, int dmax, int ib, int ie, const float *Lstar,
                               const uint32_t *keys, cudaStream_t stream, bool &taken);
+// The same for the warp-cooperative correlated-Gaussian bucket of a DMAX (gbns_slice_spec_mvn.cu).
+cudaError_t launch_slice_spec_mvn(const gbns_batch &b, int dmax, int ib, int ie, const float *Lstar, const uint32_t *keys,
+                                  cudaStream_t stream, bool &taken);
 cudaError_t launch_init(const gbns_batch &b, long long total_points, cudaStream_t stream);
 cudaError_t launch_merge(const gbns_batch &b, cudaStream_t stream);
 cudaError_t launch_finalize(const gbns_batch &b, cudaStream_t stream);

@@ -19,22 +19,18 @@
 // steps + one likelihood + ballot); the evaluations beyond the accepted one are spare work of an
 // otherwise idle GPU, which is why the launcher takes this kernel only below a chain count.
 #include "gbns_launch.h"
-#include "gbns_slice.cuh"
+#include "gbns_spec.cuh"
 
 namespace gbns {
 
-constexpr int SPEC_E = 16;    // uniforms made ahead per slice (more are derived on demand)
-constexpr int SPEC_E0 = 8;    // those of the first block, which the chain waits for
 constexpr int SPEC_TEAMS = 2; // teams of one consumer and two producer warps per CTA
 
-// One block of 32 (chain, slice) rows: row = group * slices per block + slice of the block.
+// One block of rows: row = group * slices per block + slice of the block.
 template <int DMAX>
 struct SpecBlock {
   float d[32][DMAX + 4];   // direction (row stride keeps float4 reads conflict-free)
   float rc[32][DMAX + 4];  // 1 / direction
-  float u[SPEC_E][32];     // uniform of proposal e
-  uint2 ck[32];            // the carry key after the last of them
-  float alpha[32];         // the slice's shrink factor (1 without midpoint shrink)
+  SpecDraws r;
 };
 
 template <int DMAX>
@@ -45,43 +41,13 @@ struct SpecTeam {
 
 __device__ __forceinline__ void team_barrier(int id) { asm volatile("bar.sync %0, 96;" ::"r"(id) : "memory"); }
 
-// Number of live points above the contour; the live set is sorted ascending.  One warp.  The
-// sampler's own contour is the log L of point s - 1, so the search starts at point s and ends
-// with the first 32 unless the likelihood has plateaus there; an explicit contour (s = 0) takes
-// 32 probes per step.
-__device__ __forceinline__ int warp_count_above(const float *__restrict__ L, int n, int s, float Lstar) {
-  const int lane = threadIdx.x & 31;
-  int lo = s, hi = n;
-  while (lo < hi) {
-    const int step = s > 0 ? 1 : (hi - lo + 31) >> 5;
-    const int p = lo + lane * step;
-    const bool below = p < hi && !(L[p] > Lstar);
-    const int cnt = __popc(__ballot_sync(0xffffffffu, below));  // a prefix of the probes
-    if (cnt == 0) break;
-    if (s > 0) {
-      lo += cnt;
-      if (cnt < 32) break;
-    } else {
-      hi = min(hi, lo + cnt * step);
-      lo = lo + (cnt - 1) * step + 1;
-    }
-  }
-  return n - lo;
-}
-
-// What a lane needs to make the rows of its (chain, slice-of-block) column.
-struct SpecKeys {
-  Key slices, dir0;  // the chain's slice keys root and first direction key
-  bool valid;
-};
-
 // Directions (and reciprocals) of the rows in `rows`: D normals per row, flattened over the
 // warp, then normalised one row per lane in dimension order.
 template <int DMAX>
-__device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, const SpecKeys &k, int j, int S, int D,
+__device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, const SpecKeys &k, int j, int end, int D,
                                                 uint32_t dmagic, uint32_t rows) {
   const int lane = threadIdx.x & 31;
-  const bool valid = k.valid && j < S && ((rows >> lane) & 1u);
+  const bool valid = k.valid && j < end && ((rows >> lane) & 1u);
   if (D == 1) {
     if (valid) {
       B.d[lane][0] = 1.0f;
@@ -125,31 +91,6 @@ __device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, 
         B.d[lane][q] = v;
         B.rc[lane][q] = 1.0f / v;
       }
-  }
-  __syncwarp();
-}
-
-// The first E uniforms of each row's slice and its shrink factor: the first pick's (t key
-// fold(kj, 2)), then those of the shrink steps along the carry-key chain.  The three threefry
-// blocks of a trip (this proposal's bits, the next t key, the next carry key) are independent.
-template <int DMAX>
-__device__ __forceinline__ void spec_uniforms(SpecBlock<DMAX> &B, const SpecKeys &k, int j, int S, int E, bool midpoint) {
-  const int lane = threadIdx.x & 31;
-  if (k.valid && j < S) {
-    const Key kj = fold(k.slices, (uint32_t)j);
-    Key ck = fold(kj, 0u), tk = fold(kj, 2u);
-    B.alpha[lane] = midpoint ? slice_alpha(j, S) : 1.0f;
-    for (int e = 0; e < E; ++e) {
-      uint32_t b0, b1;
-      Key tn, cn;
-      threefry2x32(tk.k0, tk.k1, 0u, 0u, b0, b1);
-      threefry2x32(ck.k0, ck.k1, 0u, 1u, tn.k0, tn.k1);
-      threefry2x32(ck.k0, ck.k1, 0u, 0u, cn.k0, cn.k1);
-      B.u[e][lane] = uniform01(((uint64_t)b0 << 32) | (uint64_t)b1);
-      if (e == E - 1) B.ck[lane] = make_uint2(ck.k0, ck.k1);  // the carry that proposal E starts from
-      tk = tn;
-      ck = cn;
-    }
   }
   __syncwarp();
 }
@@ -199,9 +140,11 @@ template <int DMAX, int FAM, int G, int SUB>
 __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
     k_slice_spec(gbns_batch b, int item_begin, const float *__restrict__ Lstar_in,
                  const uint32_t *__restrict__ keys_in) {
+  static_assert(G <= SPEC_E && SPEC_E % G == 0, "a round's uniforms are all prepared or all derived on demand");
   constexpr int GL = G * SUB;              // lanes per chain
   constexpr int NG = 32 / GL;              // chains per consumer warp
   constexpr int SB = 32 / NG;              // slices per block
+  constexpr int SB0 = SB >= 16 ? SB / 4 : (SB < 4 ? SB : 4);  // slices in the first block
   constexpr int CPC = SPEC_TEAMS * NG;     // chains per CTA
   constexpr int OWN = (DMAX + GL - 1) / GL;  // dimensions per lane in the chord bounds
   __shared__ RunSmem<DMAX, FAM> P;
@@ -259,7 +202,7 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
   SpecTeam<DMAX> &W = reinterpret_cast<SpecTeam<DMAX> *>(spec_dyn)[team];
   const int bar = 1 + team;
   const int g = lane / GL, li = lane % GL, g0 = g * GL;
-  const int nb = (S + SB - 1) / SB;
+  const int nb = spec_blocks(S, SB, SB0);
   constexpr uint32_t kHalf = 0x55555555u;  // the consumer's share of the first block's directions
 
   for (int cs = (int)blockIdx.y * CPC + team * NG; cs < c_count; cs += (int)gridDim.y * CPC) {
@@ -277,8 +220,9 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
       for (int bi = 0; bi <= nb; ++bi) {
         if (bi < nb) {
           SpecBlock<DMAX> &B = W.blk[bi & 1];
-          if (role == 1) spec_directions(B, W.key[1], sk, bi * SB + li, S, D, dmagic, bi == 0 ? ~kHalf : 0xffffffffu);
-          else spec_uniforms(B, sk, bi * SB + li, S, bi == 0 ? SPEC_E0 : SPEC_E, midpoint);
+          const int j = spec_block_begin(bi, SB, SB0) + li, end = bi == 0 ? min(S, SB0) : S;
+          if (role == 1) spec_directions(B, W.key[1], sk, j, end, D, dmagic, bi == 0 ? ~kHalf : 0xffffffffu);
+          else spec_uniforms(B.r, sk, j, end, S, bi == 0 ? spec_first(G) : SPEC_E, midpoint);
         }
         team_barrier(bar);
       }
@@ -302,7 +246,7 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
       u_own[k] = have && q < D ? liveU[(size_t)idx * D + q] : 0.0f;
     }
     if (have) logL0 = liveL[idx];
-    spec_directions(W.blk[0], W.key[0], sk, li, S, D, dmagic, kHalf);
+    spec_directions(W.blk[0], W.key[0], sk, li, min(S, SB0), D, dmagic, kHalf);
     team_barrier(bar);
 
     int j = 0, total = 0;
@@ -310,15 +254,16 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
     float left = 0.f, right = 0.f, t = 0.f, alpha = 1.0f;
     for (int bi = 0; bi < nb; ++bi) {
       SpecBlock<DMAX> &B = W.blk[bi & 1];
-      const int made = bi == 0 ? SPEC_E0 : SPEC_E;
-      const int j_end = have ? min(S, (bi + 1) * SB) : 0;
+      const int made = bi == 0 ? spec_first(G) : SPEC_E;
+      const int j_begin = spec_block_begin(bi, SB, SB0);
+      const int j_end = have ? min(S, spec_block_begin(bi + 1, SB, SB0)) : 0;
       bool start = true, ext = false;
       int e = 0;  // proposals of the slice already rejected
       Key ck = {0u, 0u};
       for (;;) {
         const bool active = j < j_end;
         if (!__any_sync(0xffffffffu, active)) break;
-        const int row = g0 / GL * SB + (active ? j - bi * SB : 0);
+        const int row = g * SB + (active ? j - j_begin : 0);
         const bool begin = active && start;
         if (__any_sync(0xffffffffu, begin)) {
           // _slice_bounds (uni_slice_sampler.py:41-64), the group's lanes over the dimensions;
@@ -348,7 +293,7 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
             d[q + 2] = a.z;
             d[q + 3] = a.w;
           }
-          alpha = B.alpha[row];
+          alpha = B.r.alpha[row];
           if (begin) {
             right = hi;
             left = lo;
@@ -357,28 +302,11 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
             ext = false;
           }
         }
-        // uniforms beyond the prepared ones: the group walks the carry-key chain, lane i keeping
-        // the key of proposal e + i, and the slots of the spent uniforms take the new ones
         const bool need = active && e >= made;
-        if (__any_sync(0xffffffffu, need)) {
-          if (need && !ext) {
-            const uint2 v = B.ck[row];
-            ck = Key{v.x, v.y};
-            ext = true;
-          }
-          Key mine = ck, run = ck;
-          for (int i = 0; i < G; ++i) {
-            if (i == li) mine = run;
-            run = fold(run, 0u);
-          }
-          if (need) ck = run;
-          __syncwarp();
-          if (need && li < G) B.u[li][row] = uniform01(bits64(fold(mine, 1u), 0u));
-          __syncwarp();
-        }
+        if (__any_sync(0xffffffffu, need)) spec_more_uniforms<G>(B.r, row, li, need, ext, ck);
         // the interval arithmetic of the next G proposals (_pick_point_in_interval and
         // _shrink_interval, uni_slice_sampler.py:67-111), each lane keeping its own
-        const float *us = &B.u[ext ? 0 : e][row];
+        const float *us = &B.r.u[ext ? 0 : e][row];
         float t_mine = 0.0f;
 #pragma unroll
         for (int i = 0; i < G; ++i) {

@@ -431,6 +431,9 @@ static cudaError_t launch_warp_bucket(const gbns_batch &b, int ib, int ie, const
                                       cudaStream_t stream) {
   const int nblk = ie - ib;
   if (nblk <= 0) return cudaSuccess;
+  bool taken = false;
+  const cudaError_t es = launch_slice_spec_mvn(b, DMAX, ib, ie, Lstar, keys, stream, taken);
+  if (taken || es != cudaSuccess) return es;
   const int warps = DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PER_CTA_32;
   const size_t sm = warp_smem_bytes<DMAX>(warps);
   static bool configured = false;

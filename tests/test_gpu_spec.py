@@ -25,7 +25,7 @@ def _spec(oracle_mod, D, S, K, prior, midpoint, n=42):
             kind, a, b = (np.arange(D) % 2).astype(np.int32), np.where(np.arange(D) % 2, mu, -6.0), \
                 np.where(np.arange(D) % 2, 2.0, 12.0)
     return RunSpec(D=D, num_live_points=n, shell_size=n // 2, num_slices=S, family=family, params=params,
-                   prior_kind=kind, prior_a=a, prior_b=b, max_samples=40 * n, term_cond={"dlogZ": 1e-4},
+                   prior_kind=kind, prior_a=a, prior_b=b, max_samples=40 * n, term_cond={"max_samples": 40 * n},
                    key=oracle_mod.PRNGKey(D + 100 * S), num_phantom=K, midpoint_shrink=midpoint, log_L_offset=offset)
 
 
@@ -40,6 +40,8 @@ def test_every_lane_count_matches_the_oracle(gpu_lib, oracle_mod, runs, D, S, K,
     spec = _spec(oracle_mod, D, S, K, prior, midpoint)
     b = NSBatch([spec] * runs, device="cuda")
     b.init()
+    b.iterate(14)  # contours tight enough that slices outlast the uniforms prepared for them
+    assert int(b.state()[0]["iterations"]) == 14
     live = b.live_view(0)["log_L_raw"].cpu().numpy()
     for at in (spec.shell_size - 1, spec.num_live_points - 2):  # the sampler's contour; a tight one (many shrinks)
         key = oracle_mod.PRNGKey(7 + at)
@@ -68,3 +70,24 @@ def test_evaluation_budget(gpu_lib, oracle_mod):
     for o in out[1:]:
         for x, y in zip(o, out[0]):
             np.testing.assert_array_equal(x.view(np.uint32), y.view(np.uint32))
+
+
+# 201 chains per run (one item each): 16 / 8 / 4 proposals per round, then the warp-cooperative kernel
+@pytest.mark.parametrize("runs", [1, 4, 16, 110])
+@pytest.mark.parametrize("D,S,K,prior,midpoint", [
+    (17, 1, 0, "uniform", True), (24, 21, 3, "uniform", False), (31, 33, 0, "mixed", True), (32, 16, 0, "normal", True),
+    (33, 9, 2, "uniform", True), (50, 18, 0, "mixed", True), (64, 17, 0, "uniform", True)])
+def test_wide_gaussians_match_the_oracle(gpu_lib, oracle_mod, runs, D, S, K, prior, midpoint):
+    from jaxns_gb300.engine import NSBatch
+    spec = _spec(oracle_mod, D, S, K, prior, midpoint, n=402)
+    b = NSBatch([spec] * runs, device="cuda")
+    b.init()
+    b.iterate(14)  # contours tight enough that slices outlast the uniforms prepared for them
+    assert int(b.state()[0]["iterations"]) == 14
+    live = b.live_view(0)["log_L_raw"].cpu().numpy()
+    for at in (spec.shell_size - 1, spec.num_live_points - 2):
+        key = oracle_mod.PRNGKey(7 + at)
+        b.slice_shell(torch.full((runs,), float(live[at])), torch.tensor(key.view(np.int32)).repeat(runs, 1))
+        torch.cuda.synchronize()
+        for r in {0, runs - 1}:
+            assert_shell_exact(oracle_mod, b, r, live[at], key)
