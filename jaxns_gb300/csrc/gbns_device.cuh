@@ -429,6 +429,14 @@ __device__ __forceinline__ FS shfl_up_fs(FS v, int o) {
   return r;
 }
 
+__device__ __forceinline__ FS shfl_fs(FS v, int src) {
+  FS r;
+  r.h = __shfl_sync(0xffffffffu, v.h, src);
+  r.l = __shfl_sync(0xffffffffu, v.l, src);
+  r.e = __shfl_sync(0xffffffffu, v.e, src);
+  return r;
+}
+
 __device__ __forceinline__ FS shfl_xor_fs(FS v, int o) {
   FS r;
   r.h = __shfl_xor_sync(0xffffffffu, v.h, o);
@@ -471,6 +479,20 @@ __device__ __forceinline__ ScaledSum ss_from_fs(FS f) {
 __device__ __forceinline__ double fs_log_d(FS a) {
   if (!(a.h > 0.0f)) return -INFINITY;
   return (double)(logf(a.h) + a.l / a.h) + (double)a.e * GBNS_LN2;
+}
+
+// log((exp L + exp Lprev) / 2) + off as a pair: max + log1p(exp(-|d|)) - ln 2 + off
+__device__ __forceinline__ void log_mid_pair(float L, float Lprev, float off_h, float off_l, float &mh, float &ml) {
+  const float m = fmaxf(L, Lprev), d = L - Lprev;
+  if (isnan(d)) {
+    mh = L + Lprev;  // both -inf (or +inf)
+    ml = 0.0f;
+    return;
+  }
+  float th, tl;
+  pair_sum2(m, 0.0f, log1pf(__expf(-fabsf(d))), 0.0f, th, tl);
+  pair_sum2(th, tl, -0.693147182464599609375f, 1.904654323148236017e-9f, th, tl);
+  pair_sum2(th, tl, off_h, off_l, mh, ml);
 }
 
 struct EvScanFsSmem {
@@ -595,7 +617,6 @@ __device__ void evidence_scan_cta(EvAcc &acc, const float *__restrict__ L, long 
   FS pHP = fs_zero(), pHQ = fs_zero();  // sum dZ L+, dZ L- (h_out)
   float off_h, off_l;
   pair_of(Loff, off_h, off_l);
-  const float ln2_h = 0.693147182464599609375f, ln2_l = -1.904654323148236017e-9f;
   float lxh, lxl, lx2h, lx2l;  // pair copies of the carried log X, log X2
   pair_of(acc.lX, lxh, lxl);
   pair_of(acc.lX2, lx2h, lx2l);
@@ -657,21 +678,10 @@ __device__ void evidence_scan_cta(EvAcc &acc, const float *__restrict__ L, long 
         pair_sum2(bx2h, bx2l, pT2h[j > 0 ? j - 1 : 0], pT2l[j > 0 ? j - 1 : 0], x2ph, x2pl);
       }
       pair_sum2(bxh, bxl, pTh[j], pTl[j], xch[j], xcl[j]);  // log X_k
-      // log((L_k + L_{k-1}) / 2) + Loff as a pair: max + log1p(exp(-|d|)) - ln 2 + Loff; -inf
-      // outside the chunk
+      // -inf outside the chunk
       const float Lcur = Lk[j], Lprev = j == 0 ? Lfirst_m1 : Lk[j > 0 ? j - 1 : 0];
       float mh = -INFINITY, ml = 0.0f;
-      if (valid) {
-        const float m = fmaxf(Lcur, Lprev), d = Lcur - Lprev;
-        if (isnan(d)) {
-          mh = Lcur + Lprev;  // both -inf (or +inf)
-        } else {
-          float th, tl;
-          pair_sum2(m, 0.0f, log1pf(__expf(-fabsf(d))), 0.0f, th, tl);
-          pair_sum2(th, tl, -ln2_h, -ln2_l, th, tl);
-          pair_sum2(th, tl, off_h, off_l, mh, ml);
-        }
-      }
+      if (valid) log_mid_pair(Lcur, Lprev, off_h, off_l, mh, ml);
       // v_dZ = (lX_prev + lt) + lmid, v_c = ((lX2_prev + ltT) - lX_cur) + lmid,
       // v_t2 = (lX2_prev + lt2) + 2 lmid
       float vch = -INFINITY, vcl = 0.0f;
