@@ -41,6 +41,11 @@ def _merge(oracle_mod, runs, n, s, K, ordered):
         b.ph_U.copy_(rep(pU))
     _ffi.call("gbns_batch_merge", ctypes.byref(b._b), b._stream())
     torch.cuda.synchronize()
+    if s == n:  # no seed points above the contour: the run ended at its start and the merge leaves it
+        rec = b.state()[runs - 1]
+        assert rec["done"] == 1 and rec["iterations"] == 0
+        np.testing.assert_array_equal(b.live_view(runs - 1)["log_L_raw"].cpu().numpy(), live)
+        return rec
     key = np.concatenate([new, live[s:]])
     perm = np.argsort(key + 0.0, kind="stable")
     r = runs - 1
