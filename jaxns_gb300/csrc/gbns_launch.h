@@ -49,7 +49,7 @@ cudaError_t lg_tc_prepare(const gbns_batch &b, const gbns_lg_bufs &lg, cudaStrea
 cudaError_t launch_lg_shell_fused(const gbns_batch &b, const gbns_lg_bufs &lg, cudaStream_t stream);
 cudaError_t lg_fused_max_clusters(const gbns_lg_bufs &lg, int *out);
 cudaError_t launch_adjoint_reduce(const double *log_w, long long M, int N, double log_sigma, const double *ss,
-                                  const double *ry, double *out, cudaStream_t stream);
+                                  const double *ry, void *scratch, double *out, cudaStream_t stream);
 cudaError_t launch_adjoint_tc(const double *U, const double *log_w, long long M, int P, const float *Phi,
                               const float *y, int N, double log_tau, double log_sigma, double *out, double *ss,
                               double *ry, float *w_scratch, float *phi_scratch, int *status, cudaStream_t stream);

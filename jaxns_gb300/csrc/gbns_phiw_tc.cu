@@ -1,17 +1,17 @@
 // gbns_phiw_tc.cu -- the Phi w residual contraction on the 5th-generation tensor cores.
 //
-// For a tile of 128 points (slice proposals, or dead points for the adjoint) and 128 / 256
+// For a tile of 128 points (slice proposals, or dead points for the adjoint) and 128 or 256
 // data rows, D[point][row] = w_point . Phi_row is one tcgen05 GEMM with K = P <= 64:
 //   * w and Phi are held as TF32 hi + lo parts (x = hi + lo, both rounded to TF32), rows
 //     padded with zeros to a multiple of 32 floats, so one K block is one 128-byte row;
-//   * one thread issues the TMA loads of the four K-major tiles (128B swizzle, one mbarrier
-//     with an expected byte count) and then, per K step of 8, the three products
-//     hi*hi + hi*lo + lo*hi as tcgen05.mma kind::tf32 into one FP32 accumulator of
-//     128 lanes x 256 columns in tensor memory (3xTF32: fp32-level accuracy);
-//   * the four warps read their 32 lanes back with tcgen05.ld (thread = point, 32 rows per
-//     load), form r = y - Phi w, and add sum r^2 and sum r y to the point's FP64 totals.
-// Every wait is bounded: on time-out the kernel sets GBNS_ERR_WAIT_TIMEOUT, skips the
-// epilogue, frees its tensor memory and returns.
+//   * one thread issues the TMA loads of the K-major tiles (128B swizzle, one mbarrier per tile
+//     with an expected byte count), one thread per K step of 8 the three products
+//     hi*hi + hi*lo + lo*hi as tcgen05.mma kind::tf32 into FP32 accumulators in tensor memory
+//     (3xTF32: fp32-level accuracy);
+//   * epilogue warps read their 32 lanes back with tcgen05.ld (thread = point, 32 rows per
+//     load), form r = y - Phi w, and add sum r^2 (and sum r y) to the point's totals.
+// Every wait is bounded: on time-out a kernel sets GBNS_ERR_WAIT_TIMEOUT, skips its remaining
+// work, frees its tensor memory and returns.
 #include <cuda.h>
 #include <cstdio>
 #include <mutex>
@@ -22,18 +22,8 @@
 namespace gbns {
 
 constexpr int TC_M = 128;                            // points per tile (tensor-memory lanes)
-constexpr int TC_N = 256;                            // data rows per tile (tensor-memory columns)
 constexpr int TC_KB = 32;                            // floats per 128-byte swizzled row (one K block)
-constexpr unsigned TC_A_BYTES = TC_M * TC_KB * 4;    // 16 KB
-constexpr unsigned TC_B_BYTES = TC_N * TC_KB * 4;    // 32 KB
-constexpr unsigned TC_KB_BYTES = 2 * TC_A_BYTES + 2 * TC_B_BYTES;  // hi + lo of both operands: 96 KB
 constexpr long long TC_WAIT_CYCLES = 2000000000ll;   // ~1 s at the maximum SM clock
-
-// Instruction descriptor of tcgen05.mma kind::tf32: D f32 (bits 4-5 = 1), A and B TF32
-// (bits 7-9, 10-12 = 2), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at
-// bits 24-28.
-constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TC_N >> 3) << 17) |
-                              ((uint32_t)(TC_M >> 4) << 24);
 
 struct alignas(128) TcMaps {
   CUtensorMap a_hi, a_lo, b_hi, b_lo;
@@ -92,15 +82,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(TC_IDESC), "r"(accumulate)
-      : "memory");
-}
-
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -119,114 +100,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-}
-
-// One 128-point x 256-row tile.  a_row / b_row: first row of the tile in the point and Phi
-// tensor maps; nkb K blocks of 32 are loaded, nk8 K steps of 8 are multiplied; npts points
-// and nrows rows are valid.  Must be called by all 128 threads of the CTA.
-__device__ void tc_resid_tile(const TcMaps &maps, int a_row, int b_row, int nkb, int nk8, int npts, int nrows,
-                              const float *__restrict__ y, double *ss_out, double *ry_out, int *status) {
-  extern __shared__ unsigned char tc_dyn[];
-  __shared__ __align__(8) unsigned long long bars[2];
-  __shared__ uint32_t tmem_slot;
-  __shared__ int fail;
-  __shared__ float ys[TC_N];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t tiles = (smem_u32(tc_dyn) + 1023u) & ~1023u;  // 1024-byte aligned for the 128B swizzle
-  const uint32_t bar_tma = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[1]);
-
-  if (tid == 0) {
-    mbar_init(bar_tma, 1);
-    mbar_init(bar_mma, 1);
-    fail = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  __syncwarp();
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "r"((uint32_t)TC_N)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  for (int q = tid; q < TC_N; q += blockDim.x) ys[q] = (q < nrows) ? y[q] : 0.0f;
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_slot;
-
-  if (tid == 0) {
-    // lane 0 of warp 0 issues the copies and the MMAs; lanes 1-31 wait for it at __syncwarp
-    mbar_expect_tx(bar_tma, (uint32_t)nkb * TC_KB_BYTES);
-    for (int kb = 0; kb < nkb; ++kb) {
-      const uint32_t base = tiles + (uint32_t)kb * TC_KB_BYTES;
-      tma_load_2d(base, &maps.a_hi, kb * TC_KB, a_row, bar_tma);
-      tma_load_2d(base + TC_A_BYTES, &maps.a_lo, kb * TC_KB, a_row, bar_tma);
-      tma_load_2d(base + 2 * TC_A_BYTES, &maps.b_hi, kb * TC_KB, b_row, bar_tma);
-      tma_load_2d(base + 2 * TC_A_BYTES + TC_B_BYTES, &maps.b_lo, kb * TC_KB, b_row, bar_tma);
-    }
-    if (mbar_wait(bar_tma, 0)) {
-      tc_fence_after();
-      uint32_t acc = 0;
-      for (int k8 = 0; k8 < nk8; ++k8) {
-        const int kb = k8 >> 2;
-        const uint32_t base = tiles + (uint32_t)kb * TC_KB_BYTES, off = (uint32_t)(k8 & 3) * 32u;
-        const uint64_t ah = smem_desc(base + off), al = smem_desc(base + TC_A_BYTES + off);
-        const uint64_t bh = smem_desc(base + 2 * TC_A_BYTES + off);
-        const uint64_t bl = smem_desc(base + 2 * TC_A_BYTES + TC_B_BYTES + off);
-        tc_mma(tmem, al, bh, acc);
-        tc_mma(tmem, ah, bl, 1u);
-        tc_mma(tmem, ah, bh, 1u);
-        acc = 1u;
-      }
-      tc_commit(bar_mma);
-    } else {
-      // the copies did not land: report, give them one more bounded wait, release the others
-      fail = 1;
-      atomicOr(status, (int)GBNS_ERR_WAIT_TIMEOUT);
-      mbar_wait(bar_tma, 0);
-      mbar_arrive(bar_mma);
-    }
-  }
-  __syncwarp();
-  bool ok = mbar_wait(bar_mma, 0);
-  ok = __all_sync(0xffffffffu, ok && fail == 0);
-  tc_fence_after();
-  if (ok) {
-    const int pt = warp * 32 + lane;
-    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-    const int nch = (nrows + 31) >> 5;
-    double s1 = 0.0, s2 = 0.0;
-    for (int ch = 0; ch < nch; ++ch) {
-      float v[32];
-      tc_ld32(taddr + (uint32_t)(ch * 32), v);
-      float p1 = 0.0f, p2 = 0.0f;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int row = ch * 32 + j;
-        if (row < nrows) {
-          const float yy = ys[row];
-          const float rr = yy - v[j];
-          p1 = fmaf(rr, rr, p1);
-          p2 = fmaf(rr, yy, p2);
-        }
-      }
-      s1 += (double)p1;
-      s2 += (double)p2;
-    }
-    if (pt < npts) {
-      atomicAdd(&ss_out[pt], s1);
-      if (ry_out) atomicAdd(&ry_out[pt], s2);
-    }
-  } else if (tid == 32) {
-    atomicOr(status, (int)GBNS_ERR_WAIT_TIMEOUT);
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TC_N) : "memory");
-  }
 }
 
 // ------------------------------------------------------------------ sampler step
@@ -268,6 +141,9 @@ __device__ __forceinline__ float sq_resid32(const float *ys, const float *v, int
 constexpr int SR_ROWS = 128;                       // data rows per tile (accumulator columns)
 constexpr unsigned SR_BOX = 128 * TC_KB * 4;       // one K block of 128 rows: 16 KB
 constexpr int SR_THREADS = 192;
+// Instruction descriptor of tcgen05.mma kind::tf32: D f32 (bits 4-5 = 1), A and B TF32
+// (bits 7-9, 10-12 = 2), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at
+// bits 24-28.
 constexpr uint32_t SR_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(SR_ROWS >> 3) << 17) |
                               ((uint32_t)(TC_M >> 4) << 24);
 
@@ -998,13 +874,219 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
   lf_cluster_sync();
 }
 
-// Adjoint: all dead points (blockIdx.x: 128-point tile) against all rows (blockIdx.y).
-__global__ void __launch_bounds__(128) k_adj_resid_tc(const __grid_constant__ TcMaps maps, long long M, int P, int N,
-                                                      const float *y, double *ss, double *ry, int *status) {
-  const long long p0 = (long long)blockIdx.x * TC_M;
-  const int row0 = blockIdx.y * TC_N;
-  tc_resid_tile(maps, (int)p0, row0, (P + TC_KB - 1) / TC_KB, (P + 7) / 8, (int)min((long long)TC_M, M - p0),
-                min(TC_N, N - row0), y + row0, ss + p0, ry + p0, status);
+// ------------------------------------------------------------------ adjoint
+//
+// All dead points against all data rows: sum r^2 and sum r y per point, r = y - Phi w.  Persistent and
+// warp-specialised, one CTA per SM; the 128-point x 128-row tiles, row tiles fastest, are dealt to
+// the CTAs in equal consecutive ranges, so a CTA keeps a W tile while it walks its row tiles and no
+// wave is left partly empty.  Warp 0 streams W and Phi tiles (hi / lo) by TMA, warp 1 issues the
+// 3xTF32 MMAs into a ring of four 128-column accumulators, warps 2-5 and 6-9 drain alternate
+// tiles (thread = point): per 32 rows one fp32 chain for each sum, the chunks in FP64 registers,
+// added to the point's totals when the point tile changes.
+// Bound: the tensor pipe (a 128 x 128 x 32 tile is ~830 cycles of 3xTF32 MMAs) and the epilogue's
+// dependent FMA chains, 32 long, which two sets of warps hide.  40,000 points x 4096 rows x 32: one
+// tile per CTA (5,008 CTAs, copy, MMAs and epilogue in turn) 119 us; see launch_adjoint_tc.
+struct AdjStages {
+  int nkb;      // K blocks of 32 floats
+  int w_bufs;   // W tiles in shared memory (2 at one K block, 1 at two)
+  int phi_bufs; // Phi tiles (4 / 2)
+};
+constexpr int ADJ_THREADS = 320;
+constexpr int ADJ_ACC = 4;
+
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_constant__ TcMaps maps, AdjStages sg, long long M,
+                                                              int P, int N, const float *__restrict__ y, double *ss,
+                                                              double *ry, int *status) {
+  extern __shared__ unsigned char adj_dyn[];
+  // 0-1 w_full, 2-3 w_empty, 4-7 phi_full, 8-11 phi_empty, 12-15 acc_full, 16-19 acc_empty
+  __shared__ __align__(8) unsigned long long bars[20];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  __shared__ __align__(16) float ys[8][SR_ROWS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t base = (smem_u32(adj_dyn) + 1023u) & ~1023u;
+  const int NK = sg.nkb, WB = sg.w_bufs, PB = sg.phi_bufs;
+  auto w_at = [&](int buf, int lo, int kb) { return base + (uint32_t)((buf * 2 + lo) * NK + kb) * SR_BOX; };
+  auto phi_at = [&](int buf, int lo, int kb) {
+    return base + (uint32_t)(2 * WB * NK + (buf * 2 + lo) * NK + kb) * SR_BOX;
+  };
+  auto bar = [&](int q) { return smem_u32(&bars[q]); };
+  const long long row_tiles = (N + SR_ROWS - 1) / SR_ROWS, tiles = ((M + TC_M - 1) / TC_M) * row_tiles;
+  const long long t0 = tiles * blockIdx.x / gridDim.x, t1 = tiles * (blockIdx.x + 1) / gridDim.x;
+
+  if (tid == 0) {
+    for (int q = 0; q < 16; ++q) mbar_init(bar(q), 1);
+    for (int q = 16; q < 20; ++q) mbar_init(bar(q), 4);  // one arrival per warp of the draining set
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncwarp();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"((uint32_t)(ADJ_ACC * SR_ROWS))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  const volatile int *ab = &abort_flag;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      long long pt = -1;
+      int wu = 0, issued = 0;
+      for (long long t = t0; t < t1 && ok; ++t) {
+        const long long p = t / row_tiles;
+        const int n = (int)(t - t0);
+        if (p != pt) {
+          const int q = wu % WB;
+          ok = mbar_wait_or_abort(bar(2 + q), (uint32_t)(((wu / WB) & 1) ^ 1), ab);
+          if (!ok) break;
+          mbar_expect_tx(bar(q), 2u * (uint32_t)NK * SR_BOX);
+          for (int kb = 0; kb < NK; ++kb) {
+            tma_load_2d(w_at(q, 0, kb), &maps.a_hi, kb * TC_KB, (int)(p * TC_M), bar(q));
+            tma_load_2d(w_at(q, 1, kb), &maps.a_lo, kb * TC_KB, (int)(p * TC_M), bar(q));
+          }
+          ++wu;
+          pt = p;
+        }
+        const int q = n % PB, r0 = (int)(t - p * row_tiles) * SR_ROWS;
+        ok = mbar_wait_or_abort(bar(8 + q), (uint32_t)(((n / PB) & 1) ^ 1), ab);
+        if (!ok) break;
+        mbar_expect_tx(bar(4 + q), 2u * (uint32_t)NK * SR_BOX);
+        for (int kb = 0; kb < NK; ++kb) {
+          tma_load_2d(phi_at(q, 0, kb), &maps.b_hi, kb * TC_KB, r0, bar(4 + q));
+          tma_load_2d(phi_at(q, 1, kb), &maps.b_lo, kb * TC_KB, r0, bar(4 + q));
+        }
+        ++issued;
+      }
+      if (!ok) {
+        abort_flag = 1;
+        atomicOr(status, (int)GBNS_ERR_WAIT_TIMEOUT);
+        // copies still in flight get one more bounded wait
+        for (int i = issued > PB ? issued - PB : 0; i < issued; ++i) mbar_wait(bar(4 + i % PB), (uint32_t)((i / PB) & 1));
+        for (int i = wu > WB ? wu - WB : 0; i < wu; ++i) mbar_wait(bar(i % WB), (uint32_t)((i / WB) & 1));
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const int nk8 = (P + 7) / 8;
+      bool ok = true;
+      long long pt = -1;
+      int wu = -1;
+      for (long long t = t0; t < t1; ++t) {
+        const long long p = t / row_tiles;
+        const int n = (int)(t - t0), q = n % PB, a = n % ADJ_ACC;
+        if (p != pt) {
+          ++wu;
+          pt = p;
+          ok = mbar_wait_or_abort(bar(wu % WB), (uint32_t)((wu / WB) & 1), ab);
+        }
+        ok = ok && mbar_wait_or_abort(bar(4 + q), (uint32_t)((n / PB) & 1), ab) &&
+             mbar_wait_or_abort(bar(16 + a), (uint32_t)(((n / ADJ_ACC) & 1) ^ 1), ab);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem + (uint32_t)(a * SR_ROWS);
+        const int wb = wu % WB;
+        for (int k8 = 0; k8 < nk8; ++k8) {
+          const int kb = k8 >> 2;
+          const uint32_t off = (uint32_t)(k8 & 3) * 32u;
+          const uint64_t ah = smem_desc(w_at(wb, 0, kb) + off), al = smem_desc(w_at(wb, 1, kb) + off);
+          const uint64_t bh = smem_desc(phi_at(q, 0, kb) + off), bl = smem_desc(phi_at(q, 1, kb) + off);
+          tc_mma_d(d, al, bh, SR_IDESC, k8 > 0 ? 1u : 0u);
+          tc_mma_d(d, ah, bl, SR_IDESC, 1u);
+          tc_mma_d(d, ah, bh, SR_IDESC, 1u);
+        }
+        tc_commit(bar(12 + a));  // accumulator a full
+        tc_commit(bar(8 + q));   // Phi buffer q free
+        if (t + 1 == t1 || (t + 1) / row_tiles != p) tc_commit(bar(2 + wb));  // W buffer free
+      }
+      if (!ok) {
+        abort_flag = 1;
+        atomicOr(status, (int)GBNS_ERR_WAIT_TIMEOUT);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue: set 0 (warps 2-5) drains the range's even tiles, set 1 (warps 6-9) the odd ones
+    const int set = (warp - 2) >> 2, qd = warp & 3, ew = warp - 2;
+    double s1 = 0.0, s2 = 0.0;
+    bool ok = true;
+    // y of the set's next tile is loaded into registers while the current one is processed
+    float yn[4];
+    auto load_y = [&](long long t) {
+      const int r0 = (int)(t % row_tiles) * SR_ROWS;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int row = r0 + lane + 32 * k;
+        yn[k] = t < t1 && row < N ? y[row] : 0.0f;
+      }
+    };
+    load_y(t0 + set);
+    for (long long t = t0 + set; t < t1; t += 2) {
+      const long long p = t / row_tiles;
+      const int n = (int)(t - t0), a = n % ADJ_ACC;
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ys[ew][lane + 32 * k] = yn[k];
+      __syncwarp();
+      load_y(t + 2);
+      ok = mbar_wait_or_abort(bar(12 + a), (uint32_t)((n / ADJ_ACC) & 1), ab);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(a * SR_ROWS);
+#pragma unroll 1
+      for (int ch = 0; ch < 4; ++ch) {
+        float v[32];
+        tc_ld32(taddr + (uint32_t)(ch * 32), v);
+        if (ch == 3) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(16 + a));  // accumulator a drained
+        }
+        // rows past the last data row have y = 0 and a zero product: they add nothing
+        float p1 = 0.0f, p2 = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 yy = *reinterpret_cast<const float4 *>(&ys[ew][ch * 32 + j]);
+          const float yv[4] = {yy.x, yy.y, yy.z, yy.w};
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const float rr = yv[x] - v[j + x];
+            p1 = fmaf(rr, rr, p1);
+            p2 = fmaf(rr, yv[x], p2);
+          }
+        }
+        s1 += (double)p1;
+        s2 += (double)p2;
+      }
+      if (t + 2 >= t1 || (t + 2) / row_tiles != p) {
+        const long long pnt = p * TC_M + qd * 32 + lane;
+        if (pnt < M) {
+          atomicAdd(&ss[pnt], s1);
+          atomicAdd(&ry[pnt], s2);
+        }
+        s1 = s2 = 0.0;
+      }
+    }
+    if (!ok && lane == 0) {
+      abort_flag = 1;
+      atomicOr(status, (int)GBNS_ERR_WAIT_TIMEOUT);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(ADJ_ACC * SR_ROWS))
+                 : "memory");
+  }
 }
 
 // Phi of every run -> TF32 hi / lo rows of 64 floats (zero beyond P).
@@ -1029,9 +1111,13 @@ __global__ void k_split_phi(gbns_batch b, gbns_lg_bufs lg) {
 // Dead points for the adjoint: w = tau * sqrt(2) * erfinv(2u - 1) (the Normal(0, tau^2)
 // quantile), and Phi, both as TF32 hi/lo rows of ld floats.
 __global__ void k_adj_split(const double *U, long long M, int P, const float *Phi, int N, float tau, int ld,
-                            float *w_hi, float *w_lo, float *phi_hi, float *phi_lo) {
+                            float *w_hi, float *w_lo, float *phi_hi, float *phi_lo, double *ss, double *ry) {
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long nw = M * ld, np = (long long)N * ld;
+  if (q < M) {  // the points' totals start at zero
+    ss[q] = 0.0;
+    ry[q] = 0.0;
+  }
   if (q >= nw + np) return;
   float h = 0.0f, l = 0.0f;
   if (q < nw) {
@@ -1094,7 +1180,7 @@ cudaError_t set_smem_attrs() {
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(mu);
   if (done[dev]) return cudaSuccess;
-  const int bytes = 2 * (int)TC_KB_BYTES + 1024;  // two K blocks: 6 x 2 x 16 KB (sampler) or 2 x 96 KB (adjoint)
+  const int bytes = 12 * (int)SR_BOX + 1024;  // twelve 16 KB tiles
   err = cudaFuncSetAttribute(k_lg_resid_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(k_adj_resid_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err == cudaSuccess) done[dev] = true;
@@ -1223,8 +1309,6 @@ cudaError_t launch_adjoint_tc(const double *U, const double *log_w, long long M,
                               int N, double log_tau, double log_sigma, double *out, double *ss, double *ry,
                               float *w_scratch, float *phi_scratch, int *status, cudaStream_t s) {
   cudaError_t e = set_smem_attrs();
-  if (e == cudaSuccess) e = cudaMemsetAsync(ss, 0, sizeof(double) * M, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(ry, 0, sizeof(double) * M, s);
   if (e != cudaSuccess) return e;
   const int ld = P > TC_KB ? 64 : 32;
   if (M > 0) {
@@ -1232,15 +1316,21 @@ cudaError_t launch_adjoint_tc(const double *U, const double *log_w, long long M,
     float *p_hi = phi_scratch, *p_lo = phi_scratch + (long long)N * ld;
     const long long tot = (M + N) * (long long)ld;
     k_adj_split<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(U, M, P, Phi, N, (float)exp(log_tau), ld, w_hi, w_lo,
-                                                              p_hi, p_lo);
+                                                              p_hi, p_lo, ss, ry);
     TcMaps maps;
     if (!encode_rows(&maps.a_hi, w_hi, M, ld, TC_M) || !encode_rows(&maps.a_lo, w_lo, M, ld, TC_M) ||
-        !encode_rows(&maps.b_hi, p_hi, N, ld, TC_N) || !encode_rows(&maps.b_lo, p_lo, N, ld, TC_N))
+        !encode_rows(&maps.b_hi, p_hi, N, ld, SR_ROWS) || !encode_rows(&maps.b_lo, p_lo, N, ld, SR_ROWS))
       return cudaErrorInvalidValue;
-    dim3 grid((unsigned)((M + TC_M - 1) / TC_M), (unsigned)((N + TC_N - 1) / TC_N));
-    k_adj_resid_tc<<<grid, 128, (ld / TC_KB) * TC_KB_BYTES + 1024, s>>>(maps, M, P, N, y, ss, ry, status);
+    // one CTA per SM (its tensor memory and 193 KB of shared memory are all of the SM's)
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const long long tiles = ((M + TC_M - 1) / TC_M) * ((N + SR_ROWS - 1) / SR_ROWS);
+    const AdjStages sg = {ld / TC_KB, ld == TC_KB ? 2 : 1, ld == TC_KB ? 4 : 2};
+    k_adj_resid_tc<<<(unsigned)(tiles < sms ? tiles : sms), ADJ_THREADS, 12 * SR_BOX + 1024, s>>>(maps, sg, M, P, N, y, ss,
+                                                                                             ry, status);
   }
-  return launch_adjoint_reduce(log_w, M, N, log_sigma, ss, ry, out, s);
+  return launch_adjoint_reduce(log_w, M, N, log_sigma, ss, ry, w_scratch, out, s);  // w is spent
 }
 
 }  // namespace gbns

@@ -16,7 +16,7 @@
 // Bound: latency (barriers ~2 us, FP64 logarithms at the ends) up to ~100 k samples per run; beyond
 // that the ~1000 instructions per sample, now on every SM.
 // us, one block per run / set -> team: one run of 936 k samples out of order with its U rows
-// 105,500 -> 990, one linear-Gaussian run of 26 k samples 1,392 -> 107, 48 runs of 13 k 166 -> 98;
+// 105,500 -> 1,620, one linear-Gaussian run of 26 k samples 1,392 -> 107, 48 runs of 13 k 166 -> 98;
 // evidence of 250 k samples with log Z per sample 2,176 -> 52, their tree count (five launches) 20 -> 17.
 #include <cooperative_groups.h>
 #include "gbns_device.cuh"
