@@ -13,14 +13,15 @@ CSRC = os.path.join(_HERE, "csrc")
 OUT_DIR = os.path.join(_HERE, "_lib")
 OBJ_DIR = os.path.join(os.path.dirname(_HERE), "_build", "obj")
 SOURCES = ["gbns_slice.cu", "gbns_slice_spec.cu", "gbns_slice_spec_mvn.cu", "gbns_slice_warp.cu", "gbns_ns.cu",
-           "gbns_results.cu", "gbns_results_team.cu", "gbns_phiw.cu", "gbns_phiw_tc.cu", "gbns_api.cu",
+           "gbns_points.cu", "gbns_results.cu", "gbns_results_team.cu", "gbns_phiw.cu", "gbns_phiw_tc.cu", "gbns_api.cu",
            "gbns_static.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 # Translation units whose fp32 arithmetic is reproduced bit for bit by a CPU model of the
 # kernels: no implicit multiply-add contraction, so every fused multiply-add is an explicit
 # fmaf in the source and the rounding sequence is the one written there.
-EXACT_FP32 = {"gbns_slice.cu", "gbns_slice_spec.cu", "gbns_slice_spec_mvn.cu", "gbns_slice_warp.cu", "gbns_ns.cu"}
+EXACT_FP32 = {"gbns_slice.cu", "gbns_slice_spec.cu", "gbns_slice_spec_mvn.cu", "gbns_slice_warp.cu", "gbns_ns.cu",
+              "gbns_points.cu"}
 
 
 def _nvcc() -> str:

@@ -3,6 +3,8 @@
 // error code and leaves a thread-local message for gbns_last_error().
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <new>
 #include "gbns_device.cuh"
 #include "gbns_launch.h"
 
@@ -94,7 +96,20 @@ int gbns_batch_init(const gbns_batch *batch, void *stream) {
                                    (cudaStream_t)stream);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize((cudaStream_t)stream);
   if ((e = check(ce, "gbns_batch_init: reading the run table"))) return e;
-  return check(gbns::launch_init(*batch, last.live_off + last.n, (cudaStream_t)stream), "gbns_batch_init");
+  // which of the two initialisations the batch needs
+  bool lg = last.family == GBNS_LIK_LINGAUSS, fp32 = !lg;
+  for (int k = 0; k < 8; ++k) fp32 = fp32 || batch->bucket_end[k] > batch->bucket_begin[k];
+  if (fp32 && !lg && batch->num_runs > 1) {
+    // (one strided copy: runs of both kinds in one batch are possible for a caller of this ABI)
+    std::unique_ptr<int[]> fam(new (std::nothrow) int[batch->num_runs]);
+    if (!fam) return fail(-1, "gbns_batch_init: out of host memory%s");
+    ce = cudaMemcpy2DAsync(fam.get(), sizeof(int), &batch->runs->family, sizeof(gbns_run_desc), sizeof(int),
+                           (size_t)batch->num_runs, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize((cudaStream_t)stream);
+    if ((e = check(ce, "gbns_batch_init: reading the run table"))) return e;
+    for (int r = 0; r < batch->num_runs; ++r) lg = lg || fam[r] == GBNS_LIK_LINGAUSS;
+  }
+  return check(gbns::launch_init(*batch, last.live_off + last.n, lg, fp32, (cudaStream_t)stream), "gbns_batch_init");
 }
 
 int gbns_batch_iterate(const gbns_batch *batch, int num_iterations, void *stream) {

@@ -25,7 +25,9 @@ cudaError_t launch_slice_spec(const gbns_batch &b, int family, int dmax, int ib,
 // The same for the warp-cooperative correlated-Gaussian bucket of a DMAX (gbns_slice_spec_mvn.cu).
 cudaError_t launch_slice_spec_mvn(const gbns_batch &b, int dmax, int ib, int ie, const float *Lstar, const uint32_t *keys,
                                   cudaStream_t stream, bool &taken);
-cudaError_t launch_init(const gbns_batch &b, long long total_points, cudaStream_t stream);
+// lg / fp32: whether the batch has linear-Gaussian runs / runs of the other families
+cudaError_t launch_init(const gbns_batch &b, long long total_points, bool lg, bool fp32, cudaStream_t stream);
+cudaError_t launch_init_lg(const gbns_batch &b, long long total_points, cudaStream_t stream);
 cudaError_t launch_merge(const gbns_batch &b, cudaStream_t stream);
 cudaError_t launch_finalize(const gbns_batch &b, cudaStream_t stream);
 cudaError_t launch_forward(const gbns_batch &b, int run, const float *U, float *logL, long long B, cudaStream_t stream);

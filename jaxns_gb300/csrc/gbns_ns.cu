@@ -12,9 +12,8 @@ namespace gbns {
 
 // ------------------------------------------------------ generic likelihood ----
 
-// Model.forward for any family with runtime D (parameters read from global memory),
-// relative to the run's log_L_offset: MVN -0.5 |Linv (x - mu)|^2, shells
-// logaddexp(-0.5 z1^2, -0.5 z2^2), linear Gaussian -0.5 |y - Phi w|^2 / sigma^2.
+// log L of one point with runtime D (parameters read from global memory), relative to the run's
+// log_L_offset: MVN -0.5 |Linv (x - mu)|^2, shells logaddexp(-0.5 z1^2, -0.5 z2^2).
 __device__ float loglik_generic(const gbns_batch &b, const gbns_run_desc &rd, const float *U) {
   const int D = rd.D;
   const float *fp = b.fparams + rd.param_off;
@@ -31,7 +30,7 @@ __device__ float loglik_generic(const gbns_batch &b, const gbns_run_desc &rd, co
       s = fmaf(acc, acc, s);
     }
     v = -0.5f * s;
-  } else if (rd.family == GBNS_LIK_SHELLS) {
+  } else {
     float r1 = 0.f, r2 = 0.f;
     for (int j = 0; j < D; ++j) {
       const float e1 = x[j] - fp[j], e2 = x[j] - fp[D + j];
@@ -44,49 +43,8 @@ __device__ float loglik_generic(const gbns_batch &b, const gbns_run_desc &rd, co
     const float s1 = -0.5f * z1 * z1, s2 = -0.5f * z2 * z2;
     const float m = fmaxf(s1, s2), dd = s1 - s2;
     v = (dd != dd) ? s1 + s2 : m + gbns_fm_log1p(gbns_fm_exp(-fabsf(dd)));
-  } else {
-    const int N = rd.N;
-    const float *Phi = fp, *y = fp + (size_t)N * D;
-    const float sigma = fp[(size_t)N * D + N];
-    float ss = 0.f;
-    for (int a = 0; a < N; ++a) {
-      float r = y[a];
-      for (int j = 0; j < D; ++j) r = fmaf(-Phi[(size_t)a * D + j], x[j], r);
-      ss = fmaf(r, r, ss);
-    }
-    v = -0.5f * ss / (sigma * sigma);
   }
   return (v != v) ? -INFINITY : v;
-}
-
-// Linear-Gaussian log L (relative to the run's offset) of an FP64 U: -|y - Phi w|^2 / (2 sigma^2).
-__device__ float loglik_lg_d(const gbns_batch &b, const gbns_run_desc &rd, const double *U) {
-  const int D = rd.D, N = rd.N;
-  const float *fp = b.fparams + rd.param_off;
-  float x[64];
-  for (int j = 0; j < D; ++j)
-    x[j] = prior_quantile_d(b.prior_kind[rd.prior_off + j], b.prior_a[rd.prior_off + j],
-                            b.prior_b[rd.prior_off + j], U[j]);
-  const float *Phi = fp, *y = fp + (size_t)N * D;
-  const float sigma = fp[(size_t)N * D + N];
-  float ss = 0.f;
-  for (int a = 0; a < N; ++a) {
-    float r = y[a];
-    for (int j = 0; j < D; ++j) r = fmaf(-Phi[(size_t)a * D + j], x[j], r);
-    ss = fmaf(r, r, ss);
-  }
-  const float v = -0.5f * ss / (sigma * sigma);
-  return (v != v) ? -INFINITY : v;
-}
-
-// U: [B, ucols] 32-bit words (FP64 U for the linear-Gaussian family).
-__global__ void k_forward(gbns_batch b, int run, const float *__restrict__ U, float *__restrict__ out, long long B) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  const gbns_run_desc &rd = b.runs[run];
-  const float v = rd.family == GBNS_LIK_LINGAUSS ? loglik_lg_d(b, rd, (const double *)U + i * rd.D)
-                                                 : loglik_generic(b, rd, U + i * rd.D);
-  out[i] = (float)((double)v + rd.log_L_offset);
 }
 
 // ------------------------------------------------------------ termination ----
@@ -213,7 +171,7 @@ __device__ void store_append(const gbns_batch &b, const gbns_run_desc &rd, long 
 
 // create_init_state (nested_samplers/common/initialisation.py:20-84): n uniform samples
 // strictly above -inf (_single_uniform_sample, common/uniform_sample.py:12-60).
-__global__ void k_init_points(gbns_batch b, long long total) {
+__global__ void k_init_points(gbns_batch b, long long total) {  // (linear-Gaussian runs: gbns_points.cu)
   const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (g >= total) return;
   int lo = 0, hi = b.num_runs;  // live points are packed: run r owns [live_off, live_off + n)
@@ -225,24 +183,18 @@ __global__ void k_init_points(gbns_batch b, long long total) {
   const gbns_run_desc &rd = b.runs[r];
   const int i = (int)(g - rd.live_off);
   const int D = rd.D;
-  const bool lg = rd.family == GBNS_LIK_LINGAUSS;
+  if (rd.family == GBNS_LIK_LINGAUSS) return;
   const Key K0 = {b.state[r].key[0], b.state[r].key[1]};
   const Key sample_key = fold(K0, 1u);
   const Key ki = fold(sample_key, (uint32_t)i);
   Key k = fold(ki, 0u), sk = fold(ki, 1u);
   float U[64];
-  double Ud[64];
   float logL;
   int ne = 0;
   for (;;) {
     const Key uk = fold(sk, 1u);  // Model.sample_U: uniform(split(key)[1], (D,))
-    if (lg) {
-      for (int j = 0; j < D; ++j) Ud[j] = uniform01_d(bits64(uk, (uint32_t)j));
-      logL = loglik_lg_d(b, rd, Ud);
-    } else {
-      for (int j = 0; j < D; ++j) U[j] = uniform01(bits64(uk, (uint32_t)j));
-      logL = loglik_generic(b, rd, U);
-    }
+    for (int j = 0; j < D; ++j) U[j] = uniform01(bits64(uk, (uint32_t)j));
+    logL = loglik_generic(b, rd, U);
     ++ne;
     if (!(logL <= -INFINITY)) break;
     if (ne >= 1000000) { atomicOr(&b.state[r].status, (int)GBNS_ERR_INIT_BUDGET); break; }
@@ -251,12 +203,7 @@ __global__ void k_init_points(gbns_batch b, long long total) {
     k = nk;
   }
   const long long o = rd.live_off + i;
-  if (lg) {
-    double *dst = (double *)(b.live_U[1] + rd.liveU_off) + (long long)i * D;
-    for (int j = 0; j < D; ++j) dst[j] = Ud[j];
-  } else {
-    for (int j = 0; j < D; ++j) b.live_U[1][rd.liveU_off + (long long)i * D + j] = U[j];
-  }
+  for (int j = 0; j < D; ++j) b.live_U[1][rd.liveU_off + (long long)i * D + j] = U[j];
   b.live_L[1][o] = logL;
   b.live_Lc[1][o] = -INFINITY;
   b.live_E[1][o] = ne;
@@ -815,10 +762,14 @@ __global__ void k_finalize(gbns_batch b) {
 
 static int max_n(const gbns_batch &b) { return b.nmax; }
 
-cudaError_t launch_init(const gbns_batch &b, long long total_points, cudaStream_t stream) {
+cudaError_t launch_init(const gbns_batch &b, long long total_points, bool lg, bool fp32, cudaStream_t stream) {
   const int T = 128;
   const long long blocks = (total_points + T - 1) / T;
-  if (blocks > 0) k_init_points<<<(unsigned)blocks, T, 0, stream>>>(b, total_points);
+  if (fp32 && blocks > 0) k_init_points<<<(unsigned)blocks, T, 0, stream>>>(b, total_points);
+  if (lg) {
+    const cudaError_t e = launch_init_lg(b, total_points, stream);
+    if (e != cudaSuccess) return e;
+  }
   int NP = 1;
   while (NP < max_n(b)) NP <<= 1;
   k_init_finish<<<b.num_runs, 1024, NP * sizeof(unsigned long long), stream>>>(b);
@@ -853,12 +804,6 @@ cudaError_t launch_merge(const gbns_batch &b, cudaStream_t stream) {
 
 cudaError_t launch_finalize(const gbns_batch &b, cudaStream_t stream) {
   k_finalize<<<b.num_runs, 256, 0, stream>>>(b);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_forward(const gbns_batch &b, int run, const float *U, float *logL, long long B, cudaStream_t stream) {
-  if (B <= 0) return cudaSuccess;
-  k_forward<<<(unsigned)((B + 127) / 128), 128, 0, stream>>>(b, run, U, logL, B);
   return cudaGetLastError();
 }
 
