@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(256) k_adj_resid(const double *U, long long M,
 // its largest a, then the sums of exp(a - max) and of the two gradient terms, and k_adj_total
 // combines the blocks.  A single block writes the result itself.
 // Bound: FP64 (an exponential and two divisions per point on ~2 lanes per clock and SM), so every
-// SM takes part: 40,000 points, one block of 1024 threads 712 us; see launch_adjoint_reduce.
+// SM takes part; what is left is FP64 latency.
 struct AdjSums {
   double mx, se, gt, gs;
 };
@@ -638,7 +638,7 @@ cudaError_t launch_adjoint(const double *U, const double *log_w, long long M, in
 // scratch: 8-byte-aligned device memory of 4 M doubles at least, or NULL (one block).
 cudaError_t launch_adjoint_reduce(const double *log_w, long long M, int N, double log_sigma, const double *ss,
                                   const double *ry, void *scratch, double *out, cudaStream_t s) {
-  // a block per 128 points, two blocks per SM at most: 40,000 points 712 -> 10 us (two launches)
+  // a block per 128 points, two blocks per SM at most: 40,000 points 712 -> 28 us (two launches)
   int dev = 0, sms = 0;
   cudaError_t e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

@@ -54,21 +54,25 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0u;
+}
+
 // Waits for phase `parity` of the barrier to complete; false after TC_WAIT_CYCLES.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
-  while (true) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
+  while (!mbar_try(bar, parity))
     if (clock64() - t0 > TC_WAIT_CYCLES) return false;
-  }
+  return true;
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
@@ -86,20 +90,28 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// 32 consecutive fp32 columns of this warp's 32 lanes: thread t gets lane (base lane + t).
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+// ------------------------------------------------------------------ sampler step
+//
+// Persistent, warp-specialised, one CTA per SM: each CTA walks work units (run, 128-chain tile,
+// range of 128-row tiles) with a grid stride.  Warp 0 streams the unit's W tile (hi / lo) and Phi
+// stages (two row tiles x one K block, hi / lo) through shared memory with TMA, warp 1 issues the
+// 3xTF32 MMAs of two row tiles at a time (256 rows, see the adjoint kernel) into two 256-column
+// accumulators in turn, and warps 2-5 and 6-9 drain a row tile each (thread = chain), keep the
+// chain's partial sum of squares in a register over the unit and add it to the chain's FP64
+// total once per unit.  Copies, MMAs and epilogue of successive row tiles overlap.  Units whose
+// chain tile has no pending proposal are skipped by every role alike (the flags are read-only
+// during the launch).
+// Bound: MMAs (~15 us of the 38 below) and, per unit, the latency of its flags and first copies.
+// Twelve problems of up to 16384 x 64: 128-row MMAs, four 128-column accumulators 47 us per launch,
+// this 38 us.
+// hi + lo += x (TwoSum of hi and x, the rounding error carried in lo).  GB300 runs FP64 at
+// about 1/64 of the FP32 rate, so the step's sums of squares travel as fp32 pairs: each adds
+// at most a few units of 2^-48 of relative error, far below the fp32 rounding of the 32-row
+// chunk sums they carry.
+__device__ __forceinline__ void lf_pair_acc(float &hi, float &lo, float x) {
+  float e;
+  pair_add(hi, x, hi, e);
+  lo += e;
 }
 
 // ------------------------------------------------------------------ sampler step
@@ -112,14 +124,39 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
 // the unit's row tiles and add it to the chain's FP64 total once per unit.  Copies, MMAs and
 // epilogue of successive row tiles overlap.  Units whose chain tile has no pending proposal
 // are skipped by every role alike (the flags are read-only during the launch).
+// 32 consecutive fp32 columns of this warp's 32 lanes (thread t gets lane base + t): the load, and
+// its wait.  The registers pass through the wait, so no use of them can be scheduled before it.  One load can be in flight while the columns before are used.
+__device__ __forceinline__ void tc_ld32_start(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+
+__device__ __forceinline__ void tc_ld32_finish(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]),
+                 "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]),
+                 "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+
 // sum_j (y_j - v_j)^2 over the first n (<= 32) of 32 accumulator columns, in four
 // independent FMA chains (j mod 4) so that the reduction does not serialise on FMA latency
-__device__ __forceinline__ float sq_resid32(const float *ys, const float *v, int n) {
+__device__ __forceinline__ float sq_resid32(const float *ys, const uint32_t (&v)[32], int n) {
   float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;
   if (n >= 32) {
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
-      const float r0 = ys[j] - v[j], r1 = ys[j + 1] - v[j + 1], r2 = ys[j + 2] - v[j + 2], r3 = ys[j + 3] - v[j + 3];
+      const float4 y = *reinterpret_cast<const float4 *>(ys + j);  // (16-byte aligned)
+      const float r0 = y.x - __uint_as_float(v[j]), r1 = y.y - __uint_as_float(v[j + 1]);
+      const float r2 = y.z - __uint_as_float(v[j + 2]), r3 = y.w - __uint_as_float(v[j + 3]);
       p0 = fmaf(r0, r0, p0);
       p1 = fmaf(r1, r1, p1);
       p2 = fmaf(r2, r2, p2);
@@ -128,7 +165,8 @@ __device__ __forceinline__ float sq_resid32(const float *ys, const float *v, int
   } else {
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
-      const float r0 = ys[j] - v[j], r1 = ys[j + 1] - v[j + 1], r2 = ys[j + 2] - v[j + 2], r3 = ys[j + 3] - v[j + 3];
+      const float r0 = ys[j] - __uint_as_float(v[j]), r1 = ys[j + 1] - __uint_as_float(v[j + 1]);
+      const float r2 = ys[j + 2] - __uint_as_float(v[j + 2]), r3 = ys[j + 3] - __uint_as_float(v[j + 3]);
       p0 = j < n ? fmaf(r0, r0, p0) : p0;
       p1 = j + 1 < n ? fmaf(r1, r1, p1) : p1;
       p2 = j + 2 < n ? fmaf(r2, r2, p2) : p2;
@@ -140,12 +178,15 @@ __device__ __forceinline__ float sq_resid32(const float *ys, const float *v, int
 
 constexpr int SR_ROWS = 128;                       // data rows per tile (accumulator columns)
 constexpr unsigned SR_BOX = 128 * TC_KB * 4;       // one K block of 128 rows: 16 KB
-constexpr int SR_THREADS = 192;
+constexpr int SR_THREADS = 320;
 // Instruction descriptor of tcgen05.mma kind::tf32: D f32 (bits 4-5 = 1), A and B TF32
 // (bits 7-9, 10-12 = 2), both K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at
 // bits 24-28.
-constexpr uint32_t SR_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(SR_ROWS >> 3) << 17) |
-                              ((uint32_t)(TC_M >> 4) << 24);
+constexpr uint32_t tc_idesc(int rows) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(rows >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+}
+constexpr int MMA_ROWS = 2 * SR_ROWS;              // data rows per MMA: two boxes
+constexpr unsigned STAGE = 4 * SR_BOX;             // a Phi stage: 256 rows x one K block, hi and lo
 
 struct alignas(128) SrMaps {
   CUtensorMap w_hi, w_lo, phi_hi, phi_lo;
@@ -161,22 +202,48 @@ __device__ __forceinline__ void tc_mma_d(uint32_t d_tmem, uint64_t adesc, uint64
       : "memory");
 }
 
+// One K block (32 floats, or the first `steps` K steps of 8) of the 3xTF32 product of two K-major
+// tiles into accumulator d: per step lo*hi, hi*lo, hi*hi.  The matrix descriptors of the tiles'
+// starts are built once; a step is 32 bytes, two units of the descriptor's address field, which
+// cannot carry out of its 32-bit word.
+struct TcOperand {
+  uint32_t hi_lo, lo_lo, up;  // low words of the hi and lo tiles' descriptors, their common high word
+};
+
+__device__ __forceinline__ TcOperand tc_operand(uint32_t hi_addr, uint32_t lo_addr) {
+  TcOperand o;
+  const uint64_t h = smem_desc(hi_addr);
+  o.hi_lo = (uint32_t)h;
+  o.lo_lo = (uint32_t)smem_desc(lo_addr);
+  o.up = (uint32_t)(h >> 32);
+  return o;
+}
+
+__device__ __forceinline__ uint64_t tc_desc(uint32_t lo, uint32_t up) { return ((uint64_t)up << 32) | (uint64_t)lo; }
+
+__device__ __forceinline__ void tc_mma_block(uint32_t d, const TcOperand &a, const TcOperand &b, int steps, uint32_t idesc,
+                                             uint32_t accumulate) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k < steps) {
+      const uint64_t ah = tc_desc(a.hi_lo + 2u * k, a.up), al = tc_desc(a.lo_lo + 2u * k, a.up);
+      const uint64_t bh = tc_desc(b.hi_lo + 2u * k, b.up), bl = tc_desc(b.lo_lo + 2u * k, b.up);
+      tc_mma_d(d, al, bh, idesc, k > 0 ? 1u : accumulate);
+      tc_mma_d(d, ah, bl, idesc, 1u);
+      tc_mma_d(d, ah, bh, idesc, 1u);
+    }
+  }
+}
+
 // Bounded wait that also gives up as soon as another role has aborted.
 __device__ __forceinline__ bool mbar_wait_or_abort(uint32_t bar, uint32_t parity, const volatile int *abort_flag) {
+  if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
-  while (true) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
+  while (!mbar_try(bar, parity)) {
     if (*abort_flag) return false;
     if (clock64() - t0 > TC_WAIT_CYCLES) return false;
   }
+  return true;
 }
 
 // Work unit u: false if the run is inactive or the chain tile has no pending proposal (the
@@ -194,31 +261,27 @@ __device__ __forceinline__ bool sr_unit(const gbns_batch &b, const gbns_lg_bufs 
 }
 
 __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constant__ SrMaps maps, gbns_batch b,
-                                                            gbns_lg_bufs lg, int nkb_max, int acc_stages) {
+                                                            gbns_lg_bufs lg, int nkb_max) {
   extern __shared__ unsigned char sr_dyn[];
-  // 0 w_full, 1 w_empty, 2-3 phi_full, 4-5 phi_empty, 6-9 acc_full, 10-13 acc_empty
-  __shared__ __align__(8) unsigned long long bars[14];
+  // 0 w_full, 1 w_empty, 2-3 phi_full, 4-5 phi_empty, 6-7 acc_full, 8-9 acc_empty
+  __shared__ __align__(8) unsigned long long bars[10];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
-  __shared__ float ys[4][SR_ROWS];
+  __shared__ __align__(16) float ys[8][SR_ROWS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = (smem_u32(sr_dyn) + 1023u) & ~1023u;
   const int NK = nkb_max;
   auto w_hi = [&](int kb) { return base + (uint32_t)kb * SR_BOX; };
   auto w_lo = [&](int kb) { return base + (uint32_t)(NK + kb) * SR_BOX; };
-  auto phi_hi = [&](int p, int kb) { return base + (uint32_t)(2 * NK + p * 2 * NK + kb) * SR_BOX; };
-  auto phi_lo = [&](int p, int kb) { return base + (uint32_t)(2 * NK + p * 2 * NK + NK + kb) * SR_BOX; };
+  auto phi_at = [&](int q, int lo) {
+    return base + (uint32_t)(2 * NK) * SR_BOX + (uint32_t)q * STAGE + (uint32_t)lo * 2u * SR_BOX;
+  };
   auto bar = [&](int q) { return smem_u32(&bars[q]); };
 
   pdl_launch_dependents();
   if (tid == 0) {
-    mbar_init(bar(0), 1);
-    mbar_init(bar(1), 1);
-    for (int q = 2; q < 6; ++q) mbar_init(bar(q), 1);
-    for (int q = 0; q < 4; ++q) {
-      mbar_init(bar(6 + q), 1);
-      mbar_init(bar(10 + q), 4);  // one arrival per epilogue warp
-    }
+    for (int q = 0; q < 8; ++q) mbar_init(bar(q), 1);
+    for (int q = 8; q < 10; ++q) mbar_init(bar(q), 8);  // one arrival per epilogue warp
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -226,7 +289,7 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
   __syncwarp();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "r"((uint32_t)(acc_stages * SR_ROWS))
+                 "r"(2u * MMA_ROWS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -239,7 +302,7 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
   pdl_wait_prior_grid();  // the chain step's proposals and tile marks
 
   if (warp == 0) {
-    // ---- producer: W tile per unit, Phi hi / lo per row tile (two stages)
+    // ---- producer: W tile per unit, Phi stages (two row tiles x one K block, two in flight)
     int wuse = 0, pt = 0;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
       int r, c0, rt0, nrt;
@@ -249,22 +312,22 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
       const int brow = (int)lg.row_base[r];
       int failed = 0;
       if (lane == 0) {
-        // Phi row tile t into the next stage (waits until the MMAs have released it)
-        auto load_phi = [&](int t) -> bool {
-          const int p = pt & 1;
-          if (!mbar_wait_or_abort(bar(4 + p), (uint32_t)(((pt >> 1) & 1) ^ 1), ab)) return false;
-          mbar_expect_tx(bar(2 + p), 2u * (uint32_t)nkb * SR_BOX);
-          const int y0 = brow + (rt0 + t) * SR_ROWS;
-          for (int kb = 0; kb < nkb; ++kb) {
-            tma_load_2d(phi_hi(p, kb), &maps.phi_hi, kb * TC_KB, y0, bar(2 + p));
-            tma_load_2d(phi_lo(p, kb), &maps.phi_lo, kb * TC_KB, y0, bar(2 + p));
+        // row tiles t, t + 1 of K block kb into the next stage (once the MMAs have released it)
+        auto load_phi = [&](int t, int kb) -> bool {
+          const int q = pt & 1, boxes = min(2, nrt - t);
+          if (!mbar_wait_or_abort(bar(4 + q), (uint32_t)(((pt >> 1) & 1) ^ 1), ab)) return false;
+          mbar_expect_tx(bar(2 + q), 2u * (uint32_t)boxes * SR_BOX);
+          for (int h = 0; h < boxes; ++h) {
+            const int y0 = brow + (rt0 + t + h) * SR_ROWS;
+            tma_load_2d(phi_at(q, 0) + h * SR_BOX, &maps.phi_hi, kb * TC_KB, y0, bar(2 + q));
+            tma_load_2d(phi_at(q, 1) + h * SR_BOX, &maps.phi_lo, kb * TC_KB, y0, bar(2 + q));
           }
           ++pt;
           return true;
         };
-        // the first Phi tile goes before the W tile, so it streams while the previous
+        // the first Phi stage goes before the W tile, so it streams while the previous
         // unit's last MMAs (which hold the W buffer) finish
-        if (!load_phi(0) || !mbar_wait_or_abort(bar(1), (uint32_t)((wuse & 1) ^ 1), ab)) {
+        if (!load_phi(0, 0) || !mbar_wait_or_abort(bar(1), (uint32_t)((wuse & 1) ^ 1), ab)) {
           failed = 1;
         } else {
           mbar_expect_tx(bar(0), 2u * (uint32_t)nkb * SR_BOX);
@@ -273,11 +336,12 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
             tma_load_2d(w_hi(kb), &maps.w_hi, kb * TC_KB, ar, bar(0));
             tma_load_2d(w_lo(kb), &maps.w_lo, kb * TC_KB, ar, bar(0));
           }
-          for (int t = 1; t < nrt; ++t)
-            if (!load_phi(t)) {
-              failed = 1;
-              break;
-            }
+          for (int t = 0; t < nrt && !failed; t += 2)
+            for (int kb = t == 0 ? 1 : 0; kb < nkb; ++kb)
+              if (!load_phi(t, kb)) {
+                failed = 1;
+                break;
+              }
         }
         if (failed) {
           abort_flag = 1;
@@ -295,31 +359,31 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
       int r, c0, rt0, nrt;
       if (!sr_unit(b, lg, u, lane, r, c0, rt0, nrt)) continue;
       const gbns_run_desc &rd = b.runs[r];
-      const int nk8 = (rd.D + 7) / 8;
+      const int nk8 = (rd.D + 7) / 8, nkb = (rd.D + TC_KB - 1) / TC_KB;
       int failed = 0;
       if (lane == 0) {
         if (!mbar_wait_or_abort(bar(0), (uint32_t)(wuse & 1), ab)) failed = 1;
-        for (int t = 0; t < nrt && !failed; ++t, ++pt, ++at) {
-          const int p = pt & 1, a = at % acc_stages;
-          if (!mbar_wait_or_abort(bar(2 + p), (uint32_t)((pt >> 1) & 1), ab) ||
-              !mbar_wait_or_abort(bar(10 + a), (uint32_t)(((at / acc_stages) & 1) ^ 1), ab)) {
+        for (int t = 0; t < nrt && !failed; t += 2, ++at) {
+          const int a = at & 1;
+          if (!mbar_wait_or_abort(bar(8 + a), (uint32_t)(((at >> 1) & 1) ^ 1), ab)) {
             failed = 1;
             break;
           }
-          tc_fence_after();
-          const uint32_t d = tmem + (uint32_t)(a * SR_ROWS);
-          for (int k8 = 0; k8 < nk8; ++k8) {
-            const int kb = k8 >> 2;
-            const uint32_t off = (uint32_t)(k8 & 3) * 32u;
-            const uint64_t ah = smem_desc(w_hi(kb) + off), al = smem_desc(w_lo(kb) + off);
-            const uint64_t bh = smem_desc(phi_hi(p, kb) + off), bl = smem_desc(phi_lo(p, kb) + off);
-            tc_mma_d(d, al, bh, SR_IDESC, k8 > 0 ? 1u : 0u);
-            tc_mma_d(d, ah, bl, SR_IDESC, 1u);
-            tc_mma_d(d, ah, bh, SR_IDESC, 1u);
+          const uint32_t idesc = nrt - t > 1 ? tc_idesc(MMA_ROWS) : tc_idesc(SR_ROWS);
+          for (int kb = 0; kb < nkb; ++kb, ++pt) {
+            const int q = pt & 1;
+            if (!mbar_wait_or_abort(bar(2 + q), (uint32_t)((pt >> 1) & 1), ab)) {
+              failed = 1;
+              break;
+            }
+            tc_fence_after();
+            tc_mma_block(tmem + (uint32_t)(a * MMA_ROWS), tc_operand(w_hi(kb), w_lo(kb)),
+                         tc_operand(phi_at(q, 0), phi_at(q, 1)), nk8 - 4 * kb, idesc, kb > 0 ? 1u : 0u);
+            tc_commit(bar(4 + q));  // Phi stage q free
           }
-          tc_commit(bar(6 + a));   // accumulator a full
-          tc_commit(bar(4 + p));   // Phi stage p free
-          if (t == nrt - 1) tc_commit(bar(1));  // W tile free
+          if (failed) break;
+          tc_commit(bar(6 + a));               // accumulator a full
+          if (t + 2 >= nrt) tc_commit(bar(1));  // W tile free
         }
         if (failed) {
           abort_flag = 1;
@@ -332,8 +396,8 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
       at = __shfl_sync(0xffffffffu, at, 0);
     }
   } else {
-    // ---- epilogue: warps 2-5 own tensor-memory lane quarters 2, 3, 0, 1
-    const int q = warp & 3, ew = warp - 2;
+    // ---- epilogue: a tensor-memory lane quarter and one of the two row tiles per warp
+    const int q = warp & 3, ew = warp - 2, half = ew >> 2;
     int at = 0;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
       int r, c0, rt0, nrt;
@@ -345,42 +409,49 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
       bool ok = true;
       // y of the next row tile is loaded into registers while the current one is processed
       float yn[4];
+      auto load_y = [&](int t) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int row = rt0 * SR_ROWS + lane + 32 * k;
-        yn[k] = row < N ? y[row] : 0.0f;
-      }
-      for (int t = 0; t < nrt; ++t, ++at) {
-        const int a = at % acc_stages;
-        const int row0 = (rt0 + t) * SR_ROWS;
-        const int nrows = min(SR_ROWS, N - row0);
+        for (int k = 0; k < 4; ++k) {
+          const int row = (rt0 + t) * SR_ROWS + lane + 32 * k;
+          yn[k] = t < nrt && row < N ? y[row] : 0.0f;
+        }
+      };
+      load_y(half);
+      for (int t = 0; t < nrt; t += 2, ++at) {
+        const int a = at & 1, tt = t + half;
+        const int nrows = tt < nrt ? min(SR_ROWS, N - (rt0 + tt) * SR_ROWS) : 0;
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 4; ++k) ys[ew][lane + 32 * k] = yn[k];
         __syncwarp();
-        if (t + 1 < nrt) {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int row = row0 + SR_ROWS + lane + 32 * k;
-            yn[k] = row < N ? y[row] : 0.0f;
-          }
-        }
-        ok = mbar_wait_or_abort(bar(6 + a), (uint32_t)((at / acc_stages) & 1), ab);
+        load_y(tt + 2);
+        ok = mbar_wait_or_abort(bar(6 + a), (uint32_t)((at >> 1) & 1), ab);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * SR_ROWS);
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * MMA_ROWS + half * SR_ROWS);
         const int nch = (nrows + 31) >> 5;
+        // the next 32 columns load while these are summed
         float part = 0.0f;
-        for (int ch = 0; ch < nch; ++ch) {
-          float v[32];
-          tc_ld32(taddr + (uint32_t)(ch * 32), v);
-          part += sq_resid32(&ys[ew][ch * 32], v, nrows - ch * 32);
+        uint32_t ra[32], rb[32];
+        if (nch > 0) {
+          tc_ld32_start(taddr, ra);
+          tc_ld32_finish(ra);
         }
-        ssum += (double)part;
+        if (nch > 1) tc_ld32_start(taddr + 32u, rb);
+        if (nch > 0) part += sq_resid32(&ys[ew][0], ra, nrows);
+        if (nch > 1) tc_ld32_finish(rb);
+        if (nch > 2) tc_ld32_start(taddr + 64u, ra);
+        if (nch > 1) part += sq_resid32(&ys[ew][32], rb, nrows - 32);
+        if (nch > 2) tc_ld32_finish(ra);
+        if (nch > 3) tc_ld32_start(taddr + 96u, rb);
+        if (nch > 2) part += sq_resid32(&ys[ew][64], ra, nrows - 64);
+        if (nch > 3) tc_ld32_finish(rb);
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(10 + a));  // accumulator a drained
+        if (lane == 0) mbar_arrive(bar(8 + a));  // accumulator a drained
+        if (nch > 3) part += sq_resid32(&ys[ew][96], rb, nrows - 96);
+        ssum += (double)part;
       }
       if (!ok) {
         if (lane == 0) {
@@ -390,16 +461,14 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
         break;
       }
       const int c = c0 + q * 32 + lane;
-      if (c < rd.s) atomicAdd(&lg.ss[rd.shell_off + c], ssum);
+      if (c < rd.s && half < nrt) atomicAdd(&lg.ss[rd.shell_off + c], ssum);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"((uint32_t)(acc_stages * SR_ROWS))
-                 : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * MMA_ROWS) : "memory");
   }
   // the last CTA to finish clears the pending-tile marks for the next chain step
   __shared__ int last;
@@ -413,7 +482,6 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
     if (tid == 0) *lg.tc_done = 0;
   }
 }
-
 
 // ------------------------------------------------------------------ fused shell
 //
@@ -473,16 +541,6 @@ __device__ __forceinline__ void lf_st_v4(uint32_t addr, uint4 v) {
 
 __device__ __forceinline__ void lf_st_f32x2(uint32_t addr, float a, float b) {
   asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
-}
-
-// hi + lo += x (TwoSum of hi and x, the rounding error carried in lo).  GB300 runs FP64 at
-// about 1/64 of the FP32 rate, so the step's sums of squares travel as fp32 pairs: each adds
-// at most a few units of 2^-48 of relative error, far below the fp32 rounding of the 32-row
-// chunk sums they carry.
-__device__ __forceinline__ void lf_pair_acc(float &hi, float &lo, float x) {
-  float e;
-  pair_add(hi, x, hi, e);
-  lo += e;
 }
 
 __device__ __forceinline__ void lf_st_s32(uint32_t addr, int v) {
@@ -814,16 +872,10 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
       tc_fence_after();
       for (int nc = 0; nc * NMMA < nbox * 128; ++nc) {
         const uint32_t d = tmem + (uint32_t)(nc * NMMA);
-        for (int k8 = 0; k8 < nk8; ++k8) {
-          const int kb = k8 >> 2;
-          const uint32_t koff = (uint32_t)(k8 & 3) * 32u;
-          const uint32_t wo = (uint32_t)kb * 16384u + koff;
-          const uint32_t po = (uint32_t)(kb * R * 128 + nc * NMMA * 128) + koff;
-          const uint64_t ah = smem_desc(w_hi + wo), al = smem_desc(w_lo + wo);
-          const uint64_t bh = smem_desc(phi_hi + po), bl = smem_desc(phi_lo + po);
-          tc_mma_d(d, al, bh, idesc, k8 > 0 ? 1u : 0u);
-          tc_mma_d(d, ah, bl, idesc, 1u);
-          tc_mma_d(d, ah, bh, idesc, 1u);
+        for (int kb = 0; 4 * kb < nk8; ++kb) {
+          const uint32_t wo = (uint32_t)kb * 16384u, po = (uint32_t)(kb * R * 128 + nc * NMMA * 128);
+          tc_mma_block(d, tc_operand(w_hi + wo, w_lo + wo), tc_operand(phi_hi + po, phi_lo + po), nk8 - 4 * kb, idesc,
+                       kb > 0 ? 1u : 0u);
         }
       }
       tc_commit(bar_mma);
@@ -843,8 +895,9 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
         const int cbeg = hs * cw, cend = min(cbeg + cw, nrows);
         const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16);
         for (int col = cbeg; col < cend; col += 32) {
-          float v[32];
-          tc_ld32(taddr + (uint32_t)col, v);
+          uint32_t v[32];
+          tc_ld32_start(taddr + (uint32_t)col, v);
+          tc_ld32_finish(v);
           lf_pair_acc(part, part_lo, sq_resid32(ys + col, v, cend - col));
         }
       }
@@ -877,46 +930,44 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
 // ------------------------------------------------------------------ adjoint
 //
 // All dead points against all data rows: sum r^2 and sum r y per point, r = y - Phi w.  Persistent and
-// warp-specialised, one CTA per SM; the 128-point x 128-row tiles, row tiles fastest, are dealt to
+// warp-specialised, one CTA per SM; the 128-point x 256-row tiles, row tiles fastest, are dealt to
 // the CTAs in equal consecutive ranges, so a CTA keeps a W tile while it walks its row tiles and no
-// wave is left partly empty.  Warp 0 streams W and Phi tiles (hi / lo) by TMA, warp 1 issues the
-// 3xTF32 MMAs into a ring of four 128-column accumulators, warps 2-5 and 6-9 drain alternate
-// tiles (thread = point): per 32 rows one fp32 chain for each sum, the chunks in FP64 registers,
-// added to the point's totals when the point tile changes.
-// Bound: the tensor pipe (a 128 x 128 x 32 tile is ~830 cycles of 3xTF32 MMAs) and the epilogue's
-// dependent FMA chains, 32 long, which two sets of warps hide.  40,000 points x 4096 rows x 32: one
-// tile per CTA (5,008 CTAs, copy, MMAs and epilogue in turn) 119 us; see launch_adjoint_tc.
+// wave is left partly empty.  Warp 0 streams W tiles and Phi stages (256 rows x one K block, hi / lo)
+// by TMA, warp 1 issues the 3xTF32 MMAs into two 256-column accumulators in turn, warps 2-5 and
+// 6-9 drain a column half each (thread = point): per 32 rows one fp32 chain for each sum, four
+// chunks as an fp32 pair, then FP64 registers, added to the point's totals when the point tile
+// changes.
+// Bound: the tensor pipe.  256 rows per MMA are what reaches it: 12 MMAs of 128 x 256 x 8 take
+// 1.66 k cycles, of 128 x 128 x 8 2.25 k for half the work (the 128-point operand is read again
+// for every one).  40,000 points x 4096 rows x 32: one tile per CTA (5,008 CTAs, copy, MMAs and
+// epilogue in turn) 119 us, persistent with 128-row MMAs 96 us, this 58 us (the MMAs alone: 29 us).
 struct AdjStages {
   int nkb;      // K blocks of 32 floats
   int w_bufs;   // W tiles in shared memory (2 at one K block, 1 at two)
-  int phi_bufs; // Phi tiles (4 / 2)
 };
 constexpr int ADJ_THREADS = 320;
-constexpr int ADJ_ACC = 4;
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_constant__ TcMaps maps, AdjStages sg, long long M,
                                                               int P, int N, const float *__restrict__ y, double *ss,
                                                               double *ry, int *status) {
   extern __shared__ unsigned char adj_dyn[];
-  // 0-1 w_full, 2-3 w_empty, 4-7 phi_full, 8-11 phi_empty, 12-15 acc_full, 16-19 acc_empty
-  __shared__ __align__(8) unsigned long long bars[20];
+  // 0-1 w_full, 2-3 w_empty, 4-5 phi_full, 6-7 phi_empty, 8-9 acc_full, 10-11 acc_empty
+  __shared__ __align__(8) unsigned long long bars[12];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   __shared__ __align__(16) float ys[8][SR_ROWS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t base = (smem_u32(adj_dyn) + 1023u) & ~1023u;
-  const int NK = sg.nkb, WB = sg.w_bufs, PB = sg.phi_bufs;
+  const int NK = sg.nkb, WB = sg.w_bufs;
   auto w_at = [&](int buf, int lo, int kb) { return base + (uint32_t)((buf * 2 + lo) * NK + kb) * SR_BOX; };
-  auto phi_at = [&](int buf, int lo, int kb) {
-    return base + (uint32_t)(2 * WB * NK + (buf * 2 + lo) * NK + kb) * SR_BOX;
-  };
+  auto phi_at = [&](int buf, int lo) { return base + (uint32_t)(2 * WB * NK) * SR_BOX + (uint32_t)buf * STAGE + (uint32_t)lo * 2u * SR_BOX; };
   auto bar = [&](int q) { return smem_u32(&bars[q]); };
-  const long long row_tiles = (N + SR_ROWS - 1) / SR_ROWS, tiles = ((M + TC_M - 1) / TC_M) * row_tiles;
+  const long long row_tiles = (N + MMA_ROWS - 1) / MMA_ROWS, tiles = ((M + TC_M - 1) / TC_M) * row_tiles;
   const long long t0 = tiles * blockIdx.x / gridDim.x, t1 = tiles * (blockIdx.x + 1) / gridDim.x;
 
   if (tid == 0) {
-    for (int q = 0; q < 16; ++q) mbar_init(bar(q), 1);
-    for (int q = 16; q < 20; ++q) mbar_init(bar(q), 4);  // one arrival per warp of the draining set
+    for (int q = 0; q < 10; ++q) mbar_init(bar(q), 1);
+    for (int q = 10; q < 12; ++q) mbar_init(bar(q), 8);  // one arrival per epilogue warp
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -924,7 +975,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
   __syncwarp();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                 "r"((uint32_t)(ADJ_ACC * SR_ROWS))
+                 "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -941,7 +992,6 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
       int wu = 0, issued = 0;
       for (long long t = t0; t < t1 && ok; ++t) {
         const long long p = t / row_tiles;
-        const int n = (int)(t - t0);
         if (p != pt) {
           const int q = wu % WB;
           ok = mbar_wait_or_abort(bar(2 + q), (uint32_t)(((wu / WB) & 1) ^ 1), ab);
@@ -954,21 +1004,24 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
           ++wu;
           pt = p;
         }
-        const int q = n % PB, r0 = (int)(t - p * row_tiles) * SR_ROWS;
-        ok = mbar_wait_or_abort(bar(8 + q), (uint32_t)(((n / PB) & 1) ^ 1), ab);
-        if (!ok) break;
-        mbar_expect_tx(bar(4 + q), 2u * (uint32_t)NK * SR_BOX);
-        for (int kb = 0; kb < NK; ++kb) {
-          tma_load_2d(phi_at(q, 0, kb), &maps.b_hi, kb * TC_KB, r0, bar(4 + q));
-          tma_load_2d(phi_at(q, 1, kb), &maps.b_lo, kb * TC_KB, r0, bar(4 + q));
+        const int r0 = (int)(t - p * row_tiles) * MMA_ROWS;
+        for (int kb = 0; kb < NK && ok; ++kb) {
+          const int q = issued & 1;
+          ok = mbar_wait_or_abort(bar(6 + q), (uint32_t)(((issued >> 1) & 1) ^ 1), ab);
+          if (!ok) break;
+          mbar_expect_tx(bar(4 + q), STAGE);
+          for (int h = 0; h < 2; ++h) {
+            tma_load_2d(phi_at(q, 0) + h * SR_BOX, &maps.b_hi, kb * TC_KB, r0 + h * SR_ROWS, bar(4 + q));
+            tma_load_2d(phi_at(q, 1) + h * SR_BOX, &maps.b_lo, kb * TC_KB, r0 + h * SR_ROWS, bar(4 + q));
+          }
+          ++issued;
         }
-        ++issued;
       }
       if (!ok) {
         abort_flag = 1;
         atomicOr(status, (int)GBNS_ERR_WAIT_TIMEOUT);
         // copies still in flight get one more bounded wait
-        for (int i = issued > PB ? issued - PB : 0; i < issued; ++i) mbar_wait(bar(4 + i % PB), (uint32_t)((i / PB) & 1));
+        for (int i = issued > 2 ? issued - 2 : 0; i < issued; ++i) mbar_wait(bar(4 + (i & 1)), (uint32_t)((i >> 1) & 1));
         for (int i = wu > WB ? wu - WB : 0; i < wu; ++i) mbar_wait(bar(i % WB), (uint32_t)((i / WB) & 1));
       }
     }
@@ -978,32 +1031,28 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
       const int nk8 = (P + 7) / 8;
       bool ok = true;
       long long pt = -1;
-      int wu = -1;
-      for (long long t = t0; t < t1; ++t) {
+      int wu = -1, used = 0;
+      for (long long t = t0; t < t1 && ok; ++t) {
         const long long p = t / row_tiles;
-        const int n = (int)(t - t0), q = n % PB, a = n % ADJ_ACC;
+        const int n = (int)(t - t0), a = n & 1;
         if (p != pt) {
           ++wu;
           pt = p;
           ok = mbar_wait_or_abort(bar(wu % WB), (uint32_t)((wu / WB) & 1), ab);
         }
-        ok = ok && mbar_wait_or_abort(bar(4 + q), (uint32_t)((n / PB) & 1), ab) &&
-             mbar_wait_or_abort(bar(16 + a), (uint32_t)(((n / ADJ_ACC) & 1) ^ 1), ab);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(a * SR_ROWS);
+        ok = ok && mbar_wait_or_abort(bar(10 + a), (uint32_t)(((n >> 1) & 1) ^ 1), ab);
         const int wb = wu % WB;
-        for (int k8 = 0; k8 < nk8; ++k8) {
-          const int kb = k8 >> 2;
-          const uint32_t off = (uint32_t)(k8 & 3) * 32u;
-          const uint64_t ah = smem_desc(w_at(wb, 0, kb) + off), al = smem_desc(w_at(wb, 1, kb) + off);
-          const uint64_t bh = smem_desc(phi_at(q, 0, kb) + off), bl = smem_desc(phi_at(q, 1, kb) + off);
-          tc_mma_d(d, al, bh, SR_IDESC, k8 > 0 ? 1u : 0u);
-          tc_mma_d(d, ah, bl, SR_IDESC, 1u);
-          tc_mma_d(d, ah, bh, SR_IDESC, 1u);
+        for (int kb = 0; kb < NK && ok; ++kb, ++used) {
+          const int q = used & 1;
+          ok = mbar_wait_or_abort(bar(4 + q), (uint32_t)((used >> 1) & 1), ab);
+          if (!ok) break;
+          tc_fence_after();
+          tc_mma_block(tmem + (uint32_t)(a * MMA_ROWS), tc_operand(w_at(wb, 0, kb), w_at(wb, 1, kb)),
+                       tc_operand(phi_at(q, 0), phi_at(q, 1)), nk8 - 4 * kb, tc_idesc(MMA_ROWS), kb > 0 ? 1u : 0u);
+          tc_commit(bar(6 + q));  // Phi stage q free
         }
-        tc_commit(bar(12 + a));  // accumulator a full
-        tc_commit(bar(8 + q));   // Phi buffer q free
+        if (!ok) break;
+        tc_commit(bar(8 + a));  // accumulator a full
         if (t + 1 == t1 || (t + 1) / row_tiles != p) tc_commit(bar(2 + wb));  // W buffer free
       }
       if (!ok) {
@@ -1013,43 +1062,37 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
     }
     __syncwarp();
   } else {
-    // ---- epilogue: set 0 (warps 2-5) drains the range's even tiles, set 1 (warps 6-9) the odd ones
-    const int set = (warp - 2) >> 2, qd = warp & 3, ew = warp - 2;
+    // ---- epilogue: a lane quarter and a column half per warp
+    const int half = (warp - 2) >> 2, qd = warp & 3, ew = warp - 2;
     double s1 = 0.0, s2 = 0.0;
     bool ok = true;
-    // y of the set's next tile is loaded into registers while the current one is processed
+    // y of the next tile is loaded into registers while the current one is processed
     float yn[4];
     auto load_y = [&](long long t) {
-      const int r0 = (int)(t % row_tiles) * SR_ROWS;
+      const int r0 = (int)(t % row_tiles) * MMA_ROWS + half * SR_ROWS;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int row = r0 + lane + 32 * k;
         yn[k] = t < t1 && row < N ? y[row] : 0.0f;
       }
     };
-    load_y(t0 + set);
-    for (long long t = t0 + set; t < t1; t += 2) {
+    load_y(t0);
+    for (long long t = t0; t < t1; ++t) {
       const long long p = t / row_tiles;
-      const int n = (int)(t - t0), a = n % ADJ_ACC;
+      const int n = (int)(t - t0), a = n & 1;
       __syncwarp();
 #pragma unroll
       for (int k = 0; k < 4; ++k) ys[ew][lane + 32 * k] = yn[k];
       __syncwarp();
-      load_y(t + 2);
-      ok = mbar_wait_or_abort(bar(12 + a), (uint32_t)((n / ADJ_ACC) & 1), ab);
+      load_y(t + 1);
+      ok = mbar_wait_or_abort(bar(8 + a), (uint32_t)((n >> 1) & 1), ab);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(a * SR_ROWS);
-#pragma unroll 1
-      for (int ch = 0; ch < 4; ++ch) {
-        float v[32];
-        tc_ld32(taddr + (uint32_t)(ch * 32), v);
-        if (ch == 3) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(16 + a));  // accumulator a drained
-        }
+      const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(a * MMA_ROWS + half * SR_ROWS);
+      // the next 32 columns load while these are used; the four chunk sums as fp32 pairs
+      float h1 = 0.0f, l1 = 0.0f, h2 = 0.0f, l2 = 0.0f;
+      auto chunk = [&](uint32_t (&r)[32], int ch) {
         // rows past the last data row have y = 0 and a zero product: they add nothing
         float p1 = 0.0f, p2 = 0.0f;
 #pragma unroll
@@ -1058,15 +1101,35 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
           const float yv[4] = {yy.x, yy.y, yy.z, yy.w};
 #pragma unroll
           for (int x = 0; x < 4; ++x) {
-            const float rr = yv[x] - v[j + x];
+            const float rr = yv[x] - __uint_as_float(r[j + x]);
             p1 = fmaf(rr, rr, p1);
             p2 = fmaf(rr, yv[x], p2);
           }
         }
-        s1 += (double)p1;
-        s2 += (double)p2;
-      }
-      if (t + 2 >= t1 || (t + 2) / row_tiles != p) {
+        lf_pair_acc(h1, l1, p1);
+        lf_pair_acc(h2, l2, p2);
+      };
+      uint32_t ra[32], rb[32];
+      tc_ld32_start(taddr, ra);
+      tc_ld32_finish(ra);
+      tc_ld32_start(taddr + 32u, rb);
+      chunk(ra, 0);
+      tc_ld32_finish(rb);
+      tc_ld32_start(taddr + 64u, ra);
+      chunk(rb, 1);
+      tc_ld32_finish(ra);
+      tc_ld32_start(taddr + 96u, rb);
+      chunk(ra, 2);
+      tc_ld32_finish(rb);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(10 + a));  // accumulator a drained
+      chunk(rb, 3);
+      s1 += (double)h1;
+      s2 += (double)h2;
+      s1 += (double)l1;
+      s2 += (double)l2;
+      if (t + 1 == t1 || (t + 1) / row_tiles != p) {
         const long long pnt = p * TC_M + qd * 32 + lane;
         if (pnt < M) {
           atomicAdd(&ss[pnt], s1);
@@ -1084,7 +1147,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(ADJ_ACC * SR_ROWS))
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
                  : "memory");
   }
 }
@@ -1208,15 +1271,14 @@ cudaError_t launch_lg_steps_tc(const gbns_batch &b, const gbns_lg_bufs &lg, int 
       !encode_rows(&maps.phi_hi, lg.Phi_hi, lg.total_rows, 64, 128) ||
       !encode_rows(&maps.phi_lo, lg.Phi_lo, lg.total_rows, 64, 128))
     return cudaErrorInvalidValue;
-  // shared memory: W tile + two Phi stages, hi and lo, nkb K blocks each (96 KB per block);
-  // tensor memory: 4 accumulators of 128 columns at one CTA per SM, 2 at two CTAs per SM
+  // shared memory: W tile (hi and lo, nkb K blocks) and two Phi stages; tensor memory: two
+  // accumulators of 256 columns; so one CTA per SM
   const int nkb = lg.pmax > TC_KB ? 2 : 1;
-  const unsigned smem = (unsigned)nkb * 6u * SR_BOX + 1024u;
-  const int per_sm = nkb == 1 ? 2 : 1, acc_stages = nkb == 1 ? 2 : 4;
+  const unsigned smem = (unsigned)nkb * 2u * SR_BOX + 2u * STAGE + 1024u;
   int dev = 0, sms = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  int grid = sms * per_sm;
+  int grid = sms;
   if (lg.num_ctas_tc > 0 && lg.num_ctas_tc < grid) grid = lg.num_ctas_tc;
   if (grid > lg.num_items_tc) grid = lg.num_items_tc;
   const int launches = steps < 0 ? 1 : steps;
@@ -1235,7 +1297,7 @@ cudaError_t launch_lg_steps_tc(const gbns_batch &b, const gbns_lg_bufs &lg, int 
       attr[0].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
-      if ((e = cudaLaunchKernelEx(&cfg, k_lg_resid_tc, maps, b, lg, nkb, acc_stages)) != cudaSuccess) return e;
+      if ((e = cudaLaunchKernelEx(&cfg, k_lg_resid_tc, maps, b, lg, nkb)) != cudaSuccess) return e;
     }
   }
   return cudaGetLastError();
@@ -1325,8 +1387,8 @@ cudaError_t launch_adjoint_tc(const double *U, const double *log_w, long long M,
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const long long tiles = ((M + TC_M - 1) / TC_M) * ((N + SR_ROWS - 1) / SR_ROWS);
-    const AdjStages sg = {ld / TC_KB, ld == TC_KB ? 2 : 1, ld == TC_KB ? 4 : 2};
+    const long long tiles = ((M + TC_M - 1) / TC_M) * ((N + MMA_ROWS - 1) / MMA_ROWS);
+    const AdjStages sg = {ld / TC_KB, ld == TC_KB ? 2 : 1};
     k_adj_resid_tc<<<(unsigned)(tiles < sms ? tiles : sms), ADJ_THREADS, 12 * SR_BOX + 1024, s>>>(maps, sg, M, P, N, y, ss,
                                                                                              ry, status);
   }

@@ -400,11 +400,12 @@ class NSBatch:
             row_base = np.concatenate([[0], np.cumsum(Ns)[:-1]]).astype(np.int64)
             rows = int(Ns.sum())
             # work units (run, 128-chain tile, first 128-row tile, row tiles): row ranges sized so
-            # that there are about two units per CTA slot; the chain tiles of one row range are
-            # adjacent, so the CTAs that share its Phi tiles run together
+            # that there are about four units per CTA, an even number of tiles (the residual kernel
+            # multiplies two at a time); the chain tiles of one row range are adjacent, so the CTAs
+            # that share its Phi tiles run together
             tiles = [((s.shell_size + 127) // 128, (s.N + 127) // 128) for s in specs]
             work = sum(ct * rt for ct, rt in tiles)
-            rs = max(1, min(16, work // (2 * 2 * 152)))
+            rs = max(2, min(16, (work // (4 * 152) + 1) // 2 * 2))
             items_tc = [(r, c0, rt0, min(rs, rt - rt0)) for r, (ct, rt) in enumerate(tiles)
                         for rt0 in range(0, rt, rs) for c0 in range(0, ct * 128, 128)]
             self.lg_tc_t = dict(W_hi=z(nc * 64), W_lo=z(nc * 64), Phi_hi=z(rows * 64), Phi_lo=z(rows * 64),
