@@ -117,24 +117,21 @@ def batch_evidence_and_grad(batch, results, thetas, tensor_cores: bool = True, c
 
 class EvidenceFn(torch.autograd.Function):
     """log Z(theta) of a fixed dead set as a differentiable function of theta = (log tau, log sigma).
-    The backward pass recomputes the per-point likelihood gradients (nothing per point is
-    stored by the forward pass)."""
+    The pass over the dead points gives the value and the gradient together, so the backward pass
+    only scales the two saved numbers (nothing per point is stored)."""
 
     @staticmethod
     def forward(ctx, theta: torch.Tensor, ds: DeadSet):
         th = theta.detach().to(torch.float64).cpu().numpy()
         out = evidence_and_grad(ds, th[0], th[1])
-        ctx.ds = ds
-        ctx.save_for_backward(theta)
+        # theta too: autograd then refuses a theta that was changed in place before the backward pass
+        ctx.save_for_backward(theta, out[1:])
         return out[0].to(device=theta.device, dtype=theta.dtype)
 
     @staticmethod
     def backward(ctx, grad_out):
-        (theta,) = ctx.saved_tensors
-        th = theta.detach().to(torch.float64).cpu().numpy()
-        out = evidence_and_grad(ctx.ds, th[0], th[1])
-        g = out[1:].to(device=theta.device, dtype=theta.dtype)
-        return grad_out.to(theta.device) * g, None
+        theta, grad = ctx.saved_tensors
+        return grad_out.to(theta.device) * grad.to(device=theta.device, dtype=theta.dtype), None
 
 
 def blr_log_evidence(Phi, y, log_tau, log_sigma):
