@@ -6,10 +6,13 @@
 // N+1 node log-likelihoods.  Dead points are appended in non-decreasing order except for
 // phantoms and rejection-sampler caps, so the CTA first tests sortedness and only runs the
 // LSD radix sort (4 x 8-bit digits, stable by construction) when it is needed.
+#include <cooperative_groups.h>
 #include "gbns_device.cuh"
 #include "gbns_launch.h"
 
 namespace gbns {
+
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ unsigned long long node_key(const float *L, long long i) {
   // node 0 is the root at -inf; node i+1 is sample i
@@ -405,87 +408,294 @@ __global__ void k_rng(int mode, const uint32_t *key, const uint32_t *counts, voi
 }
 
 // sample_evidence (utils.py:433-484): S replicas of log Z with the shrinkage drawn.
-// Replica s (one CTA): u_i = uniform(split(split(key, S)[s], M)[i]), log T_i = log(u_i) / n_i,
-// log X_i = sum_{j<i} log T_j (FP64 block scan), and log Z = logsumexp_i(log X_i +
-// log(1 - T_i) + log L_i) -- the sequential LogSpace accumulation of the reference written
-// as a prefix sum and one log-sum-exp.
-__global__ void __launch_bounds__(1024) k_sample_evidence(const uint32_t *key, const int *__restrict__ num_live,
-                                                          const double *__restrict__ log_L, long long M,
+// Replica s: u_i = uniform(split(split(key, S)[s], M)[i]), log T_i = log(u_i) / n_i,
+// log X_i = sum_{j<i} log T_j, and log Z = log sum_i X_i (1 - T_i) L_i -- the sequential LogSpace
+// accumulation of the reference as a composition of ranges: a range has the sum of its log T and
+// the log of its sum started at X = 1, and (s1, v1) before (s2, v2) is (s1 + s2, logaddexp(v1,
+// s1 + v2)).
+// A cluster of CS blocks takes RG replicas, block q the q-th part of the samples; a thread takes up
+// to SE_K consecutive samples of its tile and walks them once per replica in linear space from X = 1,
+// with the samples' 1 / n and exp(L - the thread's largest L) formed once for all replicas:
+// -expm1(log T) = 1 - T keeps its relative precision, X T = X + X expm1(log T).  Threads are composed
+// by a block scan of the log T sums and one log-sum-exp, tiles in order, blocks through distributed
+// shared memory.
+// Bound: FP64 (~2 lanes per clock and SM): one logarithm, a degree-8 Taylor polynomial of expm1
+// where |log T| < 1/32 (the function elsewhere) and five multiply-adds per sample and replica, ~45
+// instructions; one block per replica with a scan, a division, two exponentials and two
+// logarithms per sample took ~130 and left 52 of 152 SMs idle at S = 100 (100 replicas of 22,000
+// samples 835 -> 396 us a call, results to the last bits).
+constexpr int SE_T = 256;
+constexpr int SE_K = 16;
+
+struct SeSmem {
+  double scan[SE_T / 32], red[32];
+  double part_s[4], part_v[4];  // this block's (sum of log T, log of the range's sum) per replica
+};
+
+__device__ __forceinline__ double lae_fin(double a, double b) {  // logaddexp for values in [-inf, +inf)
+  const double m = fmax(a, b);
+  return m > -INFINITY ? m + log(exp(a - m) + exp(b - m)) : a + b;  // NaN stays NaN
+}
+
+// expm1(x), x <= 0
+__device__ __forceinline__ double se_expm1(double x) {
+  if (fabs(x) < 0.03125) {
+    double p = 1.0 / 40320.0;
+    p = fma(p, x, 1.0 / 5040.0);
+    p = fma(p, x, 1.0 / 720.0);
+    p = fma(p, x, 1.0 / 120.0);
+    p = fma(p, x, 1.0 / 24.0);
+    p = fma(p, x, 1.0 / 6.0);
+    p = fma(p, x, 0.5);
+    return fma(p * x, x, x);
+  }
+  return expm1(x);
+}
+
+template <int RG>
+__global__ void __launch_bounds__(SE_T) k_sample_evidence(const uint32_t *key, const int *__restrict__ num_live,
+                                                          const double *__restrict__ log_L, long long M, int S, int CS,
                                                           double *__restrict__ out) {
-  __shared__ double wsum[32];
-  __shared__ double red_m[32], red_s[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const Key ks = fold(Key{key[0], key[1]}, (uint32_t)blockIdx.x);
-  double carry = 0.0;                  // log X at the start of the chunk
-  double m = -INFINITY, acc = 0.0;     // this thread's running log-sum-exp: m + log(acc)
-  for (long long base = 0; base < M; base += blockDim.x) {
-    const long long i = base + tid;
-    double lt = 0.0;
-    if (i < M) lt = log(uniform01_d(bits64(fold(ks, (uint32_t)i), 0u))) / (double)num_live[i];
-    // inclusive scan of lt over the block
-    double v = lt;
+  extern __shared__ __align__(16) double2 se_dyn[];  // [SE_K][SE_T]: 1 / n and exp(L - ref) of the thread's samples
+  __shared__ SeSmem sm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = SE_T / 32;
+  const int rank = blockIdx.x % CS, s0 = blockIdx.x / CS * RG;
+  const Key kroot = {key[0], key[1]};
+  const long long lo = M * rank / CS, hi = M * (rank + 1) / CS;
+  double run_s[RG], run_v[RG];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double t = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += t;
+  for (int g = 0; g < RG; ++g) {
+    run_s[g] = 0.0;
+    run_v[g] = -INFINITY;
+  }
+  for (long long base = lo; base < hi; base += (long long)SE_T * SE_K) {
+    const int len = (int)min((long long)SE_T * SE_K, hi - base), per = (len + SE_T - 1) / SE_T;
+    const long long i0 = base + min(len, tid * per);
+    const int cnt = (int)(min((long long)base + len, i0 + per) - i0);
+    double ref = -INFINITY;
+    for (int k = 0; k < cnt; ++k) ref = fmax(ref, log_L[i0 + k]);
+    for (int k = 0; k < cnt; ++k) {
+      const double L = log_L[i0 + k];
+      // a sample at -inf (or NaN, as a comparison with it would have it) adds nothing
+      const double e = L == ref ? 1.0 : (L > -INFINITY ? exp(L - ref) : 0.0);
+      se_dyn[k * SE_T + tid] = make_double2(1.0 / (double)num_live[i0 + k], ref > -INFINITY ? e : 0.0);
     }
-    if (lane == 31) wsum[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-      double w = lane < nw ? wsum[lane] : 0.0;
+#pragma unroll 1
+    for (int g = 0; g < RG; ++g) {
+      const Key ks = fold(kroot, (uint32_t)(s0 + g));
+      double X = 1.0, A = 0.0, sum = 0.0;
+      for (int k = 0; k < cnt; ++k) {
+        const double2 f = se_dyn[k * SE_T + tid];
+        const double lt = log(uniform01_d(bits64(fold(ks, (uint32_t)(i0 + k)), 0u))) * f.x;
+        const double em = se_expm1(lt);  // T - 1
+        const double d = X * em;
+        if (__double2hiint(lt) < 0) A = fma(-d, f.y, A);  // T > 1 (a negative count): 1 - T has no log
+        X += d;
+        sum += lt;
+      }
+      const double v = A > 0.0 ? ref + log(A) : -INFINITY;
+      // log X at this thread's first sample: exclusive block scan of the sums
+      double incl = sum;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const double t = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += t;
+        const double t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
       }
-      if (lane < nw) wsum[lane] = w;
-    }
-    __syncthreads();
-    const double before = (warp > 0 ? wsum[warp - 1] : 0.0) + (v - lt);  // exclusive prefix in the chunk
-    const double total = wsum[nw - 1];
-    if (i < M) {
-      // X_i (1 - T_i) L_i; T_i = 1 only if u_i rounds to 1, which the 52-bit uniform cannot
-      const double term = (carry + before) + log1p(-exp(lt)) + log_L[i];
-      if (term > m) {
-        acc = acc * exp(m - term) + 1.0;
-        m = term;
-      } else if (term > -INFINITY) {
-        acc += exp(term - m);
+      if (lane == 31) sm.scan[warp] = incl;
+      __syncthreads();
+      double before = run_s[g], total = run_s[g];
+      for (int w = 0; w < nw; ++w) {
+        if (w < warp) before += sm.scan[w];
+        total += sm.scan[w];
       }
+      const double prev = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (lane > 0) before += prev;
+      const double term = v > -INFINITY ? before + v : -INFINITY;
+      double mx = term;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (lane == 0) sm.red[warp] = mx;
+      __syncthreads();
+      mx = sm.red[0];
+      for (int w = 1; w < nw; ++w) mx = fmax(mx, sm.red[w]);
+      double a = term > -INFINITY ? exp(term - mx) : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      __syncthreads();
+      if (lane == 0) sm.red[warp] = a;
+      __syncthreads();
+      if (tid == 0) {
+        double sa = 0.0;
+        for (int w = 0; w < nw; ++w) sa += sm.red[w];
+        sm.part_v[g] = mx > -INFINITY ? lae_fin(run_v[g], mx + log(sa)) : run_v[g];
+      }
+      __syncthreads();
+      // (all run_s, run_v have a static index only after unrolling: select)
+#pragma unroll
+      for (int q = 0; q < RG; ++q)
+        if (q == g) {
+          run_s[q] = total;
+          run_v[q] = sm.part_v[g];
+        }
     }
-    carry += total;
-    __syncthreads();
   }
-  // combine the threads' (m, acc)
-  double gm = m;
+  if (tid == 0)
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) gm = fmax(gm, __shfl_xor_sync(0xffffffffu, gm, o));
-  if (lane == 0) red_m[warp] = gm;
-  __syncthreads();
-  gm = -INFINITY;
-  for (int q = 0; q < nw; ++q) gm = fmax(gm, red_m[q]);
-  double a = (m > -INFINITY) ? acc * exp(m - gm) : 0.0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if (lane == 0) red_s[warp] = a;
-  __syncthreads();
-  if (tid == 0) {
-    double sum = 0.0;
-    for (int q = 0; q < nw; ++q) sum += red_s[q];
-    out[blockIdx.x] = (gm > -INFINITY) ? gm + log(sum) : -INFINITY;
+    for (int g = 0; g < RG; ++g) {
+      sm.part_s[g] = run_s[g];
+      sm.part_v[g] = run_v[g];
+    }
+  if (CS > 1) {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (rank == 0 && tid < RG && tid < S - s0) {
+      double s = 0.0, v = -INFINITY;
+      for (int q = 0; q < CS; ++q) {
+        const SeSmem *o = cluster.map_shared_rank(&sm, q);
+        v = lae_fin(v, s + o->part_v[tid]);
+        s += o->part_s[tid];
+      }
+      out[s0 + tid] = v;
+    }
+    cluster.sync();
+  } else {
+    __syncthreads();
+    if (tid < RG && tid < S - s0) out[s0 + tid] = sm.part_v[tid];
   }
 }
 
 // ------------------------------------------------------- prior transform ----
 
 // Model.transform and Model.log_prob_prior (framework/model.py:155-187) over the sorted samples
-// of _to_results (sharded_static.py:744-745), FP64: one warp per sample row, dimensions strided
-// over the lanes (coalesced row reads).  Uniform q = a + b u, Normal q = a + b Phi^-1(u) (AS 241
-// PPND16); with an affine map, X_d = c_d + sum_{k = row_start_d}^{d} A_dk q_k over q staged in
-// shared memory (the MultivariateNormalTriL blocks), else X = q.  The density is each
-// dimension's constant plus -z^2 / 2 (Normal) or 0 / -inf (Uniform, inside / outside), summed
-// per lane in dimension order and then over the warp by the xor butterfly, plus log_det and,
-// when given, log L (the log posterior density).
+// of _to_results (sharded_static.py:744-745), FP64.  Uniform q = a + b u, Normal q = a + b Phi^-1(u)
+// (AS 241 PPND16); with an affine map, X_d = c_d + sum_{k = row_start_d}^{d} A_dk q_k (the
+// MultivariateNormalTriL blocks), else X = q.  The density is each dimension's constant plus
+// -z^2 / 2 (Normal) or 0 / -inf (Uniform, inside / outside), added in the order of one warp per
+// row, dimensions strided over its lanes, then the xor butterfly; plus log_det and, when given,
+// log L (the log posterior density).
+//
+// A warp takes a tile of PT_E x 32 elements: PT_E sets of 32 / GW rows for D <= 32 (GW lanes, the
+// next power of two, per row: the butterfly's other lanes would hold zeros), else the PT_E / spr
+// rows that fill it with spr = ceil(D / 32) elements per lane.
+// Bound: FP64 (~2 lanes per clock and SM), so every lane carries an element and the quantile's two
+// branches do not both run for every 32 of them: central quantiles (85 % of uniform draws) at once,
+// the others collected in a queue over the whole tile and done 32 at a time.  500,000 rows at D = 8
+// with an 8 x 8 map: one warp per row (8 of 32 lanes, both branches) 2.98 ms, tiles 0.54 ms, the
+// same bits.
+constexpr int PT_E = 4;
+constexpr int PT_WARPS = 8;
+
+struct PtWarp {
+  double z[32 * PT_E];           // u, then z (Normal) of the tile's elements, then q
+  unsigned char queue[32 * PT_E];
+};
+
+template <typename UT>
+__global__ void __launch_bounds__(32 * PT_WARPS) k_prior_tiles(gbns_prior_table t, const UT *__restrict__ U, long long M,
+                                                               const double *__restrict__ log_L, double *__restrict__ X,
+                                                               double *__restrict__ out) {
+  extern __shared__ __align__(16) double pt_dyn[];  // A transposed (staged when D <= 64)
+  __shared__ PtWarp warps[PT_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int D = t.D;
+  PtWarp &W = warps[warp];
+  const bool staged = t.A && D <= 64;
+  if (staged) {
+    for (int q = threadIdx.x; q < D * D; q += 32 * PT_WARPS) pt_dyn[q % D * D + q / D] = t.A[q];
+    __syncthreads();
+  }
+  const double *Am = staged ? pt_dyn : t.A;
+  const int row_step = staged ? 1 : D, col_step = staged ? D : 1;
+  int GW = 32;
+  while (GW / 2 >= D) GW /= 2;
+  const int spr = (D + 31) / 32;                       // elements per lane and row (1, 2, 3 or 4)
+  const int rows_per_set = D <= 32 ? 32 / GW : 1;
+  const int sets = PT_E / spr, rows_per_tile = rows_per_set * sets;
+  const int sub = lane / GW, dl = lane % GW;           // row of the set, dimension (D <= 32)
+  const long long tiles = (M + rows_per_tile - 1) / rows_per_tile;
+  for (long long tile = (long long)blockIdx.x * PT_WARPS + warp; tile < tiles; tile += (long long)gridDim.x * PT_WARPS) {
+    const long long row0 = tile * rows_per_tile;
+    auto place = [&](int e, long long &row, int &d) {  // element e of this lane
+      if (D <= 32) {
+        row = row0 + (long long)e * rows_per_set + sub;
+        d = dl;
+      } else {
+        row = row0 + e / spr;
+        d = lane + 32 * (e % spr);
+      }
+      return row < M && d < D;
+    };
+    int queued = 0;
+#pragma unroll 1
+    for (int e = 0; e < sets * spr; ++e) {
+      long long row;
+      int d;
+      const bool have = place(e, row, d);
+      double u = have ? (double)U[row * D + d] : 0.5;
+      const bool normal = have && t.kind[d] == GBNS_PRIOR_NORMAL;
+      const bool tail = normal && !(fabs(u - 0.5) <= 0.425);
+      if (normal && !tail) u = gbns_fm_ndtri64(u);
+      W.z[e * 32 + lane] = u;
+      const unsigned m = __ballot_sync(0xffffffffu, tail);
+      if (tail) W.queue[queued + __popc(m & ((1u << lane) - 1u))] = (unsigned char)(e * 32 + lane);
+      queued += __popc(m);
+    }
+    __syncwarp();
+    for (int i = lane; i < queued; i += 32) {
+      const int at = W.queue[i];
+      W.z[at] = gbns_fm_ndtri64(W.z[at]);
+    }
+    __syncwarp();
+    double lp = 0.0;
+#pragma unroll 1
+    for (int e = 0; e < sets * spr; ++e) {
+      long long row;
+      int d;
+      const bool have = place(e, row, d);
+      if (e % spr == 0) lp = 0.0;
+      if (have) {
+        const double v = W.z[e * 32 + lane], a = t.a[d], b = t.b[d];
+        double q, ld;
+        q = fma(b, v, a);
+        if (t.kind[d] == GBNS_PRIOR_NORMAL) ld = fma(-0.5 * v, v, t.log_norm[d]);
+        else ld = (q >= a && q <= a + b) ? t.log_norm[d] : -INFINITY;
+        lp += ld;
+        if (t.A) W.z[e * 32 + lane] = q;
+        else if (X) X[row * D + d] = q;
+      }
+      if (e % spr == spr - 1) {
+        double sum = lp;
+        for (int m = GW / 2; m >= 1; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        // the row's first lane (its own row: valid when d = 0 is)
+        const long long r = D <= 32 ? row : row0 + e / spr;
+        if ((D <= 32 ? dl : lane) == 0 && r < M && out) out[r] = (log_L ? log_L[r] : 0.0) + (sum + t.log_det);
+      }
+    }
+    if (t.A) {
+      __syncwarp();
+      if (X) {
+#pragma unroll 1
+        for (int e = 0; e < sets * spr; ++e) {
+          long long row;
+          int d;
+          if (place(e, row, d)) {
+            // q_k of the row: lane group start + k (D <= 32), or element k / 32 of lane k % 32
+            const double *a_row = Am + d * row_step;
+            const double *q = &W.z[D <= 32 ? e * 32 + sub * GW : (e / spr) * spr * 32];
+            double acc = t.c[d];
+            const int k0 = t.row_start[d] > 0 ? t.row_start[d] : 0;  // k stays in [0, d]
+            for (int k = k0; k <= d; ++k) acc = fma(a_row[k * col_step], q[k], acc);
+            X[row * D + d] = acc;
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// The same for D > 32 PT_E, where a row alone fills a warp's tile: one warp per row, dimensions
+// strided over the lanes.
 template <typename UT>
 __global__ void __launch_bounds__(256) k_prior_transform(gbns_prior_table t, const UT *U, long long M,
                                                          const double *log_L, double *X, double *out) {
@@ -536,11 +746,31 @@ __global__ void __launch_bounds__(256) k_prior_transform(gbns_prior_table t, con
 cudaError_t launch_prior_transform(const gbns_prior_table &t, const float *U32, const double *U64, long long M,
                                    const double *log_L, double *X, double *out, cudaStream_t stream) {
   if (M <= 0) return cudaSuccess;
-  const size_t smem = t.A ? (size_t)8 * t.D * sizeof(double) : 0;
   int dev = 0, sms = 0;
   cudaError_t e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  if (t.D <= 32 * PT_E) {
+    int GW = 32;
+    while (GW / 2 >= t.D) GW /= 2;
+    const int rows = t.D <= 32 ? PT_E * 32 / GW : PT_E / ((t.D + 31) / 32);
+    const long long tiles = (M + rows - 1) / rows, want = (tiles + PT_WARPS - 1) / PT_WARPS;
+    const unsigned grid = (unsigned)(want < (long long)sms * 4 ? want : (long long)sms * 4);
+    const size_t smem = t.A && t.D <= 64 ? (size_t)t.D * t.D * sizeof(double) : 0;
+    if (U32) {
+      if (smem > 16 * 1024 && (e = cudaFuncSetAttribute(k_prior_tiles<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)smem)) != cudaSuccess)
+        return e;
+      k_prior_tiles<float><<<grid, 32 * PT_WARPS, smem, stream>>>(t, U32, M, log_L, X, out);
+    } else {
+      if (smem > 16 * 1024 && (e = cudaFuncSetAttribute(k_prior_tiles<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)smem)) != cudaSuccess)
+        return e;
+      k_prior_tiles<double><<<grid, 32 * PT_WARPS, smem, stream>>>(t, U64, M, log_L, X, out);
+    }
+    return cudaGetLastError();
+  }
+  const size_t smem = t.A ? (size_t)8 * t.D * sizeof(double) : 0;
   const long long want = (M + 7) / 8;
   const unsigned grid = (unsigned)(want < (long long)sms * 8 ? want : (long long)sms * 8);
   if (U32) {
@@ -559,10 +789,42 @@ cudaError_t launch_prior_transform(const gbns_prior_table &t, const float *U32, 
   return cudaGetLastError();
 }
 
+template <int RG>
+static cudaError_t launch_se(const uint32_t *key, const int *num_live, const double *log_L, long long M, int S, int CS,
+                             double *out, cudaStream_t stream) {
+  const size_t smem = (size_t)SE_K * SE_T * sizeof(double2);
+  cudaError_t e = cudaFuncSetAttribute(k_sample_evidence<RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(((unsigned)S + RG - 1) / RG * (unsigned)CS);
+  cfg.blockDim = dim3(SE_T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)CS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_sample_evidence<RG>, key, num_live, log_L, M, S, CS, out);
+}
+
 cudaError_t launch_sample_evidence(const uint32_t *key, const int *num_live, const double *log_L, long long M, int S,
                                    double *out, cudaStream_t stream) {
-  if (S > 0) k_sample_evidence<<<S, 1024, 0, stream>>>(key, num_live, log_L, M, out);
-  return cudaGetLastError();
+  if (S <= 0) return cudaSuccess;
+  int dev = 0, sms = 0;
+  cudaError_t e;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  // parts of at least two samples per thread, eight at most, and no more than give every SM four
+  // blocks; replicas share a cluster as long as every SM still gets two blocks
+  const long long quads = ((long long)S + 3) / 4;
+  int CS = 8;
+  while (CS > 1 && (M < (long long)CS * 2 * SE_T || quads * CS >= 8ll * sms)) CS /= 2;
+  if (quads * CS >= 2ll * sms) return launch_se<4>(key, num_live, log_L, M, S, CS, out, stream);
+  if (((long long)S + 1) / 2 * CS >= 2ll * sms) return launch_se<2>(key, num_live, log_L, M, S, CS, out, stream);
+  return launch_se<1>(key, num_live, log_L, M, S, CS, out, stream);
 }
 
 cudaError_t launch_rng(int mode, const uint32_t *key, const uint32_t *counts, void *out, long long n,
