@@ -384,17 +384,18 @@ static cudaError_t launch_spec_mvn(const gbns_batch &b, int ib, int ie, int per_
 // over an item's chains).  Measured on one GB300, us per shell of 5 D slices, warp-cooperative
 // against 16 / 8 / 4 proposals per round:
 //   chains   D = 24                          chains   D = 48
-//      360   4748 |  299  389  545              720   14635 |  1202  1531 1904
-//    1,440   5027 |  603  414  569            2,880   14676 |  4785  3276 2044
-//    2,880   5039 |  926  814  600            5,760   14711 |  8597  6212 4244
-//   11,520   5153 | 3114 2162 1866           11,520   14750 | 15820 11025 7875
+//      360   2782 |  300  389  545              720    8356 |  1191 1531 1904
+//    1,440   2920 |  607  414  569            2,880    8385 |  4748 3275 2042
+//    5,760   3091 | 1593 1250 1192            5,760    8425 |  8551 6287 4221
+//   11,520   3124 | 3133 2163 1866           11,520    8468 | 15731 10988 7866
+//   23,040   3179 | 6062 4255 3273           23,040    8515 | 30919 20497 13924
 // The warp-cooperative kernel stays at its latency until its CTAs fill the SMs (~39 k chains at
 // D > 32); this kernel's time grows with the chains beyond one wave of CTAs.
 static int spec_mvn_lanes(const gbns_batch &b, int dmax, long long chains) {
   if (b.gradient_guided || b.gradient_slice) return 0;
   if (chains <= 1024) return 16;
   if (chains <= (dmax > 32 ? 1536 : 2048)) return 8;
-  if (chains <= (dmax > 32 ? 20000 : 28000)) return 4;
+  if (chains <= (dmax > 32 ? 12000 : 20000)) return 4;
   return 0;
 }
 

@@ -6,14 +6,20 @@
 //   * likelihoods: the 32 proposals of a step form Delta[D x 32]; the warp computes
 //     Z = Linv * Delta as a register-tiled GEMM (each lane: 4 chains x 8 rows), Linv^T in
 //     shared memory (read as float4 broadcasts), then sum_i z_i^2 per chain;
-//   * chord bounds, the accepted-point update and the D normal variates of each new
-//     direction run lane-parallel over dimensions (two dimensions per lane).
+//   * the D normal variates of the new directions are flattened over the warp (gbns_normals.cuh);
+//     norms, chord bounds and accepted points are per lane, every lane on its own column.
 // Every chain consumes the reference's RNG stream (uni_slice_sampler.py:114-273,
 // :343-441) in the reference's order; only the work assignment differs.
+// Bound: latency and issue of 8 warps per SM at D > 32 (25 KB of chain state each); a step is
+// ~55 % directions (threefry and quantiles, ~22 draws per lane at D = 48), ~20 % GEMM.  Directions,
+// norms and bounds chain by chain with the lanes over dimensions were four times the GEMM's time:
+// D = 48 and 11,520 chains 14.75 ms per shell of 240 slices, per lane 9.5 ms, with the tail
+// quantiles queued 8.5 ms; D = 24 5.15, 3.6 and 3.1 ms.
 // Warps refill finished lanes from the CTA's chain pool, so a CTA (one work item of up to
 // a few thousand chains of one run) keeps all lanes busy until the pool is drained.
 #include "gbns_device.cuh"
 #include "gbns_launch.h"
+#include "gbns_normals.cuh"
 
 namespace gbns {
 
@@ -27,8 +33,22 @@ template <int DMAX>
 struct WarpVecs {
   float DEL[DMAX][32];  // x - mu of the current proposals (column = lane)
   float U0[DMAX][33];   // seed point of each lane's chain
-  float DIR[DMAX][33];  // current direction
+  float DIR[DMAX][33];  // current direction (rows D and above stay zero)
+  uint4 key[32];        // (direction key, lane) of the chains drawing a direction
+  TailQueue<2> tails;
 };
+
+// The xor butterfly sum (distances 16, 8, 4, 2, 1) of one lane's own column, as a tree: leaf l is
+// fmaf(v[l + 32], v[l + 32], v[l] v[l]).
+template <int DMAX, int L, int O>
+__device__ __forceinline__ float butterfly_sq(const float (*v)[33], int lane) {
+  if constexpr (O == 32) {
+    const float v0 = v[L][lane], v1 = DMAX > 32 ? v[DMAX > 32 ? L + 32 : L][lane] : 0.0f;
+    return DMAX > 32 ? fmaf(v1, v1, v0 * v0) : v0 * v0;
+  } else {
+    return butterfly_sq<DMAX, L, 2 * O>(v, lane) + butterfly_sq<DMAX, (L ^ O), 2 * O>(v, lane);
+  }
+}
 
 template <int DMAX>
 __device__ __forceinline__ float slice_alpha_w(int j, int S) {
@@ -83,6 +103,7 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
   }
   // rows k >= D of every warp's Delta stay zero
   for (int q = lane; q < DMAX * 32; q += 32) (&V.DEL[0][0])[q] = 0.0f;
+  for (int q = lane; q < DMAX * 33; q += 32) (&V.DIR[0][0])[q] = 0.0f;
   if (threadIdx.x == 0) {
     s_next = 0;
     s_all_uniform = 1;
@@ -113,6 +134,7 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
   const int budget = b.max_evals_per_slice;
   const int cg = lane >> 2, rg = lane & 3;
   const int j0 = lane, j1 = lane + 32;
+  const uint32_t dmagic = ((1u << 20) + (uint32_t)D - 1u) / (uint32_t)D;  // p / D = p * dmagic >> 20 for p < 2^14
 
   // ---- per-lane chain state
   int c = -1, j = 0, total = 0, in_slice = 0;
@@ -196,21 +218,22 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
   };
 
   for (;;) {
-    // ---- new directions (initial or after an accepted slice), lane-parallel over dims
-    unsigned dm = __ballot_sync(0xffffffffu, need_dir);
-    while (dm) {
-      const int q = __ffs(dm) - 1;
-      dm &= dm - 1;
-      const Key dk = {__shfl_sync(0xffffffffu, dir_key.k0, q), __shfl_sync(0xffffffffu, dir_key.k1, q)};
+    // ---- new directions (initial or after an accepted slice): the normals of all their chains
+    // flattened over the warp, two draws per trip, then each lane its own column's norm
+    const unsigned dm = __ballot_sync(0xffffffffu, need_dir);
+    if (dm) {
       if (D == 1) {
-        if (lane == 0) V.DIR[0][q] = 1.0f;
+        if (need_dir) V.DIR[0][lane] = 1.0f;
       } else {
-        const float v0 = (j0 < D) ? normal_from_bits(bits64(dk, (uint32_t)j0)) : 0.0f;
-        const float v1 = (DMAX > 32 && j1 < D) ? normal_from_bits(bits64(dk, (uint32_t)j1)) : 0.0f;
-        const float ss = warp_sum(fmaf(v1, v1, v0 * v0));
-        const float inv = 1.0f / sqrtf(ss);
-        if (j0 < D) V.DIR[j0][q] = v0 * inv;
-        if (DMAX > 32 && j1 < D) V.DIR[j1][q] = v1 * inv;
+        if (need_dir)
+          V.key[__popc(dm & ((1u << lane) - 1u))] = make_uint4(dir_key.k0, dir_key.k1, (uint32_t)lane, 0u);
+        __syncwarp();
+        warp_normals(__popc(dm) * D, D, dmagic, V.key, V.tails, [&](uint32_t q, int d, float v) { V.DIR[d][q] = v; });
+        if (need_dir) {
+          const float inv = 1.0f / sqrtf(butterfly_sq<DMAX, 0, 1>(V.DIR, lane));
+#pragma unroll 8
+          for (int d = 0; d < D; ++d) V.DIR[d][lane] *= inv;
+        }
       }
     }
     need_dir = false;
@@ -219,48 +242,37 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
     __syncwarp();
 
     // ---- chord bounds for lanes starting a slice (_slice_bounds, uni_slice_sampler.py:41-64)
-    unsigned sm_ = __ballot_sync(0xffffffffu, active && start);
-    while (sm_) {
-      const int q = __ffs(sm_) - 1;
-      sm_ &= sm_ - 1;
-      bool climb = false;
-      if (GRAD && b.gradient_slice) {
+    bool climb = false;
+    if (GRAD && b.gradient_slice) {
+      unsigned sm_ = __ballot_sync(0xffffffffu, active && start);
+      while (sm_) {
+        const int q = __ffs(sm_) - 1;
+        sm_ &= sm_ - 1;
         // gradient_slice (uni_slice_sampler.py:202-214): slice along the normalised gradient at
         // the seed point unless it vanishes or is not finite (one evaluation, counted below)
         float g0, g1;
         grad_col(q, g0, g1);
         const float gn = sqrtf(warp_sum(fmaf(g0, g0, g1 * g1)));
         if (gn != 0.0f && isfinite(gn)) {
-          climb = true;
+          if (lane == q) climb = true;
           if (j0 < D) V.DIR[j0][q] = g0 / gn;
           if (DMAX > 32 && j1 < D) V.DIR[j1][q] = g1 / gn;
         }
         __syncwarp();
       }
-      float t1r = INFINITY, t1l = -INFINITY, t0r = INFINITY, t0l = -INFINITY;
-#pragma unroll
-      for (int h = 0; h < (DMAX > 32 ? 2 : 1); ++h) {
-        const int dd = h ? j1 : j0;
-        if (dd < D) {
-          const float u = V.U0[dd][q], di = 1.0f / V.DIR[dd][q];
-          const float t1 = (1.0f - u) * di, t0 = -u * di;
-          t1r = fminf(t1r, t1 >= 0.f ? t1 : INFINITY);
-          t1l = fmaxf(t1l, t1 <= 0.f ? t1 : -INFINITY);
-          t0r = fminf(t0r, t0 >= 0.f ? t0 : INFINITY);
-          t0l = fmaxf(t0l, t0 <= 0.f ? t0 : -INFINITY);
-        }
+    }
+    if (active && start) {
+      float hi = INFINITY, lo = -INFINITY;
+#pragma unroll 4
+      for (int d = 0; d < D; ++d) {
+        const float u = V.U0[d][lane], di = 1.0f / V.DIR[d][lane];
+        const float t1 = (1.0f - u) * di, t0 = -u * di;
+        hi = fminf(hi, fminf(t1 >= 0.f ? t1 : INFINITY, t0 >= 0.f ? t0 : INFINITY));
+        lo = fmaxf(lo, fmaxf(t1 <= 0.f ? t1 : -INFINITY, t0 <= 0.f ? t0 : -INFINITY));
       }
-      float rgt = fminf(t0r, t1r), lft = fmaxf(t0l, t1l);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        rgt = fminf(rgt, __shfl_xor_sync(0xffffffffu, rgt, o));
-        lft = fmaxf(lft, __shfl_xor_sync(0xffffffffu, lft, o));
-      }
-      if (lane == q) {
-        right = rgt;
-        left = climb ? 0.0f : lft;  // climbing: only t >= 0 (uni_slice_sampler.py:214)
-        if (GRAD && b.gradient_slice) ++total;
-      }
+      right = hi;
+      left = climb ? 0.0f : lo;  // climbing: only t >= 0 (uni_slice_sampler.py:214)
+      if (GRAD && b.gradient_slice) ++total;
     }
 
     // ---- this lane's proposal (_new_proposal: first pick or one shrink step)
@@ -348,18 +360,11 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
       advance = accept || in_slice >= budget;
       if (advance && !accept) failed = true;
     }
-    // accepted point: U0 += t * DIR (lane-parallel over dims)
-    unsigned am = __ballot_sync(0xffffffffu, advance);
-    __syncwarp();
-    {
-      unsigned mm = am;
-      while (mm) {
-        const int q = __ffs(mm) - 1;
-        mm &= mm - 1;
-        const float tq = __shfl_sync(0xffffffffu, t, q);
-        if (j0 < D) V.U0[j0][q] = fmaf(tq, V.DIR[j0][q], V.U0[j0][q]);
-        if (DMAX > 32 && j1 < D) V.U0[j1][q] = fmaf(tq, V.DIR[j1][q], V.U0[j1][q]);
-      }
+    // accepted point: U0 += t * DIR
+    const unsigned am = __ballot_sync(0xffffffffu, advance);
+    if (advance) {
+#pragma unroll 8
+      for (int d = 0; d < D; ++d) V.U0[d][lane] = fmaf(t, V.DIR[d][lane], V.U0[d][lane]);
     }
     __syncwarp();
     bool grad_fallback = false;
