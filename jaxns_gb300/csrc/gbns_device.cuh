@@ -21,26 +21,53 @@ struct Key {
   uint32_t k0, k1;
 };
 
+// Integer addition on the multiply-add pipe.  Threefry, comparisons and conversions all want the
+// ALU pipe, which takes a warp instruction every second cycle per scheduler; with the additions of
+// the rounds moved off it a threefry block takes 90 instead of 100 cycles of a busy scheduler.
+// The multiplier is a constant that the compiler cannot fold away.  A file whose kernels are
+// faster with the compiler's own choice defines GBNS_ROUNDS_ON_ALU.
+static __constant__ uint32_t k_one = 1u;
+__host__ __device__ __forceinline__ uint32_t add_mad(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+  uint32_t r;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(k_one), "r"(b));
+  return r;
+#else
+  return a + b;
+#endif
+}
+
+#if defined(GBNS_ROUNDS_ON_ALU)
+#define GBNS_ROUND_ADD(a, b) ((a) + (b))
+#else
+#define GBNS_ROUND_ADD(a, b) add_mad(a, b)
+#endif
+
 // Threefry-2x32, 20 rounds (Salmon et al. SC'11), the cipher behind jax.random.
 __host__ __device__ __forceinline__ void threefry2x32(uint32_t k0, uint32_t k1, uint32_t c0, uint32_t c1,
                                                       uint32_t &o0, uint32_t &o1) {
   const uint32_t k2 = k0 ^ k1 ^ 0x1BD11BDAu;
   uint32_t x0 = c0 + k0, x1 = c1 + k1;
 #define GBNS_R(r)                         \
-  x0 += x1;                               \
+  x0 = GBNS_ROUND_ADD(x1, x0);            \
+  x1 = (x1 << (r)) | (x1 >> (32 - (r)));  \
+  x1 ^= x0;
+#define GBNS_RI(r, k) /* a key injection and the next round's addition at once */ \
+  x0 = x0 + (k) + x1;                     \
   x1 = (x1 << (r)) | (x1 >> (32 - (r)));  \
   x1 ^= x0;
   GBNS_R(13) GBNS_R(15) GBNS_R(26) GBNS_R(6)
-  x0 += k1; x1 += k2 + 1u;
-  GBNS_R(17) GBNS_R(29) GBNS_R(16) GBNS_R(24)
-  x0 += k2; x1 += k0 + 2u;
-  GBNS_R(13) GBNS_R(15) GBNS_R(26) GBNS_R(6)
-  x0 += k0; x1 += k1 + 3u;
-  GBNS_R(17) GBNS_R(29) GBNS_R(16) GBNS_R(24)
-  x0 += k1; x1 += k2 + 4u;
-  GBNS_R(13) GBNS_R(15) GBNS_R(26) GBNS_R(6)
+  x1 += k2 + 1u;
+  GBNS_RI(17, k1) GBNS_R(29) GBNS_R(16) GBNS_R(24)
+  x1 += k0 + 2u;
+  GBNS_RI(13, k2) GBNS_R(15) GBNS_R(26) GBNS_R(6)
+  x1 += k1 + 3u;
+  GBNS_RI(17, k0) GBNS_R(29) GBNS_R(16) GBNS_R(24)
+  x1 += k2 + 4u;
+  GBNS_RI(13, k1) GBNS_R(15) GBNS_R(26) GBNS_R(6)
   x0 += k2; x1 += k0 + 5u;
 #undef GBNS_R
+#undef GBNS_RI
   o0 = x0;
   o1 = x1;
 }
@@ -64,15 +91,69 @@ __device__ __forceinline__ uint64_t bits64(Key k, uint32_t i) {
 __device__ __forceinline__ float u64_to_float_rn(uint64_t x) { return gbns_fm_u64_to_float(x); }
 
 // jax.random.uniform(float64) in [0,1) from 64 bits: the top 52 bits M give M * 2^-52;
-// rounded once to fp32.
+// rounded once to fp32.  M = A 2^28 + B with A its upper 24 bits: A and the upper 24 bits of B,
+// the lowest of them joined with whether anything follows, convert exactly, and one fused
+// multiply-add rounds their sum as M itself (a third of the ALU work of normalising 64 bits).
+// The joined bit must lie below the rounding position, which M >= 2^29 ensures.
 __device__ __forceinline__ float uniform01(uint64_t b) {
-  return u64_to_float_rn(b >> 12) * 2.220446049250313e-16f;  // 2^-52
+  const uint32_t b0 = (uint32_t)(b >> 32), b1 = (uint32_t)b;
+  if (b0 < 512u) return u64_to_float_rn(b >> 12) * 0x1p-52f;
+  uint32_t B = __byte_perm(b1, b0, 0x7432) & 0xffffffu;  // (b0 & 0xff) << 16 | b1 >> 16
+  if (b1 & 0xf000u) B |= 1u;
+  return fmaf(__uint2float_rn(b0 & 0xffffff00u), 0x1p-32f, __uint2float_rn(B) * 0x1p-48f);
+}
+
+// 2^-54 (4 w + odd) rounded to fp32, w the 51 bits below the top bit of hi and above the low 12 of
+// lo, odd 1 or 3: as uniform01, and something always follows the upper bits.
+__device__ __forceinline__ float odd51_to_float(uint32_t hi, uint32_t lo, uint32_t odd) {
+  const uint32_t h31 = hi & 0x7fffffffu;
+  if (h31 < 256u) return u64_to_float_rn((((((uint64_t)h31) << 32) | lo) >> 12) << 2 | odd) * 0x1p-54f;
+  const uint32_t B = (__funnelshift_l(lo, hi, 17) & 0xffffffu) | 1u;
+  return fmaf(__uint2float_rn(hi & 0x7fffff80u), 0x1p-32f, __uint2float_rn(B) * 0x1p-49f);
 }
 
 // jax.random.normal(float64) = sqrt(2) erfinv(u), u = (4M + 1 - 2^53) 2^-53 (M = top 52
 // bits): the standard normal quantile of p = (4M + 1) 2^-54 with |p - 1/2| and the tail mass
-// formed exactly from the integer M (gbns_fmath.h), so the tails keep full relative precision.
-__device__ __forceinline__ float normal_from_bits(uint64_t b) { return gbns_fm_normal_from_mantissa(b >> 12); }
+// formed exactly from the integer M, so the tails keep full relative precision: the values of
+// gbns_fm_normal_from_mantissa(b >> 12).  2^54 |p - 1/2| = 4 w + 1 above 1/2, w the 51 low bits of
+// M; below it 4 w + 3 with the bits complemented; 2^54 min(p, 1 - p) is the same of the other
+// complement.
+struct NormalSplit {
+  uint32_t y0, y1, flip;  // the bits, complemented (flip all ones) below 1/2
+  float q;                // |p - 1/2|
+  __device__ __forceinline__ float tail_mass() const { return odd51_to_float(~y0, ~y1, 3u ^ (flip & 2u)); }
+  __device__ __forceinline__ uint32_t sign() const { return flip & 0x80000000u; }
+};
+
+__device__ __forceinline__ NormalSplit normal_split(uint64_t b) {
+  const uint32_t b0 = (uint32_t)(b >> 32), b1 = (uint32_t)b;
+  NormalSplit s;
+  s.flip = ~(uint32_t)((int32_t)b0 >> 31);
+  s.y0 = b0 ^ s.flip;
+  s.y1 = b1 ^ s.flip;
+  s.q = odd51_to_float(s.y0, s.y1, 1u | (s.flip & 2u));
+  return s;
+}
+
+__device__ __forceinline__ float normal_from_bits(uint64_t b) {
+  const NormalSplit s = normal_split(b);
+  const float z = s.q <= 0.425f ? gbns_fm_ndtri_center(s.q) : gbns_fm_ndtri_upper(s.tail_mass());
+  return __uint_as_float(__float_as_uint(z) ^ s.sign());
+}
+
+// The chord's ends: the smallest t >= 0 and the largest t <= 0 of the values clipped in, INF and
+// -INF without one.  Non-negative floats are ordered as their bits, and the bits of a negative
+// or NaN exceed those of INF: one unsigned minimum per end replaces a comparison, a selection
+// and a minimum.
+struct Chord {
+  uint32_t hi = 0x7f800000u, lo = 0x7f800000u;
+  __device__ __forceinline__ void clip(float t) {
+    hi = min(hi, __float_as_uint(t + 0.0f));  // -0 as 0
+    lo = min(lo, __float_as_uint(0.0f - t));
+  }
+  __device__ __forceinline__ float right() const { return __uint_as_float(hi); }
+  __device__ __forceinline__ float left() const { return 0.0f - __uint_as_float(lo); }
+};
 
 // ------------------------------------------------------------ log space ------
 

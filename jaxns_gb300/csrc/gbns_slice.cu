@@ -8,7 +8,17 @@
 // whatever their shrink counts.  The U->X prior quantile and the likelihood are evaluated
 // in registers; the run's parameters (mu, Linv, prior tables) sit in shared memory and
 // are read as broadcasts because every thread of a CTA works on chains of the same run.
+//
+// Bound: instructions (77 % of the issue slots, ALU pipe 62 %, 19 of 32 lanes).  D = 10 shells: 8.3
+// evaluations per slice with three threefry blocks each, and ten normals, are 55 % of them.  1024
+// runs x 500 chains, us per shell: 4740; bits to floats by two conversions and one multiply-add
+// instead of a 64-bit normalisation, chord ends by integer minima, the rounds' additions on the
+// multiply-add pipe 4440; the next carry key only after a rejection and in the block that also
+// makes a slice's key 4380; tail quantiles gathered (gbns_normals.cuh) 4180; two dimensions per
+// bounds check 4115; 6 CTAs per SM 4050 (first twelve shells; over the whole run 395 -> 332 ms with
+// starts by the number of lanes that wait).
 #include "gbns_launch.h"
+#include "gbns_normals.cuh"
 #include "gbns_slice.cuh"
 
 namespace gbns {
@@ -19,6 +29,7 @@ template <int DMAX>
 struct DirWarp {
   uint4 key[32];            // (direction key, lane) of each lane that needs a direction
   float buf[32][DMAX + 1];  // the normals, one row per lane
+  uint16_t tails[32 * DMAX];
 };
 
 // jax.grad of Model.forward w.r.t. U at u (analytic): d log L / dx through the prior quantile
@@ -73,13 +84,12 @@ __device__ __forceinline__ void grad_u(const RunSmem<DMAX, FAM> &P, int D, const
 // Minimum resident 128-thread CTAs per SM (8 caps registers at 64): the sampler is latency-
 // bound, and at DMAX <= 8 the cap costs a few tens of bytes of spills per thread (correlated
 // Gaussians at D <= 8: 7 is 0.8 % faster than 8 and 6 is 18 % slower).  Gaussian
-// shells at DMAX 16 run fastest at 7 (72 registers, 32 B of spills): 3.8 % faster than at 6
-// (80 registers) once the direction scratch is sized per warp, so that shared memory no longer
-// limits the resident CTAs.  The other instantiations keep the occupancy they reach without a
+// shells at DMAX 16 run fastest at 6 (80 registers): 1.7 % faster than at 7 (72), 13 % than at 8 and
+// 5 % than at 5.  The other instantiations keep the occupancy they reach without a
 // cap (3 or 4 CTAs).
 template <int DMAX, int FAM>
 constexpr int slice_min_blocks() {
-  return DMAX <= 8 ? (FAM == GBNS_LIK_MVN ? 7 : 8) : ((DMAX == 16 && FAM == GBNS_LIK_SHELLS) ? 7 : (DMAX >= 64 ? 3 : 4));
+  return DMAX <= 8 ? (FAM == GBNS_LIK_MVN ? 7 : 8) : ((DMAX == 16 && FAM == GBNS_LIK_SHELLS) ? 6 : (DMAX >= 64 ? 3 : 4));
 }
 
 // GRAD: the gradient instantiation, for UniDimSliceSampler's two gradient options (runtime
@@ -193,19 +203,22 @@ __global__ void __launch_bounds__(128, GRAD ? 2 : slice_min_blocks<DMAX, FAM>())
   };
   grab();
 
-  // --- flattened slice / shrink loop.  Slice starts (new direction, slice keys, chord bounds)
-  // run on every kStartCadence-th loop trip only: a lane whose slice ended waits for that trip,
-  // so the divergent start work of the warp's lanes is done together, once per kStartCadence
-  // trips.  A chain's draws and arithmetic do not depend on when its lane runs them.  Shells
-  // bench: 1.21x the throughput of starting at every trip (every second trip: 1.14x).
-  constexpr int kStartCadence = 3;
-  int phase = 0;  // loop trips modulo kStartCadence, the same in every lane of the warp
+  // --- flattened slice / shrink loop.  Slice starts (new direction, slice keys, chord
+  // bounds) are the divergent part, so a lane whose slice ended waits until three eighths of the
+  // warp's live lanes do, and they start together; a chain's draws and arithmetic do not depend
+  // on when its lane runs them.  Waiting costs idle evaluations, starting costs a pass for few
+  // lanes, and the best fixed cadence moves with the evaluations per slice.  Sampler time of a
+  // whole run, ms: 1024 x D = 10 shells (8.3 evaluations per slice), 1000 x D = 8 Normal priors,
+  // 600 x D = 12: every second trip 367, 198, 132; third 349, 204, 129; fourth 344, 212, 130;
+  // a quarter waiting 336, 201, 131; three eighths 332, 198, 126; half 335, 199, 127.
   for (;;) {
-    const bool cadence = phase == 0;
-    phase = phase + 1 == kStartCadence ? 0 : phase + 1;
+    const bool active = j < S;
+    const unsigned alive = __ballot_sync(0xffffffffu, active), waiting = __ballot_sync(0xffffffffu, active && start);
+    if (!alive) break;
+    const bool go = __popc(waiting) * 8 >= __popc(alive) * 3;
     // ---- new directions: the D normals of every lane that needs one, flattened over
     // (lane, dimension) pairs across the warp; lanes publish their keys in rank order
-    const unsigned dmask = __ballot_sync(0xffffffffu, need_dir && cadence);
+    const unsigned dmask = __ballot_sync(0xffffffffu, need_dir && go);
     if (dmask) {
       if (D == 1) {
         if (need_dir) d[0] = 1.0f;
@@ -213,14 +226,7 @@ __global__ void __launch_bounds__(128, GRAD ? 2 : slice_min_blocks<DMAX, FAM>())
         if (need_dir)
           W.key[__popc(dmask & ((1u << lane) - 1u))] = make_uint4(dir_key.k0, dir_key.k1, (uint32_t)lane, 0u);
         __syncwarp();
-        const int cnt = __popc(dmask) * D;
-        for (int p = lane; p < cnt; p += 32) {
-          const int g = (int)(((uint32_t)p * dmagic) >> 20);
-          const uint4 e = W.key[g];
-          const uint32_t jj = (uint32_t)(p - g * D);
-          W.buf[e.z][jj] = normal_from_bits(bits64(Key{e.x, e.y}, jj));
-        }
-        __syncwarp();
+        warp_normals<1>(__popc(dmask) * D, D, dmagic, W.key, W.tails, [&](uint32_t row, int q) -> float & { return W.buf[row][q]; });
         if (need_dir) {
           float ss = 0.0f;
 #pragma unroll
@@ -238,16 +244,13 @@ __global__ void __launch_bounds__(128, GRAD ? 2 : slice_min_blocks<DMAX, FAM>())
       }
       need_dir = false;
     }
-    const bool active = j < S;
-    if (!__any_sync(0xffffffffu, active)) break;
-    if (!active || (start && !cadence)) continue;
+    if (!active || (start && !go)) continue;
 
     // ---- one proposal: the first pick of slice j, or one shrink step (_new_proposal)
-    Key B;
-    if (start) B = fold(slices_key, (uint32_t)j);
-    else B = ck;
-    ck = fold(B, 0u);                              // run_key / next carry key
+    const Key from = start ? slices_key : ck;
+    const Key B = fold(from, start ? (uint32_t)j : 0u);  // the slice's key / the next carry key
     const Key tk = fold(B, start ? 2u : 1u);       // t_key
+    ck = B;
     if (start) {
       after_key = fold(B, 3u);
       alpha = slice_alpha(j, S);
@@ -271,21 +274,17 @@ __global__ void __launch_bounds__(128, GRAD ? 2 : slice_min_blocks<DMAX, FAM>())
         }
       }
       // _slice_bounds (uni_slice_sampler.py:41-64), with one reciprocal per direction component
-      float t1r = INFINITY, t1l = -INFINITY, t0r = INFINITY, t0l = -INFINITY;
+      Chord ch;
 #pragma unroll
       for (int q = 0; q < DMAX; ++q) {
         if (q < D) {
           const float rc = 1.0f / d[q];
-          const float t1 = (1.0f - u0[q]) * rc;
-          const float t0 = -u0[q] * rc;
-          t1r = fminf(t1r, t1 >= 0.f ? t1 : INFINITY);
-          t1l = fmaxf(t1l, t1 <= 0.f ? t1 : -INFINITY);
-          t0r = fminf(t0r, t0 >= 0.f ? t0 : INFINITY);
-          t0l = fmaxf(t0l, t0 <= 0.f ? t0 : -INFINITY);
+          ch.clip((1.0f - u0[q]) * rc);
+          ch.clip(-u0[q] * rc);
         }
       }
-      right = fminf(t0r, t1r);
-      left = climb ? 0.0f : fmaxf(t0l, t1l);  // climbing: only t >= 0 (uni_slice_sampler.py:214)
+      right = ch.right();
+      left = climb ? 0.0f : ch.left();  // climbing: only t >= 0 (uni_slice_sampler.py:214)
       in_slice = 0;
     } else {
       // _shrink_interval (uni_slice_sampler.py:92-111)

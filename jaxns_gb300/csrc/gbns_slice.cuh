@@ -101,14 +101,19 @@ __device__ __forceinline__ float loglik(const RunSmem<DMAX, FAM> &P, int D, cons
   } else {
     float r1 = 0.0f, r2 = 0.0f;
     if (P.all_uniform) {
+      // two dimensions per test against D: above an odd D the tables, the point and the direction
+      // are 0 and add 0
 #pragma unroll
-      for (int j = 0; j < DMAX; ++j) {
-        if (j < D) {
-          const float4 q = P.ab[j];
-          const float x = fmaf(q.y, fmaf(t, d[j], u0[j]), q.x);
-          const float e1 = x - q.z, e2 = x - q.w;
-          r1 = fmaf(e1, e1, r1);
-          r2 = fmaf(e2, e2, r2);
+      for (int j2 = 0; j2 < DMAX; j2 += 2) {
+        if (j2 < D) {
+#pragma unroll
+          for (int j = j2; j < j2 + 2; ++j) {
+            const float4 q = P.ab[j];
+            const float x = fmaf(q.y, fmaf(t, d[j], u0[j]), q.x);
+            const float e1 = x - q.z, e2 = x - q.w;
+            r1 = fmaf(e1, e1, r1);
+            r2 = fmaf(e2, e2, r2);
+          }
         }
       }
     } else {

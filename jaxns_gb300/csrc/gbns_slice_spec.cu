@@ -18,7 +18,10 @@
 // Bound: latency.  A chain of S slices is a serial chain of about S x (chord bounds + G interval
 // steps + one likelihood + ballot); the evaluations beyond the accepted one are spare work of an
 // otherwise idle GPU, which is why the launcher takes this kernel only below a chain count.
+// (5,760 chains of D = 8: 193 us per shell, 201 with the additions of the rounds moved)
+#define GBNS_ROUNDS_ON_ALU
 #include "gbns_launch.h"
+#include "gbns_normals.cuh"
 #include "gbns_spec.cuh"
 
 namespace gbns {
@@ -37,6 +40,7 @@ template <int DMAX>
 struct SpecTeam {
   SpecBlock<DMAX> blk[2];
   uint4 key[2][32];  // (direction key, row) of the rows whose normals are being drawn
+  uint16_t tails[2][32 * DMAX];
 };
 
 __device__ __forceinline__ void team_barrier(int id) { asm volatile("bar.sync %0, 96;" ::"r"(id) : "memory"); }
@@ -44,13 +48,14 @@ __device__ __forceinline__ void team_barrier(int id) { asm volatile("bar.sync %0
 // Directions (and reciprocals) of the rows in `rows`: D normals per row, flattened over the
 // warp, then normalised one row per lane in dimension order.
 template <int DMAX>
-__device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, const SpecKeys &k, int j, int end, int D,
+__device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, uint16_t *tails, const SpecKeys &k, int j, int end, int D,
                                                 uint32_t dmagic, uint32_t rows) {
   const int lane = threadIdx.x & 31;
   const bool valid = k.valid && j < end && ((rows >> lane) & 1u);
   if (D == 1) {
     if (valid) {
       B.d[lane][0] = 1.0f;
+      B.d[lane][1] = 0.0f;
       B.rc[lane][0] = 1.0f;
     }
     __syncwarp();
@@ -62,18 +67,8 @@ __device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, 
     key[__popc(mask & ((1u << lane) - 1u))] = make_uint4(dk.k0, dk.k1, (uint32_t)lane, 0u);
   }
   __syncwarp();
-  const int cnt = __popc(mask) * D;
   // two draws per pass, their threefry blocks interleaved
-  for (int p = lane; p < cnt; p += 64) {
-    const int p1 = p + 32 < cnt ? p + 32 : p;
-    const int ga = (int)(((uint32_t)p * dmagic) >> 20), gb = (int)(((uint32_t)p1 * dmagic) >> 20);
-    const uint4 ea = key[ga], eb = key[gb];
-    const uint32_t ja = (uint32_t)(p - ga * D), jb = (uint32_t)(p1 - gb * D);
-    const uint64_t ba = bits64(Key{ea.x, ea.y}, ja), bb = bits64(Key{eb.x, eb.y}, jb);
-    B.d[ea.z][ja] = normal_from_bits(ba);
-    if (p + 32 < cnt) B.d[eb.z][jb] = normal_from_bits(bb);
-  }
-  __syncwarp();
+  warp_normals<2>(__popc(mask) * D, D, dmagic, key, tails, [&](uint32_t row, int q) -> float & { return B.d[row][q]; });
   if (valid) {
     float d[DMAX];
     float ss = 0.0f;
@@ -91,6 +86,7 @@ __device__ __forceinline__ void spec_directions(SpecBlock<DMAX> &B, uint4 *key, 
         B.d[lane][q] = v;
         B.rc[lane][q] = 1.0f / v;
       }
+    if (D & 1) B.d[lane][D] = 0.0f;  // the other half of loglik's last pair
   }
   __syncwarp();
 }
@@ -221,7 +217,7 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
         if (bi < nb) {
           SpecBlock<DMAX> &B = W.blk[bi & 1];
           const int j = spec_block_begin(bi, SB, SB0) + li, end = bi == 0 ? min(S, SB0) : S;
-          if (role == 1) spec_directions(B, W.key[1], sk, j, end, D, dmagic, bi == 0 ? ~kHalf : 0xffffffffu);
+          if (role == 1) spec_directions(B, W.key[1], W.tails[1], sk, j, end, D, dmagic, bi == 0 ? ~kHalf : 0xffffffffu);
           else spec_uniforms(B.r, sk, j, end, S, bi == 0 ? spec_first(G) : SPEC_E, midpoint);
         }
         team_barrier(bar);
@@ -246,7 +242,7 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
       u_own[k] = have && q < D ? liveU[(size_t)idx * D + q] : 0.0f;
     }
     if (have) logL0 = liveL[idx];
-    spec_directions(W.blk[0], W.key[0], sk, li, min(S, SB0), D, dmagic, kHalf);
+    spec_directions(W.blk[0], W.key[0], W.tails[0], sk, li, min(S, SB0), D, dmagic, kHalf);
     team_barrier(bar);
 
     int j = 0, total = 0;
@@ -268,22 +264,20 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
         if (__any_sync(0xffffffffu, begin)) {
           // _slice_bounds (uni_slice_sampler.py:41-64), the group's lanes over the dimensions;
           // a group inside its slice reads its own direction again and keeps its interval
-          float hi = INFINITY, lo = -INFINITY;
+          Chord ch;
 #pragma unroll
           for (int k = 0; k < OWN; ++k) {
             const int q = li + k * GL;
             if (q < D) {
               const float rc = B.rc[row][q];
-              const float t1 = (1.0f - u_own[k]) * rc;
-              const float t0 = -u_own[k] * rc;
-              hi = fminf(hi, fminf(t1 >= 0.f ? t1 : INFINITY, t0 >= 0.f ? t0 : INFINITY));
-              lo = fmaxf(lo, fmaxf(t1 <= 0.f ? t1 : -INFINITY, t0 <= 0.f ? t0 : -INFINITY));
+              ch.clip((1.0f - u_own[k]) * rc);
+              ch.clip(-u_own[k] * rc);
             }
           }
 #pragma unroll
           for (int o = GL / 2; o > 0; o >>= 1) {
-            hi = fminf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-            lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            ch.hi = min(ch.hi, __shfl_xor_sync(0xffffffffu, ch.hi, o));
+            ch.lo = min(ch.lo, __shfl_xor_sync(0xffffffffu, ch.lo, o));
           }
 #pragma unroll
           for (int q = 0; q < DMAX; q += 4) {
@@ -295,8 +289,8 @@ __global__ void __launch_bounds__(96 * SPEC_TEAMS, DMAX <= 16 ? 3 : 1)
           }
           alpha = B.r.alpha[row];
           if (begin) {
-            right = hi;
-            left = lo;
+            right = ch.right();
+            left = ch.left();
             t = 0.0f;  // no shrink before the first pick
             e = 0;
             ext = false;
@@ -394,12 +388,12 @@ static cudaError_t launch_spec(const gbns_batch &b, int ib, int ie, const float 
 // An item holds at most chains_per_item chains per lane of its CTA, so items x chains_per_item
 // bounds the chains of the launch.  Measured on one GB300, us per shell of 5 D slices,
 // thread-per-chain against 32 (8 proposals x 4) / 8 / 4 lanes per chain:
-//   chains   MVN D = 8, Normal priors   shells D = 10            MVN D = 16
-//      120   648 | 61  104 139          636 | 68  70 112         1301 | 161 169 218   (120-240)
-//    1,920   669 | 180 129 166          654 | 151 90 119 (1,200) 1320 | 830 349 260   (3,840)
-//    5,760   677 | 420 257 220          660 | 446 184 175 (4,800)
-//   12,000   684 | 806 513 423          663 | -   488 460 (15,000) 1333 | - 846 685   (14,400)
-//   24,000   768 | -   1034 882         779 | -  2090 1740 (45,000)
+//   chains   MVN D = 8, Normal priors   shells D = 10             MVN D = 16
+//      120   602 | 62  106 137          541 |   66  70 107        1099 |  173 172 222   (150; 240)
+//    1,920   626 | 179 133 161          556 |  143  78 110 (1,200) 1126 |  890 353 244   (3,840)
+//    5,760   633 | 422 263 205          564 |  431 176 158 (4,800)
+//   12,000   643 | 808 524 390          567 | 1211 469 410 (15,000) 1139 | 2891 842 616  (14,400)
+//   24,000   727 | 1544 989 757         659 |    - 1369 1090 (45,000)
 // The thread-per-chain kernel's time hardly depends on the chain count until it fills the
 // GPU; this kernel's grows with it from the first wave on, so the line lies where they cross.
 constexpr long long SPEC_CHAINS_32 = 704, SPEC_CHAINS_8 = 3584, SPEC_CHAINS_4 = 20000;

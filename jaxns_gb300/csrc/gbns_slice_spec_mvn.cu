@@ -13,6 +13,7 @@
 // whatever the number of chains, so what counts is rounds per slice (about 1.2 at G = 16) and
 // that chains spread over all SMs: a run of 360 chains is 180 warps here and was one CTA.
 #include "gbns_launch.h"
+#include "gbns_normals.cuh"
 #include "gbns_spec.cuh"
 
 namespace gbns {
@@ -32,13 +33,14 @@ struct SpecWarpSmem {
   float U0[NG][DMAX + 4];    // seed point of each chain
   SpecRows<DMAX> blk[2];
   uint4 key[3][32];          // (direction key, row) of the rows whose normals are being drawn
+  uint16_t tails[3][32 * DMAX];
   int m, all_uniform;
 };
 
 // Directions of the rows in `rows` (one row per lane): normals flattened over (row, dimension)
 // pairs, two draws per pass, then norm and scaling row by row with the lanes over dimensions.
 template <int DMAX>
-__device__ __forceinline__ void spec_directions_w(SpecRows<DMAX> &B, uint4 *key, const SpecKeys &k, int j, int end, int D,
+__device__ __forceinline__ void spec_directions_w(SpecRows<DMAX> &B, uint4 *key, uint16_t *tails, const SpecKeys &k, int j, int end, int D,
                                                   uint32_t dmagic, uint32_t rows) {
   const int lane = threadIdx.x & 31;
   const bool valid = k.valid && j < end && ((rows >> lane) & 1u);
@@ -53,17 +55,7 @@ __device__ __forceinline__ void spec_directions_w(SpecRows<DMAX> &B, uint4 *key,
     key[__popc(mask & ((1u << lane) - 1u))] = make_uint4(dk.k0, dk.k1, (uint32_t)lane, 0u);
   }
   __syncwarp();
-  const int cnt = __popc(mask) * D;
-  for (int p = lane; p < cnt; p += 64) {
-    const int p1 = p + 32 < cnt ? p + 32 : p;
-    const int ga = (int)(((uint32_t)p * dmagic) >> 20), gb = (int)(((uint32_t)p1 * dmagic) >> 20);
-    const uint4 ea = key[ga], eb = key[gb];
-    const uint32_t ja = (uint32_t)(p - ga * D), jb = (uint32_t)(p1 - gb * D);
-    const uint64_t ba = bits64(Key{ea.x, ea.y}, ja), bb = bits64(Key{eb.x, eb.y}, jb);
-    B.d[ea.z][ja] = normal_from_bits(ba);
-    if (p + 32 < cnt) B.d[eb.z][jb] = normal_from_bits(bb);
-  }
-  __syncwarp();
+  warp_normals<2>(__popc(mask) * D, D, dmagic, key, tails, [&](uint32_t row, int q) -> float & { return B.d[row][q]; });
   const int j0 = lane, j1 = lane + 32;
   while (mask) {
     const int row = __ffs(mask) - 1;
@@ -165,7 +157,7 @@ __global__ void __launch_bounds__(128, DMAX == 32 ? 4 : 3)
             spec_uniforms(B.r, sk, j, end, S, bi == 0 ? spec_first(G) : SPEC_E, midpoint);
           } else {
             const uint32_t rows = bi == 0 ? kThird << warp : (warp == 1 ? 0x55555555u : 0xaaaaaaaau);
-            spec_directions_w(B, W.key[warp], sk, j, end, D, dmagic, rows);
+            spec_directions_w(B, W.key[warp], W.tails[warp], sk, j, end, D, dmagic, rows);
           }
         }
         cta_barrier();
@@ -183,7 +175,7 @@ __global__ void __launch_bounds__(128, DMAX == 32 ? 4 : 3)
       if (H > 1 && j1 < D) W.U0[q][j1] = liveU[(size_t)iq * D + j1];
     }
     if (have) logL0 = liveL[idx];
-    spec_directions_w(W.blk[0], W.key[0], sk, li, min(S, SB0), D, dmagic, kThird);
+    spec_directions_w(W.blk[0], W.key[0], W.tails[0], sk, li, min(S, SB0), D, dmagic, kThird);
     cta_barrier();
 
     int j = 0, total = 0;
@@ -210,25 +202,21 @@ __global__ void __launch_bounds__(128, DMAX == 32 ? 4 : 3)
           for (int q = 0; q < NG; ++q) {
             if ((beg >> (q * G)) & 1u) {
               const int rq = __shfl_sync(0xffffffffu, row, q * G);
-              float hi = INFINITY, lo = -INFINITY;
+              Chord ch;
 #pragma unroll
               for (int h = 0; h < H; ++h) {
                 const int dd = h ? j1 : j0;
                 if (dd < D) {
                   const float u = W.U0[q][dd], di = 1.0f / B.d[rq][dd];
-                  const float t1 = (1.0f - u) * di, t0 = -u * di;
-                  hi = fminf(hi, fminf(t1 >= 0.f ? t1 : INFINITY, t0 >= 0.f ? t0 : INFINITY));
-                  lo = fmaxf(lo, fmaxf(t1 <= 0.f ? t1 : -INFINITY, t0 <= 0.f ? t0 : -INFINITY));
+                  ch.clip((1.0f - u) * di);
+                  ch.clip(-u * di);
                 }
               }
-#pragma unroll
-              for (int o = 16; o > 0; o >>= 1) {
-                hi = fminf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-                lo = fmaxf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-              }
+              ch.hi = __reduce_min_sync(0xffffffffu, ch.hi);
+              ch.lo = __reduce_min_sync(0xffffffffu, ch.lo);
               if (g == q) {
-                right = hi;
-                left = lo;
+                right = ch.right();
+                left = ch.left();
                 t = 0.0f;  // no shrink before the first pick
                 alpha = B.r.alpha[row];
                 e = 0;
@@ -384,18 +372,18 @@ static cudaError_t launch_spec_mvn(const gbns_batch &b, int ib, int ie, int per_
 // over an item's chains).  Measured on one GB300, us per shell of 5 D slices, warp-cooperative
 // against 16 / 8 / 4 proposals per round:
 //   chains   D = 24                          chains   D = 48
-//      360   2782 |  300  389  545              720    8356 |  1191 1531 1904
-//    1,440   2920 |  607  414  569            2,880    8385 |  4748 3275 2042
-//    5,760   3091 | 1593 1250 1192            5,760    8425 |  8551 6287 4221
-//   11,520   3124 | 3133 2163 1866           11,520    8468 | 15731 10988 7866
-//   23,040   3179 | 6062 4255 3273           23,040    8515 | 30919 20497 13924
+//      360   2722 |  283  314  428              720    7375 |  1159 1245  1586
+//    1,440   2915 |  570  337  449            2,880    7435 |  4623 2742  1674
+//    5,760   2986 | 1496 1011  933            5,760    7477 |  8261 5171  3539
+//   11,520   3029 | 2936 1767 1457           11,520    7526 | 15196 9108  6424
+//   23,040   3052 | 5672 3487 2559           23,040    7554 | 29954 16986 11393
 // The warp-cooperative kernel stays at its latency until its CTAs fill the SMs (~39 k chains at
 // D > 32); this kernel's time grows with the chains beyond one wave of CTAs.
 static int spec_mvn_lanes(const gbns_batch &b, int dmax, long long chains) {
   if (b.gradient_guided || b.gradient_slice) return 0;
   if (chains <= 1024) return 16;
   if (chains <= (dmax > 32 ? 1536 : 2048)) return 8;
-  if (chains <= (dmax > 32 ? 12000 : 20000)) return 4;
+  if (chains <= (dmax > 32 ? 13000 : 27000)) return 4;
   return 0;
 }
 

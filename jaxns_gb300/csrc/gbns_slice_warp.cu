@@ -14,7 +14,7 @@
 // ~55 % directions (threefry and quantiles, ~22 draws per lane at D = 48), ~20 % GEMM.  Directions,
 // norms and bounds chain by chain with the lanes over dimensions were four times the GEMM's time:
 // D = 48 and 11,520 chains 14.75 ms per shell of 240 slices, per lane 9.5 ms, with the tail
-// quantiles queued 8.5 ms; D = 24 5.15, 3.6 and 3.1 ms.
+// quantiles gathered 7.5 ms; D = 24 5.15, 3.6 and 3.0 ms.
 // Warps refill finished lanes from the CTA's chain pool, so a CTA (one work item of up to
 // a few thousand chains of one run) keeps all lanes busy until the pool is drained.
 #include "gbns_device.cuh"
@@ -35,7 +35,6 @@ struct WarpVecs {
   float U0[DMAX][33];   // seed point of each lane's chain
   float DIR[DMAX][33];  // current direction (rows D and above stay zero)
   uint4 key[32];        // (direction key, lane) of the chains drawing a direction
-  TailQueue<2> tails;
 };
 
 // The xor butterfly sum (distances 16, 8, 4, 2, 1) of one lane's own column, as a tree: leaf l is
@@ -228,7 +227,9 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
         if (need_dir)
           V.key[__popc(dm & ((1u << lane) - 1u))] = make_uint4(dir_key.k0, dir_key.k1, (uint32_t)lane, 0u);
         __syncwarp();
-        warp_normals(__popc(dm) * D, D, dmagic, V.key, V.tails, [&](uint32_t q, int d, float v) { V.DIR[d][q] = v; });
+        // (the list of tails takes 64 D of the 128 D bytes of the proposals, which are written later)
+        warp_normals<2>(__popc(dm) * D, D, dmagic, V.key, (uint16_t *)&V.DEL[0][0],
+                        [&](uint32_t q, int d) -> float & { return V.DIR[d][q]; });
         if (need_dir) {
           const float inv = 1.0f / sqrtf(butterfly_sq<DMAX, 0, 1>(V.DIR, lane));
 #pragma unroll 8
@@ -262,16 +263,15 @@ __global__ void __launch_bounds__(32 * (DMAX == 64 ? WARPS_PER_CTA_64 : WARPS_PE
       }
     }
     if (active && start) {
-      float hi = INFINITY, lo = -INFINITY;
+      Chord ch;
 #pragma unroll 4
       for (int d = 0; d < D; ++d) {
         const float u = V.U0[d][lane], di = 1.0f / V.DIR[d][lane];
-        const float t1 = (1.0f - u) * di, t0 = -u * di;
-        hi = fminf(hi, fminf(t1 >= 0.f ? t1 : INFINITY, t0 >= 0.f ? t0 : INFINITY));
-        lo = fmaxf(lo, fmaxf(t1 <= 0.f ? t1 : -INFINITY, t0 <= 0.f ? t0 : -INFINITY));
+        ch.clip((1.0f - u) * di);
+        ch.clip(-u * di);
       }
-      right = hi;
-      left = climb ? 0.0f : lo;  // climbing: only t >= 0 (uni_slice_sampler.py:214)
+      right = ch.right();
+      left = climb ? 0.0f : ch.left();  // climbing: only t >= 0 (uni_slice_sampler.py:214)
       if (GRAD && b.gradient_slice) ++total;
     }
 
