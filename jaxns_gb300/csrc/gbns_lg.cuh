@@ -29,8 +29,8 @@ __device__ __forceinline__ float ndtri_pair(float a, float s) {
   pair_add(a, s, hi, lo);
   const float q = (hi - 0.5f) + lo;  // u - 1/2
   if (fabsf(q) <= 0.425f) return gbns_fm_ndtri_center(q);
-  if (q > 0.0f) return gbns_fm_ndtri_upper((1.0f - hi) - lo);
-  return -gbns_fm_ndtri_upper(hi + lo);
+  const float z = gbns_fm_ndtri_upper(q > 0.0f ? (1.0f - hi) - lo : hi + lo);  // one tail for both signs
+  return q > 0.0f ? z : -z;
 }
 
 __device__ __forceinline__ float prior_quantile_pair(int kind, float pa, float pb, float a, float s) {

@@ -231,28 +231,19 @@ __global__ void __launch_bounds__(256) k_lg_step(gbns_batch b, gbns_lg_bufs lg, 
         }
       }
       // chord of u0 + t d in the unit cube; 1 - u = (1 - a) - b keeps the tails exact
-      float t1r = INFINITY, t1l = -INFINITY, t0r = INFINITY, t0l = -INFINITY;
+      Chord ch;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const bool have = h ? hb : ha;
         if (have) {
           const float uu = h ? ub : ua, ll = h ? lb : la, dd = h ? db : da;
-          const float t1 = ((1.0f - uu) - ll) / dd, t0 = -(uu + ll) / dd;
-          t1r = fminf(t1r, t1 >= 0.f ? t1 : INFINITY);
-          t1l = fmaxf(t1l, t1 <= 0.f ? t1 : -INFINITY);
-          t0r = fminf(t0r, t0 >= 0.f ? t0 : INFINITY);
-          t0l = fmaxf(t0l, t0 <= 0.f ? t0 : -INFINITY);
+          ch.clip(((1.0f - uu) - ll) / dd);
+          ch.clip(-(uu + ll) / dd);
         }
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        t1r = fminf(t1r, __shfl_xor_sync(0xffffffffu, t1r, o));
-        t1l = fmaxf(t1l, __shfl_xor_sync(0xffffffffu, t1l, o));
-        t0r = fminf(t0r, __shfl_xor_sync(0xffffffffu, t0r, o));
-        t0l = fmaxf(t0l, __shfl_xor_sync(0xffffffffu, t0l, o));
-      }
-      right = fminf(t0r, t1r);
-      left = climb ? 0.0f : fmaxf(t0l, t1l);
+      right = __uint_as_float(__reduce_min_sync(0xffffffffu, ch.hi));
+      ch.lo = __reduce_min_sync(0xffffffffu, ch.lo);
+      left = climb ? 0.0f : ch.left();
       in_slice = 0;
     } else {
       if (t < 0.f) left = t;

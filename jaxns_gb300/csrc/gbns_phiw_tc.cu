@@ -90,20 +90,6 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// ------------------------------------------------------------------ sampler step
-//
-// Persistent, warp-specialised, one CTA per SM: each CTA walks work units (run, 128-chain tile,
-// range of 128-row tiles) with a grid stride.  Warp 0 streams the unit's W tile (hi / lo) and Phi
-// stages (two row tiles x one K block, hi / lo) through shared memory with TMA, warp 1 issues the
-// 3xTF32 MMAs of two row tiles at a time (256 rows, see the adjoint kernel) into two 256-column
-// accumulators in turn, and warps 2-5 and 6-9 drain a row tile each (thread = chain), keep the
-// chain's partial sum of squares in a register over the unit and add it to the chain's FP64
-// total once per unit.  Copies, MMAs and epilogue of successive row tiles overlap.  Units whose
-// chain tile has no pending proposal are skipped by every role alike (the flags are read-only
-// during the launch).
-// Bound: MMAs (~15 us of the 38 below) and, per unit, the latency of its flags and first copies.
-// Twelve problems of up to 16384 x 64: 128-row MMAs, four 128-column accumulators 47 us per launch,
-// this 38 us.
 // hi + lo += x (TwoSum of hi and x, the rounding error carried in lo).  GB300 runs FP64 at
 // about 1/64 of the FP32 rate, so the step's sums of squares travel as fp32 pairs: each adds
 // at most a few units of 2^-48 of relative error, far below the fp32 rounding of the 32-row
@@ -114,18 +100,9 @@ __device__ __forceinline__ void lf_pair_acc(float &hi, float &lo, float x) {
   lo += e;
 }
 
-// ------------------------------------------------------------------ sampler step
-//
-// Persistent, warp-specialised: each CTA walks work units (run, 128-chain tile, range of
-// 128-row tiles) with a grid stride.  Warp 0 streams the unit's W tile (hi / lo) and its Phi
-// row tiles (hi / lo) through shared memory with TMA, warp 1 issues the 3xTF32 MMAs of each
-// row tile into a ring of 128-column accumulators in tensor memory, and warps 2-5 drain the
-// accumulators (thread = chain), keep the chain's partial sum of squares in a register over
-// the unit's row tiles and add it to the chain's FP64 total once per unit.  Copies, MMAs and
-// epilogue of successive row tiles overlap.  Units whose chain tile has no pending proposal
-// are skipped by every role alike (the flags are read-only during the launch).
 // 32 consecutive fp32 columns of this warp's 32 lanes (thread t gets lane base + t): the load, and
-// its wait.  The registers pass through the wait, so no use of them can be scheduled before it.  One load can be in flight while the columns before are used.
+// its wait.  The registers pass through the wait, so no use of them can be scheduled before it.
+// One load can be in flight while the columns before are used.
 __device__ __forceinline__ void tc_ld32_start(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -147,22 +124,37 @@ __device__ __forceinline__ void tc_ld32_finish(uint32_t (&r)[32]) {
                : "memory");
 }
 
+// Two fp32 fused multiply-adds in one instruction (each rounded as its own).
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+__device__ __forceinline__ float sum2(uint64_t a) {
+  return __uint_as_float((uint32_t)a) + __uint_as_float((uint32_t)(a >> 32));
+}
+constexpr uint64_t MINUS_ONE2 = 0xBF800000BF800000ull;
+
 // sum_j (y_j - v_j)^2 over the first n (<= 32) of 32 accumulator columns, in four
 // independent FMA chains (j mod 4) so that the reduction does not serialise on FMA latency
 __device__ __forceinline__ float sq_resid32(const float *ys, const uint32_t (&v)[32], int n) {
-  float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;
   if (n >= 32) {
+    uint64_t p01 = 0ull, p23 = 0ull;
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
-      const float4 y = *reinterpret_cast<const float4 *>(ys + j);  // (16-byte aligned)
-      const float r0 = y.x - __uint_as_float(v[j]), r1 = y.y - __uint_as_float(v[j + 1]);
-      const float r2 = y.z - __uint_as_float(v[j + 2]), r3 = y.w - __uint_as_float(v[j + 3]);
-      p0 = fmaf(r0, r0, p0);
-      p1 = fmaf(r1, r1, p1);
-      p2 = fmaf(r2, r2, p2);
-      p3 = fmaf(r3, r3, p3);
+      const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(ys + j);  // (16-byte aligned)
+      const uint64_t r01 = fma2(pack2(v[j], v[j + 1]), MINUS_ONE2, y.x), r23 = fma2(pack2(v[j + 2], v[j + 3]), MINUS_ONE2, y.y);
+      p01 = fma2(r01, r01, p01);
+      p23 = fma2(r23, r23, p23);
     }
-  } else {
+    return sum2(p01) + sum2(p23);
+  }
+  float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f, p3 = 0.0f;
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
       const float r0 = ys[j] - __uint_as_float(v[j]), r1 = ys[j + 1] - __uint_as_float(v[j + 1]);
@@ -172,10 +164,23 @@ __device__ __forceinline__ float sq_resid32(const float *ys, const uint32_t (&v)
       p2 = j + 2 < n ? fmaf(r2, r2, p2) : p2;
       p3 = j + 3 < n ? fmaf(r3, r3, p3) : p3;
     }
-  }
   return (p0 + p1) + (p2 + p3);
 }
 
+// ------------------------------------------------------------------ sampler step
+//
+// Persistent, warp-specialised, one CTA per SM: each CTA walks work units (run, 128-chain tile,
+// range of 128-row tiles) with a grid stride.  Warp 0 streams the unit's W tile (hi / lo) and Phi
+// stages (two row tiles x one K block, hi / lo) through shared memory with TMA, warp 1 issues the
+// 3xTF32 MMAs of two row tiles at a time (256 rows, see the adjoint kernel) into two 256-column
+// accumulators in turn, and warps 2-5 and 6-9 drain a row tile each (thread = chain), keep the
+// chain's partial sum of squares in a register over the unit and add it to the chain's FP64
+// total once per unit.  Copies, MMAs and epilogue of successive row tiles overlap.  Units whose
+// chain tile has no pending proposal are skipped by every role alike (the flags are read-only
+// during the launch).
+// Bound: MMAs (~15 us of the 38 below) and, per unit, the latency of its flags and first copies.
+// Twelve problems of up to 16384 x 64: 128-row MMAs, four 128-column accumulators 47 us per launch,
+// this 38 us.
 constexpr int SR_ROWS = 128;                       // data rows per tile (accumulator columns)
 constexpr unsigned SR_BOX = 128 * TC_KB * 4;       // one K block of 128 rows: 16 KB
 constexpr int SR_THREADS = 320;
@@ -494,16 +499,24 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
 //   1. every owner warp consumes its chain's residual sum, advances the slice logic and writes
 //      the chain's next proposal (one TF32 hi / lo row) into the W tile of every CTA of the
 //      cluster (distributed shared memory);
-//   2. cluster barrier; the CTAs' counts of active chains travel with it, and the cluster
-//      leaves the loop when none is left;
-//   3. one thread issues the 3xTF32 tcgen05 MMAs of W (128 chains) x Phi slice (R rows);
+//   2. cluster barrier; a chain that is done has cleared its flag in every CTA by then, and the
+//      cluster leaves the loop when no flag is left;
+//   3. an extra warp issues the 3xTF32 tcgen05 MMAs of W (128 chains) x Phi slice (R rows); the
+//      chain warps meanwhile derive both continuations of the next step;
 //   4. every warp drains a lane quarter x column slice of the accumulator (thread = chain),
 //      sums (y - Phi w)^2 over its rows (fp32 over 32-row chunks, the chunks as an fp32
 //      pair) and stores the partial sum in the owner CTA's shared memory; cluster barrier.
 // The owner adds a chain's partial sums in a fixed butterfly order, so the sum is
-// deterministic.  Every
-// mbarrier wait is bounded: a CTA whose wait timed out reports it through its active count,
-// every CTA of the cluster then leaves at the same barrier, and the run's status gets
+// deterministic.
+// Bound: latency.  A step of 4096 x 32 over 16 CTAs is ~9.1 k cycles: chain step 1.6 k, rows to the
+// other CTAs 1.9 k (30 KB per CTA of distributed shared memory), barrier 1.2 k, MMAs with the
+// speculation 2.4 k, epilogue 1.4 k, second barrier.  11.8 k with the speculation between the
+// barriers, the epilogue's sums one multiply-add per instruction instead of two, and the
+// prior, the flags of all CTAs and both quantile tails read and done again every step.  One shell of
+// 512 chains x 160 slices: 2165 -> 1770 us.
+// Every
+// mbarrier wait is bounded: a CTA whose wait timed out tells every CTA before the next barrier of
+// 2., the cluster then leaves at that barrier together, and the run's status gets
 // GBNS_ERR_WAIT_TIMEOUT.
 
 struct LfArgs {
@@ -553,14 +566,15 @@ __device__ __forceinline__ uint32_t lf_sw128(int row, int k) {
   return (uint32_t)row * 128u + ((((uint32_t)k >> 2) ^ ((uint32_t)row & 7u)) << 4) + (((uint32_t)k & 3u) << 2);
 }
 
-constexpr int LF_ABORT = -(1 << 24);
 constexpr int LF_M_TILE = 128;  // chains per cluster tile (tensor-memory lanes)
 
-__global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ LfMaps maps, gbns_batch b,
+template <int THREADS, int PER_SM>
+__global__ void __launch_bounds__(THREADS, PER_SM) k_lg_shell_fused(const __grid_constant__ LfMaps maps, gbns_batch b,
                                                         gbns_lg_bufs lg, LfArgs la) {
   extern __shared__ unsigned char lf_dyn[];
   __shared__ __align__(8) unsigned long long bars[2];  // 0: Phi slice landed, 1: MMAs of a step done
   __shared__ uint32_t tmem_slot;
+  __shared__ int abort_here;  // a wait of this CTA timed out
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int CS = la.cs, R = la.rows, NKB = la.nkb, CPC = la.cpc, H = la.cpc / 4;
   const uint32_t rank = lf_cluster_rank();
@@ -580,19 +594,23 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
   const uint32_t w_hi = base + (uint32_t)(2 * NKB * R * 128), w_lo = w_hi + (uint32_t)(NKB * 16384);
   const uint32_t ys_s = w_lo + (uint32_t)(NKB * 16384);
   const uint32_t slots_s = ys_s + (uint32_t)(R * 4);                  // float2 [CS][H][CPC]
-  const uint32_t active_s = slots_s + (uint32_t)(CS * H * CPC * 8);   // int [CS]
+  const uint32_t alive_s = slots_s + (uint32_t)(CS * H * CPC * 8);    // int [128]: the chain is not done
+  const uint32_t abort_s = alive_s + 4u * LF_M_TILE;                  // int: some CTA's wait timed out
   // slots: fp32 pairs (hi, lo) [CS][H][CPC]
   auto gptr = [&](uint32_t sa) { return (void *)(lf_dyn + (sa - dyn0)); };
   float *ys = (float *)gptr(ys_s);
   const float2 *slots = (const float2 *)gptr(slots_s);
-  const int *active_in = (const int *)gptr(active_s);
+  volatile int *alive = (volatile int *)gptr(alive_s), *abort_all = (volatile int *)gptr(abort_s);
   const uint32_t bar_phi = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[1]);
 
   if (tid == 0) {
     mbar_init(bar_phi, 1);
     mbar_init(bar_mma, 1);
+    abort_here = 0;
+    *abort_all = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (tid < LF_M_TILE) alive[tid] = tile_c0 + tid < s;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"((uint32_t)R)
@@ -620,14 +638,14 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
         tma_load_2d(phi_lo + o, &maps.phi_lo, kb * TC_KB, brow + 128 * i, bar_phi);
       }
   }
-  int abort_local = 0;
-  if (nbox > 0) abort_local = __syncthreads_or(!mbar_wait(bar_phi, 0)) ? 1 : 0;
+  if (nbox > 0 && !mbar_wait(bar_phi, 0)) abort_here = 1;
 
   // ---- the owned chain (warp): seed point, keys (k_lg_init)
   const float *liveL = b.live_L[st.parity] + rd.live_off;
   const float Lstar = liveL[rd.s - 1];
   const int crow = (int)rank * CPC + warp;  // chain row in the tile
-  const int c = tile_c0 + crow;
+  const bool owner = warp < CPC;             // the last warp issues the MMAs
+  const int c = owner ? tile_c0 + crow : s;
   const int pa_ = lane, pb_ = lane + 32;
   const bool ha = pa_ < P, hb = pb_ < P;
   int flags = LG_DONE;
@@ -666,13 +684,17 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
   const float *fp = b.fparams + rd.param_off;
   const float sigma = fp[(size_t)N * P + N];
   const float inv2s2 = 0.5f / (sigma * sigma);
-  const int *kind = b.prior_kind + rd.prior_off;
-  const float *pra = b.prior_a + rd.prior_off, *prb = b.prior_b + rd.prior_off;
+  // what a step reads of the run and the prior, in registers (every asm below is a memory barrier)
+  const int kind_a = ha ? b.prior_kind[rd.prior_off + pa_] : 0, kind_b = hb ? b.prior_kind[rd.prior_off + pb_] : 0;
+  const float pra_a = ha ? b.prior_a[rd.prior_off + pa_] : 0.0f, pra_b = hb ? b.prior_a[rd.prior_off + pb_] : 0.0f;
+  const float prb_a = ha ? b.prior_b[rd.prior_off + pa_] : 0.0f, prb_b = hb ? b.prior_b[rd.prior_off + pb_] : 0.0f;
+  const bool midpoint = rd.midpoint != 0;
+  const int budget = b.max_evals_per_slice;
   lf_cluster_sync();  // every CTA initialised before the first remote store
 
   // ---- speculation.  Both possible continuations of a chain's next step are fixed by its
-  // keys, so each warp computes them while the cluster exchanges partial sums, off the critical
-  // path: the direction of the next slice (the normals of the current slice's after_key, lanes
+  // keys, so each warp computes them while the MMAs run, off the critical path (2,500 of a
+  // step's 11,800 cycles when they stood between the barriers): the direction of the next slice (the normals of the current slice's after_key, lanes
   // over dimensions), the keys and uniform of the next slice's first pick (B' = split(slices_key)[j],
   // then run / t / after keys), and the keys and uniform of the next shrink step (from the
   // current carry key).  The chain step then only selects.
@@ -680,39 +702,52 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
   // key B' and the keys and uniform of its first pick) is the same for every step of a slice:
   // it is derived at the slice's first step (spec_j records for which slice) and reused; only
   // the shrink continuation changes from step to step.
-  float sa_va = 0.f, sa_vb = 0.f, sa_nrm = 1.f, sa_u = 0.f, sr_u = 0.f;
+  float sa_da = 0.f, sa_db = 0.f, sa_alpha = 0.f, sa_u = 0.f, sr_u = 0.f;
   Key sa_ck = {0u, 0u}, sa_after = {0u, 0u}, sr_ck = {0u, 0u};
   int spec_j = -1;
+  auto bcast = [&](uint32_t x0, uint32_t x1, int from) {
+    return Key{__shfl_sync(0xffffffffu, x0, from), __shfl_sync(0xffffffffu, x1, from)};
+  };
+  // lanes 0-15 work on the next slice, 16-31 on the shrink step: three threefry blocks deep
   auto speculate = [&](Key next_dir_key, int next_j, Key cur_ck) {
+    const bool shrink = lane >= 16;
     uint32_t x0, x1;
     if (next_j != spec_j) {
       spec_j = next_j;
-      if (P > 1) {
-        sa_va = ha ? normal_from_bits(bits64(next_dir_key, (uint32_t)pa_)) : 0.0f;
-        sa_vb = hb ? normal_from_bits(bits64(next_dir_key, (uint32_t)pb_)) : 0.0f;
-        sa_nrm = sqrtf(warp_sum(fmaf(sa_va, sa_va, sa_vb * sa_vb)));
+      const uint64_t na = bits64(next_dir_key, (uint32_t)pa_);
+      // B' = fold(slices_key, next_j); the shrink's carry fold(ck, 0) and t key fold(ck, 1)
+      const Key k1 = shrink ? cur_ck : slices_key;
+      threefry2x32(k1.k0, k1.k1, 0u, shrink ? (uint32_t)(lane & 1) : (uint32_t)next_j, x0, x1);
+      sr_ck = bcast(x0, x1, 16);
+      const Key tkr = bcast(x0, x1, 17);
+      // lanes 0-2: run, t and after keys of B' (counters 0, 2, 3); 16-31: the shrink's 64 bits
+      if (shrink) {
+        x0 = tkr.k0;
+        x1 = tkr.k1;
       }
-      // B' = fold(slices_key, next_j); then lanes 0-2: its run, t and after keys (counters
-      // 0, 2, 3); then the first pick's 64 random bits
-      threefry2x32(slices_key.k0, slices_key.k1, 0u, (uint32_t)next_j, x0, x1);
       const uint32_t c2 = lane == 1 ? 2u : (lane == 2 ? 3u : 0u);
       threefry2x32(x0, x1, 0u, c2, x0, x1);
-      sa_ck.k0 = __shfl_sync(0xffffffffu, x0, 0);
-      sa_ck.k1 = __shfl_sync(0xffffffffu, x1, 0);
-      const Key tka = {__shfl_sync(0xffffffffu, x0, 1), __shfl_sync(0xffffffffu, x1, 1)};
-      sa_after.k0 = __shfl_sync(0xffffffffu, x0, 2);
-      sa_after.k1 = __shfl_sync(0xffffffffu, x1, 2);
-      threefry2x32(tka.k0, tka.k1, 0u, 0u, x0, x1);
-      sa_u = uniform01(((uint64_t)x0 << 32) | (uint64_t)x1);
+      sa_ck = bcast(x0, x1, 0);
+      const Key tka = bcast(x0, x1, 1), sb = bcast(x0, x1, 16);
+      sa_after = bcast(x0, x1, 2);
+      sr_u = uniform01(((uint64_t)sb.k0 << 32) | (uint64_t)sb.k1);
+      sa_u = uniform01(bits64(tka, 0u));
+      if (P > 1) {
+        const float va = ha ? normal_from_bits(na) : 0.0f;
+        const float vb = hb ? normal_from_bits(bits64(next_dir_key, (uint32_t)pb_)) : 0.0f;
+        const float nrm = sqrtf(warp_sum(fmaf(va, va, vb * vb)));
+        sa_da = va / nrm;
+        sa_db = vb / nrm;
+      } else {
+        sa_da = 1.0f;
+      }
+      sa_alpha = lg_alpha(next_j, S);
+    } else {
+      threefry2x32(cur_ck.k0, cur_ck.k1, 0u, (uint32_t)(lane & 1), x0, x1);
+      sr_ck = bcast(x0, x1, 0);
+      const Key tkr = bcast(x0, x1, 1);
+      sr_u = uniform01(bits64(tkr, 0u));
     }
-    // the shrink continuation -- lane 1: carry fold(ck, 0); lane 2: t key fold(ck, 1); then
-    // the t key's 64 random bits
-    threefry2x32(cur_ck.k0, cur_ck.k1, 0u, lane == 2 ? 1u : 0u, x0, x1);
-    sr_ck.k0 = __shfl_sync(0xffffffffu, x0, 1);
-    sr_ck.k1 = __shfl_sync(0xffffffffu, x1, 1);
-    const Key tkr = {__shfl_sync(0xffffffffu, x0, 2), __shfl_sync(0xffffffffu, x1, 2)};
-    threefry2x32(tkr.k0, tkr.k1, 0u, 0u, x0, x1);
-    sr_u = uniform01(((uint64_t)x0 << 32) | (uint64_t)x1);
   };
   if (!(flags & LG_DONE)) speculate(dir_key, 0, ck);
 
@@ -747,7 +782,7 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
         ++in_slice;
         const bool accept = (logL > Lstar) || ((logL0 == Lstar) && (logL == Lstar));
         start_now = false;
-        if (accept || in_slice >= b.max_evals_per_slice) {
+        if (accept || in_slice >= budget) {
           if (!accept) flags |= LG_FAILED;
           pair_add(ua, fmaf(t, da, la_), ua, la_);
           pair_add(ub, fmaf(t, db, lb), ub, lb);
@@ -774,48 +809,37 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
           b.new_E[rd.shell_off + c] = total;
           if (flags & LG_FAILED) atomicOr(&st.status, (int)GBNS_ERR_SHRINK_BUDGET);
         }
+        if (lane < CS) lf_st_s32(lf_mapa(alive_s + 4u * (uint32_t)crow, (uint32_t)lane), 0);
       } else {
         float u;
         if (start_now) {
-          if (P == 1) {
-            da = 1.0f;
-          } else {
-            da = sa_va / sa_nrm;
-            db = sa_vb / sa_nrm;
-          }
+          da = sa_da;
+          db = sa_db;
           ck = sa_ck;
           after_key = sa_after;
           u = sa_u;
-          alpha = lg_alpha(j, S);
-          float t1r = INFINITY, t1l = -INFINITY, t0r = INFINITY, t0l = -INFINITY;
+          alpha = sa_alpha;
+          Chord ch;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const bool have = h ? hb : ha;
             if (have) {
               const float uu = h ? ub : ua, ll = h ? lb : la_, dd = h ? db : da;
-              const float t1 = ((1.0f - uu) - ll) / dd, t0 = -(uu + ll) / dd;
-              t1r = fminf(t1r, t1 >= 0.f ? t1 : INFINITY);
-              t1l = fmaxf(t1l, t1 <= 0.f ? t1 : -INFINITY);
-              t0r = fminf(t0r, t0 >= 0.f ? t0 : INFINITY);
-              t0l = fmaxf(t0l, t0 <= 0.f ? t0 : -INFINITY);
+              ch.clip(((1.0f - uu) - ll) / dd);
+              ch.clip(-(uu + ll) / dd);
             }
           }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            t1r = fminf(t1r, __shfl_xor_sync(0xffffffffu, t1r, o));
-            t1l = fmaxf(t1l, __shfl_xor_sync(0xffffffffu, t1l, o));
-            t0r = fminf(t0r, __shfl_xor_sync(0xffffffffu, t0r, o));
-            t0l = fmaxf(t0l, __shfl_xor_sync(0xffffffffu, t0l, o));
-          }
-          right = fminf(t0r, t1r);
-          left = fmaxf(t0l, t1l);
+          ch.hi = __reduce_min_sync(0xffffffffu, ch.hi);
+          ch.lo = __reduce_min_sync(0xffffffffu, ch.lo);
+          right = ch.right();
+          left = ch.left();
           in_slice = 0;
         } else {
           ck = sr_ck;
           u = sr_u;
           if (t < 0.f) left = t;
           if (t > 0.f) right = t;
-          if (rd.midpoint) {
+          if (midpoint) {
             if (t < 0.f) left = alpha * left;
             if (t > 0.f) right = alpha * right;
           }
@@ -823,14 +847,14 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
         t = fmaf(u, right - left, left);
         // the proposal w as a TF32 hi / lo row of the W tile
         if (ha) {
-          const float w = prior_quantile_pair(kind[pa_], pra[pa_], prb[pa_], ua, fmaf(t, da, la_));
+          const float w = prior_quantile_pair(kind_a, pra_a, prb_a, ua, fmaf(t, da, la_));
           float h, l;
           tf32_split(w, h, l);
           *(float *)gptr(w_hi + lf_sw128(crow, pa_)) = h;
           *(float *)gptr(w_lo + lf_sw128(crow, pa_)) = l;
         }
         if (hb) {
-          const float w = prior_quantile_pair(kind[pb_], pra[pb_], prb[pb_], ub, fmaf(t, db, lb));
+          const float w = prior_quantile_pair(kind_b, pra_b, prb_b, ub, fmaf(t, db, lb));
           float h, l;
           tf32_split(w, h, l);
           *(float *)gptr(w_hi + 16384u + lf_sw128(crow, lane)) = h;
@@ -842,32 +866,35 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
     }
     __syncwarp();
     if (wrote) {
-      if (lane < 16 * NKB) {
-        // copy the row (hi and lo, NKB blocks of 128 bytes) to the other CTAs of the cluster
-        const int blk = lane >> 3, chunk = lane & 7;
+      {
+        // copy the row (hi and lo, NKB blocks of 128 bytes) to the other CTAs of the cluster; at one
+        // block the half-warps take every other CTA
+        const int blk = NKB == 1 ? (lane >> 3) & 1 : lane >> 3, chunk = lane & 7;
+        const int q_step = NKB == 1 ? 2 : 1;
         const uint32_t off = ((blk & 1) ? w_lo : w_hi) + (uint32_t)(blk >> 1) * 16384u + (uint32_t)crow * 128u +
                              (uint32_t)chunk * 16u;
         const uint4 v = *(const uint4 *)gptr(off);
-        for (int q = 0; q < CS; ++q)
+        for (int q = NKB == 1 ? lane >> 4 : 0; q < CS; q += q_step)
           if (q != (int)rank) lf_st_v4(lf_mapa(off, (uint32_t)q), v);
       }
       // the tensor cores of every CTA read the row through the async proxy
       asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
     }
-    const int act = __syncthreads_count(lane == 0 && !(flags & LG_DONE));
-    if (tid < CS) lf_st_s32(lf_mapa(active_s + 4u * rank, (uint32_t)tid), abort_local ? LF_ABORT : act);
-    lf_cluster_sync();  // (A) W tiles and active counts complete in every CTA
-    int total_active = 0;
-    for (int q = 0; q < CS; ++q) total_active += active_in[q];
-    if (total_active <= 0 || step >= lg.max_steps) {
+    if (warp == 0 && lane < CS && *(volatile int *)&abort_here) lf_st_s32(lf_mapa(abort_s, (uint32_t)lane), 1);
+    lf_cluster_sync();  // (A) W tiles, chains done and aborts known in every CTA
+    int left_over = 0;
+#pragma unroll
+    for (int q = 0; q < LF_M_TILE / 32; ++q) left_over |= alive[lane + 32 * q];
+    const bool any = __any_sync(0xffffffffu, left_over != 0), aborted = *abort_all != 0;
+    if (!any || aborted || step >= lg.max_steps) {
       if (tid == 0 && rank == 0) {
-        if (total_active < 0) atomicOr(&st.status, (int)GBNS_ERR_WAIT_TIMEOUT);
-        else if (total_active > 0) atomicOr(&st.status, (int)GBNS_ERR_SHRINK_BUDGET);
+        if (aborted) atomicOr(&st.status, (int)GBNS_ERR_WAIT_TIMEOUT);
+        else if (any) atomicOr(&st.status, (int)GBNS_ERR_SHRINK_BUDGET);
       }
       break;
     }
     // ---- 2. 3xTF32 MMAs: accumulator[chain][row] = W[chain] . Phi[row] over this CTA's rows
-    if (nbox > 0 && tid == 0) {
+    if (nbox > 0 && !owner && lane == 0) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       tc_fence_after();
       for (int nc = 0; nc * NMMA < nbox * 128; ++nc) {
@@ -881,12 +908,12 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
       tc_commit(bar_mma);
     }
     // ---- 3. epilogue: this warp's 32 chains x its column slice
+    // (while the MMAs run, the continuations of the next step)
+    if (flags & LG_PENDING) speculate(after_key, j + 1, ck);
     float part = 0.0f, part_lo = 0.0f;
-    if (nbox > 0) {
-      bool ok = mbar_wait(bar_mma, mma_phase);
-      ok = __syncthreads_and(ok);
-      if (!ok) {
-        abort_local = 1;
+    if (nbox > 0 && owner) {
+      if (!__all_sync(0xffffffffu, mbar_wait(bar_mma, mma_phase))) {
+        abort_here = 1;      // (reported at the next barrier A, where the whole cluster leaves)
         mma_pending = true;  // the phase stays the one still owed
       } else {
         mma_phase ^= 1u;
@@ -902,18 +929,14 @@ __global__ void __launch_bounds__(512) k_lg_shell_fused(const __grid_constant__ 
         }
       }
     }
-    {
+    if (owner) {
       const int row_c = qd * 32 + lane;  // chain row of this thread's accumulator lane
-      const int owner = row_c / CPC, lc = row_c - owner * CPC;
-      lf_st_f32x2(lf_mapa(slots_s + 8u * (uint32_t)(((int)rank * H + hs) * CPC + lc), (uint32_t)owner), part,
+      const int to = row_c / CPC, lc = row_c - to * CPC;
+      lf_st_f32x2(lf_mapa(slots_s + 8u * (uint32_t)(((int)rank * H + hs) * CPC + lc), (uint32_t)to), part,
                   part_lo);
     }
     tc_fence_before();
-    // (B) partial sums complete in their owners; the continuations of the next step are
-    // computed between the arrival and the wait
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    if (flags & LG_PENDING) speculate(after_key, j + 1, ck);
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    lf_cluster_sync();  // (B) partial sums complete in their owners
   }
   // a timed-out MMA may still be in flight: give it one more bounded wait before the
   // tensor memory is released
@@ -1304,6 +1327,11 @@ cudaError_t launch_lg_steps_tc(const gbns_batch &b, const gbns_lg_bufs &lg, int 
 }
 
 
+// The instantiation for 128 / CS chains per CTA (16 CTAs of 8 chain warps, two per SM where their
+// shared and tensor memory allow, or 8 of 16).
+using LfKernel = void (*)(LfMaps, gbns_batch, gbns_lg_bufs, LfArgs);
+static LfKernel lf_kernel(int cpc) { return cpc <= 8 ? k_lg_shell_fused<288, 2> : k_lg_shell_fused<544, 1>; }
+
 // Launch configuration of the fused shell: clusters of lg.cluster_size CTAs over lg.items_fused.
 static cudaError_t lf_config(const gbns_lg_bufs &lg, cudaStream_t s, cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr,
                              LfArgs &la) {
@@ -1316,17 +1344,17 @@ static cudaError_t lf_config(const gbns_lg_bufs &lg, cudaStream_t s, cudaLaunchC
   // SM's shared memory, so that the CTAs resident on one SM never ask for more than its 512
   // tensor-memory columns (an allocation that has to wait could stall a cluster barrier)
   size_t smem = 1024 + (size_t)2 * nkb * R * 128 + (size_t)2 * nkb * 16384 + (size_t)R * 4 +
-                (size_t)cs * (cpc / 4) * cpc * 8 + (size_t)cs * 4;
+                (size_t)cs * (cpc / 4) * cpc * 8 + (size_t)(LF_M_TILE + 1) * 4;
   const size_t per_sm = 233472, floor_bytes = per_sm / (size_t)(512 / R + 1) + 1;
   if (smem < floor_bytes) smem = floor_bytes;
   if (smem > 232448) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_lg_shell_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess && cs > 8)
-    e = cudaFuncSetAttribute(k_lg_shell_fused, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  const auto k = lf_kernel(cpc);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && cs > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   cfg = cudaLaunchConfig_t{};
   cfg.gridDim = dim3((unsigned)(lg.num_items_fused * cs));
-  cfg.blockDim = dim3((unsigned)(32 * cpc));
+  cfg.blockDim = dim3((unsigned)(32 * cpc + 32));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1352,7 +1380,7 @@ cudaError_t launch_lg_shell_fused(const gbns_batch &b, const gbns_lg_bufs &lg, c
   if (!encode_rows(&maps.phi_hi, lg.Phi_hi, lg.total_rows, 64, 128) ||
       !encode_rows(&maps.phi_lo, lg.Phi_lo, lg.total_rows, 64, 128))
     return cudaErrorInvalidValue;
-  e = cudaLaunchKernelEx(&cfg, k_lg_shell_fused, maps, b, lg, la);
+  e = cudaLaunchKernelEx(&cfg, lf_kernel(la.cpc), maps, b, lg, la);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
@@ -1364,7 +1392,7 @@ cudaError_t lg_fused_max_clusters(const gbns_lg_bufs &lg, int *out) {
   LfArgs la;
   cudaError_t e = lf_config(lg, 0, cfg, attr, la);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveClusters(out, k_lg_shell_fused, &cfg);
+  return cudaOccupancyMaxActiveClusters(out, lf_kernel(la.cpc), &cfg);
 }
 
 cudaError_t launch_adjoint_tc(const double *U, const double *log_w, long long M, int P, const float *Phi, const float *y,
