@@ -241,14 +241,21 @@ __global__ void __launch_bounds__(128, DMAX == 32 ? 4 : 3)
         }
         // ---- x - mu of the proposal into this lane's column of Delta
         if (all_uniform) {
-          for (int dd = 0; dd < D; dd += 4) {
-            const float4 dv = *reinterpret_cast<const float4 *>(&B.d[row][dd]);
-            const float4 uv = *reinterpret_cast<const float4 *>(&W.U0[g][dd]);
-            const float dq[4] = {dv.x, dv.y, dv.z, dv.w}, uq[4] = {uv.x, uv.y, uv.z, uv.w};
+          // (all loads of a trip before its stores, which the compiler may not move them across; the
+          // rows above D are not read)
+          for (int dd = 0; dd < D; dd += 8) {
+            float4 dv[2], uv[2], q[8];
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-              const float4 q = W.ab[dd + x];
-              W.DEL[dd + x][lane] = fmaf(q.y, fmaf(t_mine, dq[x], uq[x]), q.x) - q.z;
+            for (int h = 0; h < 2; ++h) {
+              dv[h] = *reinterpret_cast<const float4 *>(&B.d[row][dd + 4 * h]);
+              uv[h] = *reinterpret_cast<const float4 *>(&W.U0[g][dd + 4 * h]);
+            }
+#pragma unroll
+            for (int x = 0; x < 8; ++x) q[x] = W.ab[dd + x];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+              const float dq = (&dv[x >> 2].x)[x & 3], uq = (&uv[x >> 2].x)[x & 3];
+              W.DEL[dd + x][lane] = fmaf(q[x].y, fmaf(t_mine, dq, uq), q[x].x) - q[x].z;
             }
           }
         } else {
@@ -372,18 +379,19 @@ static cudaError_t launch_spec_mvn(const gbns_batch &b, int ib, int ie, int per_
 // over an item's chains).  Measured on one GB300, us per shell of 5 D slices, warp-cooperative
 // against 16 / 8 / 4 proposals per round:
 //   chains   D = 24                          chains   D = 48
-//      360   2722 |  283  314  428              720    7375 |  1159 1245  1586
-//    1,440   2915 |  570  337  449            2,880    7435 |  4623 2742  1674
-//    5,760   2986 | 1496 1011  933            5,760    7477 |  8261 5171  3539
-//   11,520   3029 | 2936 1767 1457           11,520    7526 | 15196 9108  6424
-//   23,040   3052 | 5672 3487 2559           23,040    7554 | 29954 16986 11393
+//      360   2719 |  248  275  372              720    7394 |   993 1096  1381
+//    1,440   2875 |  503  304  396            2,880    7439 |  3984 2463  1506
+//    5,760   2993 | 1325  917  844            5,760    7468 |  7126 4507  3196
+//   11,520   3027 | 2598 1623 1330           11,520    7532 | 13018 8183  5755
+//   23,040   3055 | 5041 3192 2348           23,040    7560 | 25624 15084 10204
+// (A trip's loads of the proposals before its stores: 283 -> 248 and 1159 -> 993 us for one run.)
 // The warp-cooperative kernel stays at its latency until its CTAs fill the SMs (~39 k chains at
 // D > 32); this kernel's time grows with the chains beyond one wave of CTAs.
 static int spec_mvn_lanes(const gbns_batch &b, int dmax, long long chains) {
   if (b.gradient_guided || b.gradient_slice) return 0;
   if (chains <= 1024) return 16;
   if (chains <= (dmax > 32 ? 1536 : 2048)) return 8;
-  if (chains <= (dmax > 32 ? 13000 : 27000)) return 4;
+  if (chains <= (dmax > 32 ? 15000 : 29000)) return 4;
   return 0;
 }
 
