@@ -868,14 +868,15 @@ __global__ void __launch_bounds__(THREADS, PER_SM) k_lg_shell_fused(const __grid
     if (wrote) {
       {
         // copy the row (hi and lo, NKB blocks of 128 bytes) to the other CTAs of the cluster; at one
-        // block the half-warps take every other CTA
+        // block the half-warps take every other CTA.  Every CTA starts at its own neighbour, so that no
+        // CTA receives from all the others at once.
         const int blk = NKB == 1 ? (lane >> 3) & 1 : lane >> 3, chunk = lane & 7;
         const int q_step = NKB == 1 ? 2 : 1;
         const uint32_t off = ((blk & 1) ? w_lo : w_hi) + (uint32_t)(blk >> 1) * 16384u + (uint32_t)crow * 128u +
                              (uint32_t)chunk * 16u;
         const uint4 v = *(const uint4 *)gptr(off);
-        for (int q = NKB == 1 ? lane >> 4 : 0; q < CS; q += q_step)
-          if (q != (int)rank) lf_st_v4(lf_mapa(off, (uint32_t)q), v);
+        for (int i = 1 + (NKB == 1 ? lane >> 4 : 0); i < CS; i += q_step)
+          lf_st_v4(lf_mapa(off, (rank + (uint32_t)i) & (uint32_t)(CS - 1)), v);
       }
       // the tensor cores of every CTA read the row through the async proxy
       asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
