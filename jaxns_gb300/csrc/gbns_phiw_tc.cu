@@ -509,11 +509,11 @@ __global__ void __launch_bounds__(SR_THREADS) k_lg_resid_tc(const __grid_constan
 // The owner adds a chain's partial sums in a fixed butterfly order, so the sum is
 // deterministic.
 // Bound: latency.  A step of 4096 x 32 over 16 CTAs is ~9.1 k cycles: chain step 1.6 k, rows to the
-// other CTAs 1.9 k (30 KB per CTA of distributed shared memory), barrier 1.2 k, MMAs with the
+// other CTAs 1.7 k (30 KB per CTA of distributed shared memory), barrier 1.1 k, MMAs with the
 // speculation 2.4 k, epilogue 1.4 k, second barrier.  11.8 k with the speculation between the
 // barriers, the epilogue's sums one multiply-add per instruction instead of two, and the
 // prior, the flags of all CTAs and both quantile tails read and done again every step.  One shell of
-// 512 chains x 160 slices: 2165 -> 1770 us.
+// 512 chains x 160 slices: 2165 -> 1680 us.
 // Every
 // mbarrier wait is bounded: a CTA whose wait timed out tells every CTA before the next barrier of
 // 2., the cluster then leaves at that barrier together, and the run's status gets

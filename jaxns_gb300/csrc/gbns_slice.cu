@@ -9,7 +9,7 @@
 // in registers; the run's parameters (mu, Linv, prior tables) sit in shared memory and
 // are read as broadcasts because every thread of a CTA works on chains of the same run.
 //
-// Bound: instructions (77 % of the issue slots, ALU pipe 62 %, 19 of 32 lanes).  D = 10 shells: 8.3
+// Bound: instructions (70-77 % of the issue slots, ALU pipe 66 %, 25 of 32 lanes).  D = 10 shells: 8.3
 // evaluations per slice with three threefry blocks each, and ten normals, are 55 % of them.  1024
 // runs x 500 chains, us per shell: 4740; bits to floats by two conversions and one multiply-add
 // instead of a 64-bit normalisation, chord ends by integer minima, the rounds' additions on the
