@@ -410,36 +410,85 @@ __global__ void k_rng(int mode, const uint32_t *key, const uint32_t *counts, voi
 // sample_evidence (utils.py:433-484): S replicas of log Z with the shrinkage drawn.
 // Replica s: u_i = uniform(split(split(key, S)[s], M)[i]), log T_i = log(u_i) / n_i,
 // log X_i = sum_{j<i} log T_j, and log Z = log sum_i X_i (1 - T_i) L_i -- the sequential LogSpace
-// accumulation of the reference as a composition of ranges: a range has the sum of its log T and
-// the log of its sum started at X = 1, and (s1, v1) before (s2, v2) is (s1 + s2, logaddexp(v1,
-// s1 + v2)).
+// accumulation of the reference as a composition of ranges: a range has the sum s of its log T and
+// its sum started at X = 1 as a exp(m), and (s1, a1, m1) before (s2, a2, m2) is (s1 + s2, a1 exp(m1)
+// + a2 exp(m2 + s1)), kept at the larger exponent.
 // A cluster of CS blocks takes RG replicas, block q the q-th part of the samples; a thread takes up
 // to SE_K consecutive samples of its tile and walks them once per replica in linear space from X = 1,
 // with the samples' 1 / n and exp(L - the thread's largest L) formed once for all replicas:
 // -expm1(log T) = 1 - T keeps its relative precision, X T = X + X expm1(log T).  Threads are composed
 // by a block scan of the log T sums and one log-sum-exp, tiles in order, blocks through distributed
 // shared memory.
-// Bound: FP64 (~2 lanes per clock and SM): one logarithm, a degree-8 Taylor polynomial of expm1
-// where |log T| < 1/32 (the function elsewhere) and five multiply-adds per sample and replica, ~45
-// instructions; one block per replica with a scan, a division, two exponentials and two
-// logarithms per sample took ~130 and left 52 of 152 SMs idle at S = 100 (100 replicas of 22,000
-// samples 835 -> 396 us a call, results to the last bits).
+// Bound: FP64 (~2 lanes per clock and SM): per sample and replica a table-driven logarithm (12
+// operations), a degree-8 Taylor polynomial of expm1 where |log T| < 1/32 (the function elsewhere)
+// and five multiply-adds.  100 replicas of 22,000 samples, a call: one block per replica with a scan,
+// a division, two exponentials and two logarithms per sample (52 of 152 SMs idle) 835 us; clusters
+// and the library's logarithm 400 us, this 260 us.  Error of log Z against extended precision, rms in
+// units of 1e-17 at 1,500 / 5,000 / 22,000 / 60,000 samples: 6.3 / 5.8 / 6.2 / 7.3 (6.1 / 6.3 / 8.1 / 7.6
+// one block per replica; 9 to 10 with the ranges' sums kept as logarithms).
 constexpr int SE_T = 256;
 constexpr int SE_K = 16;
 
 struct SeSmem {
   double scan[SE_T / 32], red[32];
-  double part_s[4], part_v[4];  // this block's (sum of log T, log of the range's sum) per replica
+  // this block's range per replica: sum of log T; the range's sum a exp(m)
+  double part_s[4], part_m[4], part_a[4];
 };
 
-__device__ __forceinline__ double lae_fin(double a, double b) {  // logaddexp for values in [-inf, +inf)
-  const double m = fmax(a, b);
-  return m > -INFINITY ? m + log(exp(a - m) + exp(b - m)) : a + b;  // NaN stays NaN
+// Tables of the logarithm (P. T. P. Tang, "Table-driven implementation of the logarithm function in
+// IEEE floating-point arithmetic", ACM TOMS 16, 1990): the reciprocal of the middle of each 128th
+// of [1, 2) rounded to fp32 and minus its logarithm, halved from sqrt(2) on; e ln 2.
+struct SeLog {
+  double2 c[128];
+  double e[64];
+};
+
+__device__ __forceinline__ void se_log_tables(SeLog &T) {
+  for (int i = threadIdx.x; i < 128; i += blockDim.x) {
+    const bool half = i >= 54;  // 1 + 54 / 128 > sqrt(2): m / 2
+    const double mid = (1.0 + ((double)i + 0.5) / 128.0) * (half ? 0.5 : 1.0);
+    // the cells next to 1 take 1 itself: m - 1 is exact there and the logarithm keeps its relative precision
+    const double inv = i == 0 || i == 127 ? 1.0 : (double)(float)(1.0 / mid);
+    T.c[i] = make_double2(half ? 0.5 * inv : inv, -log(inv));
+  }
+  for (int i = threadIdx.x; i < 64; i += blockDim.x) T.e[i] = -(double)i * GBNS_LN2;
 }
 
-// expm1(x), x <= 0
+// log(M 2^-52), M < 2^52: M = 2^k m, m in [1, 2), and log = e ln 2 - log(inv) + log1p(m inv - 1) with
+// |m inv - 1| <= 1 / 128, a Taylor polynomial through the eighth power.
+__device__ __forceinline__ double se_log(const SeLog &T, uint64_t M) {
+  if (M == 0ull) return -INFINITY;
+  const int nz = __clzll((long long)M);  // 12 .. 63
+  const uint64_t frac = ((M << nz) & 0x7FFFFFFFFFFFFFFFull) >> 11;  // the 52 bits below the first
+  const int i = (int)(frac >> 45);
+  const double2 c = T.c[i];
+  const double m = __longlong_as_double((long long)(0x3FF0000000000000ull | frac));
+  const double x = fma(m, c.x, -1.0);
+  double p = -1.0 / 8.0;
+  p = fma(p, x, 1.0 / 7.0);
+  p = fma(p, x, -1.0 / 6.0);
+  p = fma(p, x, 1.0 / 5.0);
+  p = fma(p, x, -1.0 / 4.0);
+  p = fma(p, x, 1.0 / 3.0);
+  p = fma(p, x, -1.0 / 2.0);
+  const int down = nz - 11 - (i >= 54);  // u = m 2^(11 - nz)
+  return (T.e[down] + c.y) + fma(p * x, x, x);
+}
+
+// a exp(m) += b exp(at + lo)
+__device__ __forceinline__ void se_add(double &m, double &a, double at, double lo, double b) {
+  if (at > m) {
+    a = b + (m > -INFINITY ? a * exp((m - at) - lo) : 0.0);
+    m = at;
+    a = lo != 0.0 ? a * (1.0 + lo) : a;  // (|lo| is half a unit of the last place of at)
+  } else if (at > -INFINITY) {
+    a = fma(b, exp((at - m) + lo), a);
+  }
+}
+
+// expm1(x)
 __device__ __forceinline__ double se_expm1(double x) {
-  if (fabs(x) < 0.03125) {
+  if ((uint32_t)(__double2hiint(x) & 0x7fffffff) < 0x3fa00000u) {  // |x| < 1/32
     double p = 1.0 / 40320.0;
     p = fma(p, x, 1.0 / 5040.0);
     p = fma(p, x, 1.0 / 720.0);
@@ -458,15 +507,17 @@ __global__ void __launch_bounds__(SE_T) k_sample_evidence(const uint32_t *key, c
                                                           double *__restrict__ out) {
   extern __shared__ __align__(16) double2 se_dyn[];  // [SE_K][SE_T]: 1 / n and exp(L - ref) of the thread's samples
   __shared__ SeSmem sm;
+  __shared__ SeLog lt_tab;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = SE_T / 32;
+  se_log_tables(lt_tab);
+  __syncthreads();
   const int rank = blockIdx.x % CS, s0 = blockIdx.x / CS * RG;
   const Key kroot = {key[0], key[1]};
   const long long lo = M * rank / CS, hi = M * (rank + 1) / CS;
-  double run_s[RG], run_v[RG];
-#pragma unroll
-  for (int g = 0; g < RG; ++g) {
-    run_s[g] = 0.0;
-    run_v[g] = -INFINITY;
+  if (tid < RG) {
+    sm.part_s[tid] = 0.0;
+    sm.part_m[tid] = -INFINITY;
+    sm.part_a[tid] = 0.0;
   }
   for (long long base = lo; base < hi; base += (long long)SE_T * SE_K) {
     const int len = (int)min((long long)SE_T * SE_K, hi - base), per = (len + SE_T - 1) / SE_T;
@@ -486,14 +537,13 @@ __global__ void __launch_bounds__(SE_T) k_sample_evidence(const uint32_t *key, c
       double X = 1.0, A = 0.0, sum = 0.0;
       for (int k = 0; k < cnt; ++k) {
         const double2 f = se_dyn[k * SE_T + tid];
-        const double lt = log(uniform01_d(bits64(fold(ks, (uint32_t)(i0 + k)), 0u))) * f.x;
+        const double lt = se_log(lt_tab, bits64(fold(ks, (uint32_t)(i0 + k)), 0u) >> 12) * f.x;
         const double em = se_expm1(lt);  // T - 1
         const double d = X * em;
         if (__double2hiint(lt) < 0) A = fma(-d, f.y, A);  // T > 1 (a negative count): 1 - T has no log
         X += d;
         sum += lt;
       }
-      const double v = A > 0.0 ? ref + log(A) : -INFINITY;
       // log X at this thread's first sample: exclusive block scan of the sums
       double incl = sum;
 #pragma unroll
@@ -503,14 +553,16 @@ __global__ void __launch_bounds__(SE_T) k_sample_evidence(const uint32_t *key, c
       }
       if (lane == 31) sm.scan[warp] = incl;
       __syncthreads();
-      double before = run_s[g], total = run_s[g];
+      double before = sm.part_s[g], total = before;
       for (int w = 0; w < nw; ++w) {
         if (w < warp) before += sm.scan[w];
         total += sm.scan[w];
       }
       const double prev = __shfl_up_sync(0xffffffffu, incl, 1);
       if (lane > 0) before += prev;
-      const double term = v > -INFINITY ? before + v : -INFINITY;
+      // the thread's part is A exp(term); the parts keep their own exponents to the end, so that each
+      // one's rounding is its own and no logarithm of a partial sum is rounded at the size of log Z
+      const double term = A != 0.0 ? before + ref : -INFINITY;
       double mx = term;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -518,7 +570,7 @@ __global__ void __launch_bounds__(SE_T) k_sample_evidence(const uint32_t *key, c
       __syncthreads();
       mx = sm.red[0];
       for (int w = 1; w < nw; ++w) mx = fmax(mx, sm.red[w]);
-      double a = term > -INFINITY ? exp(term - mx) : 0.0;
+      double a = term > -INFINITY ? A * exp(term - mx) : 0.0;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       __syncthreads();
@@ -527,40 +579,30 @@ __global__ void __launch_bounds__(SE_T) k_sample_evidence(const uint32_t *key, c
       if (tid == 0) {
         double sa = 0.0;
         for (int w = 0; w < nw; ++w) sa += sm.red[w];
-        sm.part_v[g] = mx > -INFINITY ? lae_fin(run_v[g], mx + log(sa)) : run_v[g];
+        se_add(sm.part_m[g], sm.part_a[g], mx, 0.0, sa);
+        sm.part_s[g] = total;
       }
       __syncthreads();
-      // (all run_s, run_v have a static index only after unrolling: select)
-#pragma unroll
-      for (int q = 0; q < RG; ++q)
-        if (q == g) {
-          run_s[q] = total;
-          run_v[q] = sm.part_v[g];
-        }
     }
   }
-  if (tid == 0)
-#pragma unroll
-    for (int g = 0; g < RG; ++g) {
-      sm.part_s[g] = run_s[g];
-      sm.part_v[g] = run_v[g];
-    }
+  __syncthreads();
   if (CS > 1) {
     cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
     if (rank == 0 && tid < RG && tid < S - s0) {
-      double s = 0.0, v = -INFINITY;
+      double s = 0.0, m = -INFINITY, a = 0.0;
       for (int q = 0; q < CS; ++q) {
         const SeSmem *o = cluster.map_shared_rank(&sm, q);
-        v = lae_fin(v, s + o->part_v[tid]);
+        const double at = s + o->part_m[tid], bb = at - s;
+        const double lo = fabs(at) < INFINITY ? (s - (at - bb)) + (o->part_m[tid] - bb) : 0.0;  // TwoSum
+        se_add(m, a, at, lo, o->part_a[tid]);
         s += o->part_s[tid];
       }
-      out[s0 + tid] = v;
+      out[s0 + tid] = m > -INFINITY ? m + log(a) : -INFINITY;
     }
     cluster.sync();
-  } else {
-    __syncthreads();
-    if (tid < RG && tid < S - s0) out[s0 + tid] = sm.part_v[tid];
+  } else if (tid < RG && tid < S - s0) {
+    out[s0 + tid] = sm.part_m[tid] > -INFINITY ? sm.part_m[tid] + log(sm.part_a[tid]) : -INFINITY;
   }
 }
 
