@@ -896,10 +896,12 @@ cudaError_t launch_results(const gbns_batch &b, const gbns_results_bufs &res, cu
   return cudaGetLastError();
 }
 
-// One block up to this many samples, a team of one block per SM beyond (gbns_results_team.cu): the
-// team pays about 17 us of grid barriers and prologue whatever the size, one block about 1 us per
-// 1000 samples in order (8 us per 1000 for the evidence) and more out of order.
-constexpr long long TEAM_MIN_SAMPLES = 16384;
+// One block up to this many samples, a team of up to one block per SM beyond (gbns_results_team.cu):
+// the team pays its grid barriers whatever the size, one block its passes.  Live-point counts and
+// evidence through the package, us (one block / team), in order and with phantoms out of order:
+// 1000 samples 67 / 69, 67 / 81; 2000 67 / 70, 80 / 83; 4000 76 / 70, 241 / 156; 8000 115 / 72,
+// 335 / 134; 16000 197 / 70, 720 / 174.
+constexpr long long TEAM_MIN_SAMPLES = 3000;
 
 cudaError_t launch_count_crossed_edges(const int *sender, const float *L, long long N, int *samples_indices,
                                        int *num_live, long long *scratch_ll, int *scratch_i, cudaStream_t stream) {

@@ -95,3 +95,10 @@ def test_team_launches_are_capturable(gpu_lib):
     graph.replay()
     torch.cuda.synchronize()
     np.testing.assert_array_equal(again["scalars"].cpu().numpy(), out["scalars"].cpu().numpy())
+
+
+@pytest.mark.parametrize("N,live,shuffle", [(2999, 50, True), (3000, 50, False), (3000, 400, True), (3001, 100, True),
+                                            (7001, 300, True)])
+@pytest.mark.parametrize("lz", [True, False])
+def test_sets_at_the_hand_over_match_the_oracle(gpu_lib, oracle_mod, N, live, shuffle, lz):
+    test_long_sets_match_the_oracle(gpu_lib, oracle_mod, N, live, shuffle, lz)
