@@ -107,7 +107,10 @@ __device__ __forceinline__ unsigned long long sort_key(float L, int i) {
 // Bitonic sort of NP (power of two) 64-bit keys in shared memory, ascending, by the first
 // `threads` threads of the CTA (a multiple of 32; the others must not call).  A warp's pairs of a
 // stride up to 32 lie in its own 64 keys, so only the wider strides need the barrier.
-__device__ __forceinline__ void sort_barrier(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
+__device__ __forceinline__ void sort_barrier(int threads) {
+  __syncwarp();  // an aligned barrier takes whole warps: the lanes leave the loops before it at different trips
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
 
 __device__ void cta_bitonic(unsigned long long *k, int NP, int threads) {
   bool wide = true;  // the keys, or the previous stage, came from other warps

@@ -536,7 +536,10 @@ __device__ __forceinline__ uint32_t lf_cluster_rank() {
   return r;
 }
 
+// The aligned barrier takes whole warps: the lane that issues the MMAs, and lanes that leave the row
+// copies or the abort stores at different trips, rejoin their warp before it.
 __device__ __forceinline__ void lf_cluster_sync() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
@@ -611,6 +614,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM) k_lg_shell_fused(const __grid
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (tid < LF_M_TILE) alive[tid] = tile_c0 + tid < s;
+  __syncwarp();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"((uint32_t)R)

@@ -65,6 +65,7 @@ __device__ float lgp_sum(LgpSmem &sm, float *phi, const float *__restrict__ Phi,
       } else {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
+      __syncwarp();  // (an aligned barrier takes whole warps)
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const int i = tid & (LGP_ROWS - 1), row = ps * LGP_ROWS + i, p0 = tid < LGP_ROWS ? 0 : 4;
       if (row < N) {

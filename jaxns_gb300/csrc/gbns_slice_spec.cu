@@ -43,7 +43,10 @@ struct SpecTeam {
   uint16_t tails[2][32 * DMAX];
 };
 
-__device__ __forceinline__ void team_barrier(int id) { asm volatile("bar.sync %0, 96;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void team_barrier(int id) {
+  __syncwarp();  // (an aligned barrier takes whole warps)
+  asm volatile("bar.sync %0, 96;" ::"r"(id) : "memory");
+}
 
 // Directions (and reciprocals) of the rows in `rows`: D normals per row, flattened over the
 // warp, then normalised one row per lane in dimension order.

@@ -71,7 +71,10 @@ __device__ __forceinline__ void spec_directions_w(SpecRows<DMAX> &B, uint4 *key,
 }
 
 // A barrier of the CTA that its consumer and producer warps reach at their own places.
-__device__ __forceinline__ void cta_barrier() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void cta_barrier() {
+  __syncwarp();  // (an aligned barrier takes whole warps)
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+}
 
 template <int DMAX, int G>
 __global__ void __launch_bounds__(128, DMAX == 32 ? 4 : 3)
