@@ -155,10 +155,9 @@ __device__ __forceinline__ void copy_words(float *__restrict__ dst, const float 
 __device__ void store_append(const gbns_batch &b, const gbns_run_desc &rd, long long nsi, long long cnt,
                              const float *L, const int *S, int S_const, const int *E, const float *U, int phantom, int t0,
                              int nt) {
+  if (cnt > rd.cap) cnt = rd.cap;  // more than the store holds (a capacity below one shell, or below the live set)
   if (cnt <= 0) return;
-  long long start = nsi;
-  if (start > rd.cap - cnt) start = rd.cap - cnt;
-  if (start < 0) start = 0;
+  const long long start = min(nsi, rd.cap - cnt);
   const int W = rd.ucols;
   for (long long i = t0; i < cnt; i += nt) {
     const long long o = rd.store_off + start + i;
