@@ -149,24 +149,42 @@ __device__ __forceinline__ void copy_words(float *__restrict__ dst, const float 
   for (; q < cnt; q += nt) dst[q] = src[q];
 }
 
-// Append cnt entries of a run to its store at next_sample_idx, with the start clamped like
-// lax.dynamic_update_slice (internals/maps.py:15-25, sharded_static.py:40-85); by threads
-// t0, t0 + nt, ...
-__device__ void store_append(const gbns_batch &b, const gbns_run_desc &rd, long long nsi, long long cnt,
-                             const float *L, const int *S, int S_const, const int *E, const float *U, int phantom, int t0,
-                             int nt) {
-  if (cnt > rd.cap) cnt = rd.cap;  // more than the store holds (a capacity below one shell, or below the live set)
+// Slots of a run's store: first of them, and their number.
+struct StoreRange {
+  long long start, cnt;
+};
+
+// Where cnt entries appended at nsi go: the start clamped like lax.dynamic_update_slice
+// (internals/maps.py:15-25, sharded_static.py:40-85), and no more than the store holds (a capacity
+// below one shell, or below the live set).
+__device__ __forceinline__ StoreRange store_range(const gbns_run_desc &rd, long long nsi, long long cnt) {
+  if (cnt > rd.cap) cnt = rd.cap;
+  return {min(nsi, rd.cap - cnt), cnt};
+}
+
+// The first to.cnt of a run's entries to its store, by threads t0, t0 + nt, ...; slots of `later`,
+// which an append that comes after this one writes, are left to it (the two may run side by side).
+__device__ void store_append(const gbns_batch &b, const gbns_run_desc &rd, StoreRange to, StoreRange later, const float *L,
+                             const int *S, int S_const, const int *E, const float *U, int phantom, int t0, int nt) {
+  const long long cnt = to.cnt;
   if (cnt <= 0) return;
-  const long long start = min(nsi, rd.cap - cnt);
+  // entries [0, head) and [tail, cnt) are outside `later`
+  const long long head = later.cnt > 0 ? min(max(later.start - to.start, 0ll), cnt) : cnt;
+  const long long tail = later.cnt > 0 ? min(max(later.start + later.cnt - to.start, head), cnt) : cnt;
   const int W = rd.ucols;
   for (long long i = t0; i < cnt; i += nt) {
-    const long long o = rd.store_off + start + i;
+    if (i >= head && i < tail) continue;
+    const long long o = rd.store_off + to.start + i;
     b.store_L[o] = L[i];
     b.store_S[o] = S ? S[i] : S_const;
     b.store_E[o] = E ? E[i] : 0;
     b.store_P[o] = (uint8_t)phantom;
   }
-  if (rd.ustore_off >= 0 && b.store_U) copy_words(b.store_U + rd.ustore_off + start * W, U, cnt * W, t0, nt);
+  if (rd.ustore_off >= 0 && b.store_U) {
+    float *dst = b.store_U + rd.ustore_off + to.start * W;
+    copy_words(dst, U, head * W, t0, nt);
+    if (tail < cnt) copy_words(dst + tail * W, U + tail * W, (cnt - tail) * W, t0, nt);
+  }
 }
 
 // ------------------------------------------------------------------ init ----
@@ -545,10 +563,9 @@ __global__ void __launch_bounds__(512, 1) k_merge(gbns_batch b) {
       oS[i] = fresh ? sender_idx : Sd[f];
     }
     // the discarded shell and the phantoms (add_phantom_samples_to_state, sharded_static.py:181-207)
-    store_append(b, rd, nsi0, s, L, Sd, 0, E, U, 0, t0, nt);
-    if (K > 0)
-      store_append(b, rd, nsi1, (long long)s * K, b.ph_L + rd.phL_off, nullptr, sender_idx, nullptr, b.ph_U + rd.phU_off,
-                   1, t0, nt);
+    const StoreRange none = {0, 0}, ph = store_range(rd, nsi1, (long long)s * K);
+    store_append(b, rd, store_range(rd, nsi0, s), ph, L, Sd, 0, E, U, 0, t0, nt);
+    store_append(b, rd, ph, none, b.ph_L + rd.phL_off, nullptr, sender_idx, nullptr, b.ph_U + rd.phU_off, 1, t0, nt);
   }
 
   // ---- register and termination
@@ -726,7 +743,7 @@ __global__ void __launch_bounds__(512, 1) k_merge(gbns_batch b) {
   const long long nsi2 = (nsi1 + (long long)s * K) % cap;
   if (sm.done) {
     // consume the live points (sharded_static.py:833-838)
-    store_append(b, rd, nsi2, n, b.live_L[npar] + o, b.live_S[npar] + o, 0, b.live_E[npar] + o,
+    store_append(b, rd, store_range(rd, nsi2, n), {0, 0}, b.live_L[npar] + o, b.live_S[npar] + o, 0, b.live_E[npar] + o,
                  b.live_U[npar] + rd.liveU_off, 0, tid, T);
     __syncthreads();
   }
@@ -750,8 +767,8 @@ __global__ void k_finalize(gbns_batch b) {
   if (st.phase == 2 || !st.done) return;
   const int par = st.parity;
   const long long o = rd.live_off;
-  store_append(b, rd, st.next_sample_idx, rd.n, b.live_L[par] + o, b.live_S[par] + o, 0, b.live_E[par] + o,
-               b.live_U[par] + rd.liveU_off, 0, threadIdx.x, blockDim.x);
+  store_append(b, rd, store_range(rd, st.next_sample_idx, rd.n), {0, 0}, b.live_L[par] + o, b.live_S[par] + o, 0,
+               b.live_E[par] + o, b.live_U[par] + rd.liveU_off, 0, threadIdx.x, blockDim.x);
   __syncthreads();
   if (threadIdx.x == 0) {
     st.next_sample_idx = (st.next_sample_idx + rd.n) % rd.cap;

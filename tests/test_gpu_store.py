@@ -38,3 +38,28 @@ def test_appends_stay_in_the_store(gpu_lib, oracle_mod, n, s, K, cap):
     live = both.live_view(0)["log_L_raw"].cpu().numpy()
     if cap <= n:  # the live points, appended last, fill the whole store
         np.testing.assert_array_equal(both.store_L[:cap].cpu().numpy(), live[:cap])
+
+
+@pytest.mark.parametrize("runs", [1, 60, 320])  # many, two and one block per run
+def test_phantoms_overwrite_the_shell_they_overlap(gpu_lib, oracle_mod, runs):
+    """Capacity 18 for a shell of 8 and 16 phantoms: the phantoms start at slot 2, over the shell
+    written before them, and the live points follow at slot 6."""
+    from jaxns_gb300 import _ffi
+    from jaxns_gb300.engine import NSBatch
+    n, s, K, cap = 9, 8, 2, 18
+    b = NSBatch([_spec(oracle_mod, n, s, K, cap)] * runs)
+    b.init()
+    old = b.live_view(runs - 1)
+    old = {k: old[k].cpu().numpy().copy() for k in ("log_L_raw", "U")}
+    _ffi.call("gbns_batch_shell", ctypes.byref(b._b), b._stream())
+    pL = b.ph_L[-s * K:].cpu().numpy()
+    pU = b.ph_U[-s * K * 2:].view(-1, 2).cpu().numpy()
+    _ffi.call("gbns_batch_merge", ctypes.byref(b._b), b._stream())
+    new = b.live_view(runs - 1)
+    L, U = b.store_L[-cap:].cpu().numpy(), b.store_U[-2 * cap:].view(-1, 2).cpu().numpy()
+    for got, shell, ph, live in ((L, old["log_L_raw"], pL, new["log_L_raw"]), (U, old["U"], pU, new["U"])):
+        np.testing.assert_array_equal(got[:2], shell[:2])
+        np.testing.assert_array_equal(got[2:6], ph[:4])
+        np.testing.assert_array_equal(got[6:15], live.cpu().numpy())
+        np.testing.assert_array_equal(got[15:], ph[13:])
+    np.testing.assert_array_equal(b.store_P[-cap:].cpu().numpy(), [0] * 2 + [1] * 4 + [0] * 9 + [1] * 3)
