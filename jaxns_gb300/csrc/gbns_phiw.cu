@@ -505,15 +505,22 @@ __global__ void __launch_bounds__(1024) k_adj_reduce(const double *log_w, long l
   const double s2 = exp(2.0 * log_sigma);
   const double c = -0.5 * (double)N * (log(2.0 * 3.141592653589793) + 2.0 * log_sigma);
   AdjSums t = {-INFINITY, 0.0, 0.0, 0.0};
-  int bad = 0;
+  int bad = 0, unbounded = 0;
   for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
     const double a = c - 0.5 * ss[i] / s2 + log_w[i];
     t.mx = fmax(t.mx, a);
     bad |= a != a;
+    unbounded |= !(fabs(ss[i]) < INFINITY && fabs(ry[i]) < INFINITY);
   }
   bad = __syncthreads_or(bad);
+  unbounded = __syncthreads_or(unbounded);
   t.mx = cta_max_d(t.mx, red);
-  if (bad && !(t.mx > -INFINITY)) t.se = t.gt = t.gs = NAN;  // a NaN point makes the sums NaN
+  // a range without a finite a: what its points add to the sums of a set that has one.  A NaN point
+  // makes them NaN, a point of infinite residual (weight 0) the gradient's
+  if (!(t.mx > -INFINITY)) {
+    if (bad) t.se = NAN;
+    if (bad || unbounded) t.gt = t.gs = NAN;
+  }
   if (t.mx > -INFINITY) {
     for (long long i = lo + threadIdx.x; i < hi; i += blockDim.x) {
       const double a = c - 0.5 * ss[i] / s2 + log_w[i];
@@ -539,7 +546,7 @@ __global__ void __launch_bounds__(256) k_adj_total(const AdjSums *part, int bloc
   t.mx = cta_max_d(t.mx, red);
   for (int q = threadIdx.x; q < blocks; q += blockDim.x) {
     const AdjSums p = part[q];
-    if (p.mx > -INFINITY || p.se != p.se) {
+    if (p.mx > -INFINITY || p.se != p.se || p.gt != p.gt) {
       const double f = exp(p.mx - t.mx);
       t.se += f * p.se;
       t.gt += f * p.gt;

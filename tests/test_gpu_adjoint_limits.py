@@ -36,3 +36,13 @@ def test_overflowing_points_have_no_weight(gpu_lib, P, tensor_cores):
     # w = 0 in the other points: y^2 in fp32 chains of 32, N products
     assert abs(out[0] - ref) <= 40 * 2.0 ** -24 * 0.5 * (y @ y) / s2
     assert np.isnan(out[1]) and np.isnan(out[2])
+
+
+@pytest.mark.parametrize("tensor_cores", [True, False])
+def test_a_whole_range_of_overflowing_points(gpu_lib, tensor_cores):
+    """The first 128 points all overflow: one block of the reduction has nothing finite, and the result
+    is the one of the single block that takes all points."""
+    from jaxns_gb300.adjoint import evidence_and_grad
+    ds = _dead_set(512, 3, 300, np.arange(128))
+    out = evidence_and_grad(ds, math.log(1e19), 0.3, tensor_cores=tensor_cores).cpu().numpy()
+    assert np.isfinite(out[0]) and np.isnan(out[1]) and np.isnan(out[2])
