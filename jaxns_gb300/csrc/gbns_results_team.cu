@@ -13,6 +13,8 @@
 // evidence_scan_cta (gbns_device.cuh); a range's A_{k-1} is its base (the c sums before it)
 // plus a, so sum dZ A = base * sum dZ + sum dZ a, and one barrier serves both.  Each thread takes
 // consecutive elements, two passes of exponentials and one block scan per range.
+// log T and log T2 are pairs within a thread and FP64 between threads and blocks, as A and Z are
+// between blocks, so the register is as exact as the one-block scan's.
 // Bound: latency (barriers ~2 us, FP64 logarithms at the ends) up to ~100 k samples per run; beyond
 // that the ~1000 instructions per sample, now on every SM.
 // us, one block per run / set -> team: one run of 936 k samples out of order with its U rows
@@ -32,7 +34,7 @@ constexpr long long TEAM_MIN_RANGE = 512;  // positions per block below which a 
 
 struct TeamTotals {        // one block's sums
   long long edges;         // out-degree - 1 over its positions
-  float4 T;                // log T and log T2, fp32 pairs
+  double2 T;               // log T and log T2
   FS c, dZ, dza, t2, hP, hQ;
 };
 
@@ -49,8 +51,9 @@ struct TeamSmem {
   };
   long long wsum[TEAM_W], carry, lred[32];
   TeamTotals own;          // a team of one block exchanges nothing
-  float4 base_T;
-  FS z_all, z_before, fin[6];
+  double2 warp_T[TEAM_W], base_T;
+  FS z_before;
+  ScaledSum fin[6];
   double lg[4], h[2];
 };
 
@@ -254,6 +257,22 @@ __device__ void team_tree(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, Visit 
   }
 }
 
+// Warp sums of scaled values (every lane gets them).
+__device__ __forceinline__ FS warp_sum_fs(FS v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fs_sum(v, shfl_xor_fs(v, o));
+  return v;
+}
+
+__device__ __forceinline__ ScaledSum warp_sum_ss(ScaledSum v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const ScaledSum u = {__shfl_xor_sync(0xffffffffu, v.q, o), __shfl_xor_sync(0xffffffffu, v.e, o)};
+    v = ss_sum(v, u);
+  }
+  return v;
+}
+
 // Exclusive block prefix of a pair-scaled value per thread, and the block's total.
 __device__ __forceinline__ FS team_scan_fs(FS v, FS *ws, FS &total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -279,21 +298,31 @@ __device__ __forceinline__ FS team_scan_fs(FS v, FS *ws, FS &total) {
 }
 
 // One element of the recurrence (evidence_scan_cta): the coefficients of its live-point count,
-// log X before (x, x2) and after (xc, x2c) it, and its terms as log-space pairs.
+// log X before (x, x2) and after (xc) it, and its terms as log-space pairs.  log X is the base
+// before the thread's first element plus the sum since then, added once per element, so its
+// rounding does not build up along a thread.
 struct TeamElem {
   float cp[10];
+  float bh, bl, b2h, b2l;      // log X, log X2 before the thread's first element
+  float ph, pl, p2h, p2l;      // log T, log T2 summed from there
   float xh, xl, x2h, x2l;      // before; advanced by next()
   float xch, xcl;              // log X after it
   float mh, ml;
+  __device__ __forceinline__ void start(float h, float l, float h2, float l2) {
+    bh = xh = h; bl = xl = l; b2h = x2h = h2; b2l = x2l = l2;
+    ph = pl = p2h = p2l = 0.0f;
+  }
   __device__ __forceinline__ void load(const double *ncoef, int nmax, int n, float L, float Lp, float oh, float ol) {
     ncoef_pairs(ncoef, nmax, n < 0 ? 0 : n, cp);
-    pair_sum2(xh, xl, cp[0], cp[1], xch, xcl);
+    pair_sum2(ph, pl, cp[0], cp[1], ph, pl);
+    pair_sum2(bh, bl, ph, pl, xch, xcl);
     log_mid_pair(L, Lp, oh, ol, mh, ml);
   }
   __device__ __forceinline__ void next() {
     xh = xch;
     xl = xcl;
-    pair_sum2(x2h, x2l, cp[4], cp[5], x2h, x2l);
+    pair_sum2(p2h, p2l, cp[4], cp[5], p2h, p2l);
+    pair_sum2(b2h, b2l, p2h, p2l, x2h, x2l);
   }
   __device__ __forceinline__ FS c() const {
     if (!(mh > -INFINITY)) return fs_zero();
@@ -322,8 +351,8 @@ struct TeamElem {
 
 // compute_evidence_stats (internals/shrinkage_statistics.py:131-157) of the run by its team;
 // every block of the grid calls it.  After it block 0 of the run has in sm: fin[0..3] = Z, Z2,
-// dZ2, A (pair-scaled), lg[0..2] their logs (every block: lg[0] = log Z), base_T the total of the
-// log T, log T2 pairs, h the dZ-weighted means of max(L, 0) and max(-L, 0).  out(k, log X pair,
+// dZ2, A, lg[0..3] their logs (every block: lg[0] = log Z), base_T the totals of
+// log T and log T2, h the dZ-weighted means of max(L, 0) and max(-L, 0).  out(k, log X pair,
 // log dZ pair, Z through k) is called for every sample of the block's range.
 template <bool OUT_LZ, typename Out>
 __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, const int *nl, const double *ncoef,
@@ -336,7 +365,7 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
   TeamTotals *tot = R.Y == 1 ? &sm.own : R.tot;
   float oh, ol;
   pair_of(Loff, oh, ol);
-  float ah = 0.f, al = 0.f, bh = 0.f, bl = 0.f;  // log X, log X2 before this thread's first element
+  float ah = 0.f, al = 0.f, bh = 0.f, bl = 0.f;  // log X, log X2 before this thread's first element (pairs)
   __syncthreads();
   if (work) {
     float sh = 0.f, sl = 0.f, s2h = 0.f, s2l = 0.f;
@@ -352,38 +381,43 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
     cta_scan_p2(ah, al, bh, bl, t, sm.ev.pair);
     pair_sum2(ah, al, -sh, -sl, ah, al);
     pair_sum2(bh, bl, -s2h, -s2l, bh, bl);
-    if (tid == 0) tot[R.y].T = t;
+    // the block's total in FP64 from the threads' sums
+    const double d = warp_sum((double)sh + (double)sl), d2 = warp_sum((double)s2h + (double)s2l);
+    if (lane == 0) sm.warp_T[warp] = make_double2(d, d2);
+    __syncthreads();
+    if (tid < 2) {
+      double v = 0.0;
+      for (int q = 0; q < TEAM_W; ++q) v += tid == 0 ? sm.warp_T[q].x : sm.warp_T[q].y;
+      (tid == 0 ? tot[R.y].T.x : tot[R.y].T.y) = v;
+    }
   }
   grid.sync();
   FS z_thread = fs_zero();
   if (work) {
     if (warp == 0) {
       // the log T sums of the blocks before this one; for block 0, of all blocks (the end)
-      float h = 0.f, l = 0.f, h2 = 0.f, l2 = 0.f;
+      double d = 0.0, d2 = 0.0;
       for (int q = lane; q < (R.y == 0 ? R.Y : R.y); q += 32) {
-        const float4 t = tot[q].T;
-        pair_sum2(h, l, t.x, t.y, h, l);
-        pair_sum2(h2, l2, t.z, t.w, h2, l2);
+        const double2 t = tot[q].T;
+        d += t.x;
+        d2 += t.y;
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float uh = __shfl_xor_sync(0xffffffffu, h, o), ul = __shfl_xor_sync(0xffffffffu, l, o);
-        const float vh = __shfl_xor_sync(0xffffffffu, h2, o), vl = __shfl_xor_sync(0xffffffffu, l2, o);
-        pair_sum2(h, l, uh, ul, h, l);
-        pair_sum2(h2, l2, vh, vl, h2, l2);
-      }
-      if (lane == 0) sm.base_T = make_float4(h, l, h2, l2);
+      d = warp_sum(d);
+      d2 = warp_sum(d2);
+      if (lane == 0) sm.base_T = make_double2(d, d2);
     }
     __syncthreads();
     if (R.y > 0) {
-      const float4 t = sm.base_T;
-      pair_sum2(t.x, t.y, ah, al, ah, al);
-      pair_sum2(t.z, t.w, bh, bl, bh, bl);
+      float h, l;
+      pair_of(sm.base_T.x, h, l);
+      pair_sum2(h, l, ah, al, ah, al);
+      pair_of(sm.base_T.y, h, l);
+      pair_sum2(h, l, bh, bl, bh, bl);
     }
     const float Lp0 = t0 < t1 && t0 > 0 ? team_L(R, t0 - 1) : -INFINITY;
     TeamElem e;
     FS cs = fs_zero(), zs = fs_zero();
-    e.xh = ah; e.xl = al; e.x2h = bh; e.x2l = bl;
+    e.start(ah, al, bh, bl);
     float Lp = Lp0;
     for (long long k = t0; k < t1; ++k) {
       const float L = team_L(R, k);
@@ -403,7 +437,7 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
     FS s[5];  // dZ, dZ a, t2, dZ L+, dZ L-
 #pragma unroll
     for (int q = 0; q < 5; ++q) s[q] = fs_zero();
-    e.xh = ah; e.xl = al; e.x2h = bh; e.x2l = bl;
+    e.start(ah, al, bh, bl);
     Lp = Lp0;
     for (long long k = t0; k < t1; ++k) {
       const float L = team_L(R, k);
@@ -422,9 +456,7 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
       Lp = L;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int q = 0; q < 5; ++q) s[q] = fs_sum(s[q], shfl_xor_fs(s[q], o));
+    for (int q = 0; q < 5; ++q) s[q] = warp_sum_fs(s[q]);
     if (lane == 0)
 #pragma unroll
       for (int q = 0; q < 5; ++q) sm.ev.red[q][warp] = s[q];
@@ -451,18 +483,16 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
   grid.sync();
   if (work) {
     if (warp == 0) {
-      // Z of the whole run, and of the blocks before this one
-      FS all = fs_zero(), bef = fs_zero();
+      // Z of the whole run (FP64), and of the blocks before this one
+      ScaledSum all = ss_zero();
+      FS bef = fs_zero();
       for (int q = lane; q < R.Y; q += 32) {
         const FS z = tot[q].dZ;
-        all = fs_sum(all, z);
+        all = ss_sum(all, ss_from_fs(z));
         if (q < R.y) bef = fs_sum(bef, z);
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        all = fs_sum(all, shfl_xor_fs(all, o));
-        bef = fs_sum(bef, shfl_xor_fs(bef, o));
-      }
+      all = warp_sum_ss(all);
+      bef = warp_sum_fs(bef);
       if (lane == 0) {
         sm.fin[0] = all;
         sm.z_before = bef;
@@ -470,10 +500,12 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
     } else if (warp == 1 && R.y == 0) {
       // A's base of every block: the c sums before it; Z2 = sum 2 (base dZ + dZ a) + t2
       FS carry = fs_zero(), z2 = fs_zero(), t2 = fs_zero(), hP = fs_zero(), hQ = fs_zero();
+      ScaledSum A = ss_zero();
       for (int q0 = 0; q0 < R.Y; q0 += 32) {
         const int q = q0 + lane;
         const bool ok = q < R.Y;
         FS v = ok ? tot[q].c : fs_zero();
+        A = ss_sum(A, ss_from_fs(v));
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const FS u = shfl_up_fs(v, o);
@@ -492,27 +524,25 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
         }
         carry = fs_sum(carry, shfl_fs(v, 31));
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        z2 = fs_sum(z2, shfl_xor_fs(z2, o));
-        t2 = fs_sum(t2, shfl_xor_fs(t2, o));
-        hP = fs_sum(hP, shfl_xor_fs(hP, o));
-        hQ = fs_sum(hQ, shfl_xor_fs(hQ, o));
-      }
+      A = warp_sum_ss(A);
+      z2 = warp_sum_fs(z2);
+      t2 = warp_sum_fs(t2);
+      hP = warp_sum_fs(hP);
+      hQ = warp_sum_fs(hQ);
       if (lane == 0) {
-        sm.fin[1] = z2;
-        sm.fin[2] = t2;
-        sm.fin[3] = carry;
-        sm.fin[4] = hP;
-        sm.fin[5] = hQ;
+        sm.fin[1] = ss_from_fs(z2);
+        sm.fin[2] = ss_from_fs(t2);
+        sm.fin[3] = A;
+        sm.fin[4] = ss_from_fs(hP);
+        sm.fin[5] = ss_from_fs(hQ);
       }
     }
     __syncthreads();
     if (warp == 0) {
       const int nfin = R.y == 0 ? 4 : 1;
-      if (lane < nfin) sm.lg[lane] = ss_log(ss_from_fs(sm.fin[lane]));
+      if (lane < nfin) sm.lg[lane] = ss_log(sm.fin[lane]);
       else if (R.y == 0 && lane >= 8 && lane < 10) {
-        const ScaledSum z = ss_from_fs(sm.fin[0]), h = ss_from_fs(sm.fin[lane - 4]);
+        const ScaledSum z = sm.fin[0], h = sm.fin[lane - 4];
         sm.h[lane - 8] = (z.q > 0.0 && h.q > 0.0) ? (h.q / z.q) * pow2i(h.e - z.e) : 0.0;
       }
     }
@@ -521,7 +551,7 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
   grid.sync();  // the totals are read: their memory may be an output
   if (work) {
     TeamElem e;
-    e.xh = ah; e.xl = al; e.x2h = bh; e.x2l = bl;
+    e.start(ah, al, bh, bl);
     float Lp = t0 < t1 && t0 > 0 ? team_L(R, t0 - 1) : -INFINITY;
     FS z = OUT_LZ ? fs_sum(sm.z_before, z_thread) : fs_zero();
     for (long long k = t0; k < t1; ++k) {
@@ -580,10 +610,10 @@ __global__ void __launch_bounds__(TEAM_T, 1)
                           if (k == N - 1) fin->log_dZ_mean = pair_to_double(h, l);
                         });
   if (R.Y > 0 && R.y == 0 && threadIdx.x == 0) {
-    const double X = (double)sm.base_T.x + (double)sm.base_T.y;
+    const double X = sm.base_T.x;
     fin->log_L = (double)L[N - 1];
     fin->log_X_mean = X;
-    fin->log_X2_mean = (double)sm.base_T.z + (double)sm.base_T.w;
+    fin->log_X2_mean = sm.base_T.y;
     fin->log_Z_mean = sm.lg[0];
     fin->log_Z2_mean = sm.lg[1];
     fin->log_dZ2_mean = sm.lg[2];

@@ -10,34 +10,36 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-def _spec(oracle_mod, n, s, K, cap):
+def _spec(oracle_mod, n, s, K, cap, limit=False):
     from jaxns_gb300.engine import RunSpec, mvn_offset, mvn_params
     D = 2
     mu, cov = corr_gauss(D, 1)
     return RunSpec(D=D, num_live_points=n, shell_size=s, num_slices=K + 1, family=0, params=mvn_params(mu, cov),
                    prior_kind=np.zeros(D, np.int32), prior_a=np.full(D, -10.0), prior_b=np.full(D, 20.0), max_samples=cap,
-                   term_cond={"max_samples": float(cap)}, key=oracle_mod.PRNGKey(5), num_phantom=K,
+                   term_cond={"max_samples": float(cap)} if limit else {"dlogZ": 1e-30}, key=oracle_mod.PRNGKey(5), num_phantom=K,
                    log_L_offset=float(mvn_offset(cov)))
 
 
+@pytest.mark.parametrize("limit", [False, True])  # with the sample limit the run ends before its first shell
 @pytest.mark.parametrize("n,s,K,cap", [(16, 8, 0, 4), (16, 8, 0, 8), (16, 8, 2, 8), (300, 150, 0, 150), (9, 8, 3, 5)])
-def test_appends_stay_in_the_store(gpu_lib, oracle_mod, n, s, K, cap):
+def test_appends_stay_in_the_store(gpu_lib, oracle_mod, n, s, K, cap, limit):
     """A capacity below one shell, its phantoms or the live set: the run's appends end at its own
     last slot, and the next run's store holds what it holds alone."""
     from jaxns_gb300.engine import NSBatch
-    small, big = _spec(oracle_mod, n, s, K, cap), _spec(oracle_mod, 64, 32, 1, 64 * 40)
+    small, big = _spec(oracle_mod, n, s, K, cap, limit), _spec(oracle_mod, 64, 32, 1, 64 * 40)
     alone, both = NSBatch([big]), NSBatch([small, big])
     for b in (alone, both):
         b.init()
         b.iterate(1)
+        b.finalize()
     st = both.state()
-    assert st["done"][0] == 1 and st["done"][1] == 0 and st["num_samples"][1] == 64
+    assert st["iterations"][0] == (0 if limit else 1) and st["iterations"][1] == 1 and st["num_samples"][1] == 128
     for f in ("store_L", "store_S", "store_E", "store_P"):
         np.testing.assert_array_equal(getattr(both, f)[cap:].cpu().numpy(), getattr(alone, f).cpu().numpy(), err_msg=f)
     np.testing.assert_array_equal(both.store_U[2 * cap:].cpu().numpy(), alone.store_U.cpu().numpy())
+    # the live points, appended last, fill the whole store
     live = both.live_view(0)["log_L_raw"].cpu().numpy()
-    if cap <= n:  # the live points, appended last, fill the whole store
-        np.testing.assert_array_equal(both.store_L[:cap].cpu().numpy(), live[:cap])
+    np.testing.assert_array_equal(both.store_L[:cap].cpu().numpy(), live[:cap])
 
 
 @pytest.mark.parametrize("runs", [1, 60, 320])  # many, two and one block per run
