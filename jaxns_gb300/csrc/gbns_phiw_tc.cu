@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM) k_lg_shell_fused(const __grid
 // by TMA, warp 1 issues the 3xTF32 MMAs into two 256-column accumulators in turn, warps 2-5 and
 // 6-9 drain a column half each (thread = point): per 32 rows one fp32 chain for each sum, then FP64
 // registers, added to the point's totals when the point tile changes.  (A sum of squares beyond fp32 is
-// infinite: the point's weight is zero.  fp32 pairs for the chunks made it NaN.)
+// infinite and the point's weight zero; fp32 pairs for the four chunks of a tile, 8 us less, made it NaN.)
 // Bound: the tensor pipe.  256 rows per MMA are what reaches it: 12 MMAs of 128 x 256 x 8 take
 // 1.66 k cycles, of 128 x 128 x 8 2.25 k for half the work (the 128-point operand is read again
 // for every one).  40,000 points x 4096 rows x 32: one tile per CTA (5,008 CTAs, copy, MMAs and
@@ -1118,7 +1118,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(a * MMA_ROWS + half * SR_ROWS);
-      // the next 32 columns load while these are used
+      // the next 32 columns load while these are used; the FP64 additions wait until the
+      // accumulator is released
+      float c1[4], c2[4];
       auto chunk = [&](uint32_t (&r)[32], int ch) {
         // rows past the last data row have y = 0 and a zero product: they add nothing
         float p1 = 0.0f, p2 = 0.0f;
@@ -1133,8 +1135,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
             p2 = fmaf(rr, yv[x], p2);
           }
         }
-        s1 += (double)p1;
-        s2 += (double)p2;
+        c1[ch] = p1;
+        c2[ch] = p2;
       };
       uint32_t ra[32], rb[32];
       tc_ld32_start(taddr, ra);
@@ -1152,6 +1154,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_resid_tc(const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(10 + a));  // accumulator a drained
       chunk(rb, 3);
+      s1 += ((double)c1[0] + (double)c1[1]) + ((double)c1[2] + (double)c1[3]);
+      s2 += ((double)c2[0] + (double)c2[1]) + ((double)c2[2] + (double)c2[3]);
       if (t + 1 == t1 || (t + 1) / row_tiles != p) {
         const long long pnt = p * TC_M + qd * 32 + lane;
         if (pnt < M) {
