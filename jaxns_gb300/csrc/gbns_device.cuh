@@ -612,6 +612,7 @@ __device__ __forceinline__ void cta_scan_fs(FS v, FS &incl, FS &excl, FS &tot, E
 
 struct EvScanPairSmem {
   float4 w[32];
+  float4 own[32];  // each warp's own totals, left for the caller
 };
 
 // Inclusive CTA scan of two fp32 pairs (a = ah + al, b = bh + bl); every thread also gets
@@ -628,10 +629,10 @@ __device__ __forceinline__ void cta_scan_p2(float &ah, float &al, float &bh, flo
       pair_sum2(ubh, ubl, bh, bl, bh, bl);
     }
   }
-  if (lane == 31) sm.w[w] = make_float4(ah, al, bh, bl);
+  if (lane == 31) sm.own[w] = make_float4(ah, al, bh, bl);
   __syncthreads();
   if (w == 0) {
-    float4 x = lane < nw ? sm.w[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x = lane < nw ? sm.own[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float uah = __shfl_up_sync(0xffffffffu, x.x, o), ual = __shfl_up_sync(0xffffffffu, x.y, o);

@@ -19,7 +19,9 @@
 // that the ~1000 instructions per sample, now on every SM.
 // us, one block per run / set -> team: one run of 936 k samples out of order with its U rows
 // 105,500 -> 1,620, one linear-Gaussian run of 26 k samples 1,392 -> 107, 48 runs of 13 k 166 -> 98;
-// evidence of 250 k samples with log Z per sample 2,176 -> 52, their tree count (five launches) 20 -> 17.
+// evidence of 250 k samples with log Z per sample 2,176 -> 54 (52 with the FP64 sums as fp32 pairs), their
+// tree count (five launches) 20 -> 17.
+#include <climits>
 #include <cooperative_groups.h>
 #include "gbns_device.cuh"
 #include "gbns_launch.h"
@@ -51,7 +53,8 @@ struct TeamSmem {
   };
   long long wsum[TEAM_W], carry, lred[32];
   TeamTotals own;          // a team of one block exchanges nothing
-  double2 warp_T[TEAM_W], base_T;
+  double2 base_T;
+  float4 base_pairs;       // the same as fp32 pairs
   FS z_before;
   ScaledSum fin[6];
   double lg[4], h[2];
@@ -264,13 +267,23 @@ __device__ __forceinline__ FS warp_sum_fs(FS v) {
   return v;
 }
 
-__device__ __forceinline__ ScaledSum warp_sum_ss(ScaledSum v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const ScaledSum u = {__shfl_xor_sync(0xffffffffu, v.q, o), __shfl_xor_sync(0xffffffffu, v.e, o)};
-    v = ss_sum(v, u);
+// The sum of one of the blocks' totals in FP64, by a warp: at the largest exponent, so that the
+// additions are plain ones (a scaled addition per block and level costs three times the latency).
+__device__ __forceinline__ ScaledSum warp_fold(const TeamTotals *tot, int Y, FS TeamTotals::*which) {
+  const int lane = threadIdx.x & 31;
+  int e = INT_MIN;
+  for (int q = lane; q < Y; q += 32) {
+    const FS v = tot[q].*which;
+    if (v.h > 0.0f) e = max(e, v.e);
   }
-  return v;
+  e = __reduce_max_sync(0xffffffffu, e);
+  if (e == INT_MIN) return ss_zero();
+  double sum = 0.0;
+  for (int q = lane; q < Y; q += 32) {
+    const FS v = tot[q].*which;
+    if (v.h > 0.0f) sum = fma((double)v.h + (double)v.l, pow2i(v.e - e), sum);
+  }
+  return {warp_sum(sum), e};
 }
 
 // Exclusive block prefix of a pair-scaled value per thread, and the block's total.
@@ -377,18 +390,17 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
       pair_sum2(s2h, s2l, cp[4], cp[5], s2h, s2l);
     }
     ah = sh; al = sl; bh = s2h; bl = s2l;
-    float4 t;
+    float4 t;  // (the total as a pair is not used)
     cta_scan_p2(ah, al, bh, bl, t, sm.ev.pair);
     pair_sum2(ah, al, -sh, -sl, ah, al);
     pair_sum2(bh, bl, -s2h, -s2l, bh, bl);
-    // the block's total in FP64 from the threads' sums
-    const double d = warp_sum((double)sh + (double)sl), d2 = warp_sum((double)s2h + (double)s2l);
-    if (lane == 0) sm.warp_T[warp] = make_double2(d, d2);
-    __syncthreads();
-    if (tid < 2) {
-      double v = 0.0;
-      for (int q = 0; q < TEAM_W; ++q) v += tid == 0 ? sm.warp_T[q].x : sm.warp_T[q].y;
-      (tid == 0 ? tot[R.y].T.x : tot[R.y].T.y) = v;
+    if (warp == 0) {
+      // the block's total in FP64 from the warps' sums: log T in even lanes, log T2 in odd ones
+      const float2 *w = reinterpret_cast<const float2 *>(sm.ev.pair.own);
+      double v = lane < 2 * TEAM_W ? (double)w[lane].x + (double)w[lane].y : 0.0;
+#pragma unroll
+      for (int o = TEAM_W; o > 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < 2) (&tot[R.y].T.x)[lane] = v;
     }
   }
   grid.sync();
@@ -404,15 +416,19 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
       }
       d = warp_sum(d);
       d2 = warp_sum(d2);
-      if (lane == 0) sm.base_T = make_double2(d, d2);
+      if (lane == 0) {
+        float4 t;
+        pair_of(d, t.x, t.y);
+        pair_of(d2, t.z, t.w);
+        sm.base_T = make_double2(d, d2);
+        sm.base_pairs = t;
+      }
     }
     __syncthreads();
     if (R.y > 0) {
-      float h, l;
-      pair_of(sm.base_T.x, h, l);
-      pair_sum2(h, l, ah, al, ah, al);
-      pair_of(sm.base_T.y, h, l);
-      pair_sum2(h, l, bh, bl, bh, bl);
+      const float4 t = sm.base_pairs;
+      pair_sum2(t.x, t.y, ah, al, ah, al);
+      pair_sum2(t.z, t.w, bh, bl, bh, bl);
     }
     const float Lp0 = t0 < t1 && t0 > 0 ? team_L(R, t0 - 1) : -INFINITY;
     TeamElem e;
@@ -483,29 +499,22 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
   grid.sync();
   if (work) {
     if (warp == 0) {
-      // Z of the whole run (FP64), and of the blocks before this one
-      ScaledSum all = ss_zero();
-      FS bef = fs_zero();
-      for (int q = lane; q < R.Y; q += 32) {
-        const FS z = tot[q].dZ;
-        all = ss_sum(all, ss_from_fs(z));
-        if (q < R.y) bef = fs_sum(bef, z);
-      }
-      all = warp_sum_ss(all);
-      bef = warp_sum_fs(bef);
-      if (lane == 0) {
-        sm.fin[0] = all;
-        sm.z_before = bef;
+      // Z of the whole run, and of the blocks before this one
+      const ScaledSum all = warp_fold(tot, R.Y, &TeamTotals::dZ);
+      if (lane == 0) sm.fin[0] = all;
+      if (OUT_LZ) {
+        FS bef = fs_zero();
+        for (int q = lane; q < R.y; q += 32) bef = fs_sum(bef, tot[q].dZ);
+        bef = warp_sum_fs(bef);
+        if (lane == 0) sm.z_before = bef;
       }
     } else if (warp == 1 && R.y == 0) {
       // A's base of every block: the c sums before it; Z2 = sum 2 (base dZ + dZ a) + t2
       FS carry = fs_zero(), z2 = fs_zero(), t2 = fs_zero(), hP = fs_zero(), hQ = fs_zero();
-      ScaledSum A = ss_zero();
       for (int q0 = 0; q0 < R.Y; q0 += 32) {
         const int q = q0 + lane;
         const bool ok = q < R.Y;
         FS v = ok ? tot[q].c : fs_zero();
-        A = ss_sum(A, ss_from_fs(v));
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const FS u = shfl_up_fs(v, o);
@@ -524,7 +533,6 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
         }
         carry = fs_sum(carry, shfl_fs(v, 31));
       }
-      A = warp_sum_ss(A);
       z2 = warp_sum_fs(z2);
       t2 = warp_sum_fs(t2);
       hP = warp_sum_fs(hP);
@@ -532,10 +540,12 @@ __device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, co
       if (lane == 0) {
         sm.fin[1] = ss_from_fs(z2);
         sm.fin[2] = ss_from_fs(t2);
-        sm.fin[3] = A;
         sm.fin[4] = ss_from_fs(hP);
         sm.fin[5] = ss_from_fs(hQ);
       }
+    } else if (warp == 2 && R.y == 0) {
+      const ScaledSum A = warp_fold(tot, R.Y, &TeamTotals::c);
+      if (lane == 0) sm.fin[3] = A;
     }
     __syncthreads();
     if (warp == 0) {

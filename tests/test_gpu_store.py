@@ -33,13 +33,14 @@ def test_appends_stay_in_the_store(gpu_lib, oracle_mod, n, s, K, cap, limit):
         b.iterate(1)
         b.finalize()
     st = both.state()
-    assert st["iterations"][0] == (0 if limit else 1) and st["iterations"][1] == 1 and st["num_samples"][1] == 128
+    assert st["iterations"][0] == (0 if limit else 1) and st["iterations"][1] == 1
+    assert st["num_samples"][1] == alone.state()["num_samples"][0]
     for f in ("store_L", "store_S", "store_E", "store_P"):
         np.testing.assert_array_equal(getattr(both, f)[cap:].cpu().numpy(), getattr(alone, f).cpu().numpy(), err_msg=f)
     np.testing.assert_array_equal(both.store_U[2 * cap:].cpu().numpy(), alone.store_U.cpu().numpy())
-    # the live points, appended last, fill the whole store
-    live = both.live_view(0)["log_L_raw"].cpu().numpy()
-    np.testing.assert_array_equal(both.store_L[:cap].cpu().numpy(), live[:cap])
+    if st["done"][0]:  # (a store of exactly one shell goes on) the live points, appended last, fill the whole store
+        live = both.live_view(0)["log_L_raw"].cpu().numpy()
+        np.testing.assert_array_equal(both.store_L[:cap].cpu().numpy(), live[:cap])
 
 
 @pytest.mark.parametrize("runs", [1, 60, 320])  # many, two and one block per run

@@ -13,8 +13,9 @@ pytestmark = pytest.mark.gpu
 def test_register_log_X_is_fp64(gpu_lib, live):
     """One sample per thread of every block, all with the same live-point count: the exact sum of the
     table's entries (fp32 pairs, exact in FP64) against the register.  Roundings of 2^-53 of the sum at
-    most: five levels of a warp, sixteen warps in turn (each the size of its partial sum: 8.5 in all),
-    five blocks per lane (3), five levels.  As fp32 pairs these counts are off by up to 42 2^-53."""
+    most: five levels of a warp, four levels or sixteen in turn over the warps (8.5 at most, each the size
+    of its partial sum), five blocks per lane (3), five levels.  As fp32 pairs these counts are off by up to
+    42 2^-53."""
     from jaxns_gb300 import _ffi
     from jaxns_gb300.engine import ncoef_table
     N = 512 * torch.cuda.get_device_properties(0).multi_processor_count - 1
