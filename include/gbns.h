@@ -142,7 +142,7 @@ typedef struct {
     int termination_reason;
     int parity;                 /* which live buffer is current */
     int status;                 /* gbns_status bits */
-    int pad1;
+    int pad1;                   /* work word of the merge; any value between calls */
 } gbns_run_state;
 
 /* Log-likelihoods are held on the device in fp32 relative to the run's FP64 log_L_offset

@@ -118,7 +118,7 @@ int gbns_batch_iterate(const gbns_batch *batch, int num_iterations, void *stream
   if (num_iterations < 0) return fail(-1, "gbns_batch_iterate: negative iteration count%s");
   for (int it = 0; it < num_iterations; ++it) {
     if ((e = check(gbns::launch_slice_shells(*batch, nullptr, nullptr, (cudaStream_t)stream), "slice shell"))) return e;
-    if ((e = check(gbns::launch_merge(*batch, (cudaStream_t)stream), "merge"))) return e;
+    if ((e = check(gbns::launch_merge(*batch, it == 0, (cudaStream_t)stream), "merge"))) return e;
   }
   return 0;
 }
@@ -132,7 +132,7 @@ int gbns_batch_shell(const gbns_batch *batch, void *stream) {
 int gbns_batch_merge(const gbns_batch *batch, void *stream) {
   int e = check_batch(batch);
   if (e) return e;
-  return check(gbns::launch_merge(*batch, (cudaStream_t)stream), "gbns_batch_merge");
+  return check(gbns::launch_merge(*batch, true, (cudaStream_t)stream), "gbns_batch_merge");
 }
 
 int gbns_record_event(void *event, void *stream) {

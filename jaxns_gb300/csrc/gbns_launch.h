@@ -28,7 +28,8 @@ cudaError_t launch_slice_spec_mvn(const gbns_batch &b, int dmax, int ib, int ie,
 // lg / fp32: whether the batch has linear-Gaussian runs / runs of the other families
 cudaError_t launch_init(const gbns_batch &b, long long total_points, bool lg, bool fp32, cudaStream_t stream);
 cudaError_t launch_init_lg(const gbns_batch &b, long long total_points, cudaStream_t stream);
-cudaError_t launch_merge(const gbns_batch &b, cudaStream_t stream);
+// first: whether the caller has not launched a merge of this batch before in the same call
+cudaError_t launch_merge(const gbns_batch &b, bool first, cudaStream_t stream);
 cudaError_t launch_finalize(const gbns_batch &b, cudaStream_t stream);
 cudaError_t launch_forward(const gbns_batch &b, int run, const float *U, float *logL, long long B, cudaStream_t stream);
 cudaError_t launch_results(const gbns_batch &b, const gbns_results_bufs &res, cudaStream_t stream);

@@ -276,7 +276,7 @@ __global__ void k_init_finish(gbns_batch b) {
     st.num_likelihood_evaluations = 0;
     st.num_samples = 0;
     st.next_sample_idx = 0;
-    st.pad1 = 0;  // the merge's arrival counter
+    st.pad1 = 0;
     st.iterations = 0;
     st.plateau = 0;
     st.parity = 0;
@@ -730,7 +730,8 @@ __global__ void __launch_bounds__(512, 1) k_merge(gbns_batch b) {
   }
   // ---- the last of the run's blocks commits
   __syncthreads();
-  if (tid == 0) {
+  if (tid == 0 && Y == 1) sm.last = 1;
+  if (tid == 0 && Y > 1) {
     __threadfence();
     const int add = 1 + (y == 0 && sm.done ? 1 << 16 : 0);
     const int all = atomicAdd(&st.pad1, add) + add;
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(512, 1) k_merge(gbns_batch b) {
     __syncthreads();
   }
   if (tid == 0) {
-    st.pad1 = 0;
+    if (Y > 1) st.pad1 = 0;
     st.parity = npar;
     st.next_sample_idx = sm.done ? (nsi2 + n) % cap : nsi2;
     if (sm.done) {
@@ -795,7 +796,7 @@ cudaError_t launch_init(const gbns_batch &b, long long total_points, bool lg, bo
   return cudaGetLastError();
 }
 
-cudaError_t launch_merge(const gbns_batch &b, cudaStream_t stream) {
+cudaError_t launch_merge(const gbns_batch &b, bool first, cudaStream_t stream) {
   int NP = 1;
   while (NP < max_n(b)) NP <<= 1;
   const size_t smem = NP * sizeof(unsigned long long) + 3 * (size_t)max_n(b) * sizeof(float);
@@ -817,6 +818,11 @@ cudaError_t launch_merge(const gbns_batch &b, cudaStream_t stream) {
     threads = max_n(b) <= 512 ? 256 : 512;
     blocks = sms / runs < 1 ? 1 : (sms / runs > 16 ? 16 : sms / runs);
   }
+  // A run's blocks count themselves in its state's pad1, whatever a caller left there: zeroed before
+  // the first merge of a call, and by every merge after itself.
+  if (blocks > 1 && first &&
+      (e = cudaMemset2DAsync(&b.state->pad1, sizeof(gbns_run_state), 0, sizeof(int), (size_t)runs, stream)) != cudaSuccess)
+    return e;
   k_merge<<<dim3((unsigned)runs, (unsigned)blocks), threads, smem, stream>>>(b);
   return cudaGetLastError();
 }

@@ -1487,7 +1487,7 @@ int gbns_lg_iterate(const gbns_batch *batch, const gbns_lg_bufs *lg, int num_ite
   if (num_iterations < 0) return tc_fail(-1, "gbns_lg_iterate: negative iteration count");
   for (int k = 0; k < num_iterations; ++k) {
     cudaError_t e = gbns::launch_lg_shell_fused(*batch, *lg, (cudaStream_t)stream);
-    if (e == cudaSuccess) e = gbns::launch_merge(*batch, (cudaStream_t)stream);
+    if (e == cudaSuccess) e = gbns::launch_merge(*batch, k == 0, (cudaStream_t)stream);
     if (e != cudaSuccess) return tc_fail(-2, cudaGetErrorString(e));
   }
   return 0;
