@@ -804,8 +804,10 @@ cudaError_t launch_merge(const gbns_batch &b, bool first, cudaStream_t stream) {
   cudaError_t e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if (smem > 32 * 1024 &&
-      (e = cudaFuncSetAttribute(k_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+  // the limit is the process's: every caller sets what the largest live set (4096 points) takes, so
+  // that no thread lowers it between another's call here and its launch
+  if (smem > 32 * 1024 && (e = cudaFuncSetAttribute(k_merge, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    4096 * 8 + 3 * 4096 * 4)) != cudaSuccess)
     return e;
   // Up to two runs per SM: wide blocks, and as many of them per run as give every SM one (16 at
   // most); beyond, 128-thread blocks that share the SMs.  us per merge, one 128-thread block per

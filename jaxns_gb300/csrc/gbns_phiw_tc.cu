@@ -1351,9 +1351,12 @@ static cudaError_t lf_config(const gbns_lg_bufs &lg, cudaStream_t s, cudaLaunchC
                 (size_t)cs * (cpc / 4) * cpc * 8 + (size_t)(LF_M_TILE + 1) * 4;
   const size_t per_sm = 233472, floor_bytes = per_sm / (size_t)(512 / R + 1) + 1;
   if (smem < floor_bytes) smem = floor_bytes;
-  if (smem > 232448) return cudaErrorInvalidValue;
+  // (one limit for every size, below the SM's by the static variables: the limit is the process's, and
+  // no caller may lower it between another's call here and its launch)
+  constexpr int max_smem = 232448 - 1024;
+  if (smem > (size_t)max_smem) return cudaErrorInvalidValue;
   const auto k = lf_kernel(cpc);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
   if (e == cudaSuccess && cs > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return e;
   cfg = cudaLaunchConfig_t{};

@@ -799,32 +799,29 @@ cudaError_t launch_prior_transform(const gbns_prior_table &t, const float *U32, 
     const long long tiles = (M + rows - 1) / rows, want = (tiles + PT_WARPS - 1) / PT_WARPS;
     const unsigned grid = (unsigned)(want < (long long)sms * 4 ? want : (long long)sms * 4);
     const size_t smem = t.A && t.D <= 64 ? (size_t)t.D * t.D * sizeof(double) : 0;
+    static_assert(64 * 64 * sizeof(double) + PT_WARPS * sizeof(PtWarp) <= 48 * 1024, "no larger limit to ask for");
     if (U32) {
-      if (smem > 16 * 1024 && (e = cudaFuncSetAttribute(k_prior_tiles<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        (int)smem)) != cudaSuccess)
-        return e;
       k_prior_tiles<float><<<grid, 32 * PT_WARPS, smem, stream>>>(t, U32, M, log_L, X, out);
     } else {
-      if (smem > 16 * 1024 && (e = cudaFuncSetAttribute(k_prior_tiles<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        (int)smem)) != cudaSuccess)
-        return e;
       k_prior_tiles<double><<<grid, 32 * PT_WARPS, smem, stream>>>(t, U64, M, log_L, X, out);
     }
     return cudaGetLastError();
   }
   const size_t smem = t.A ? (size_t)8 * t.D * sizeof(double) : 0;
+  // (the limit is the process's: every caller sets that of the largest D, so that none lowers it)
+  const int max_smem = 8 * 3600 * (int)sizeof(double);
   const long long want = (M + 7) / 8;
   const unsigned grid = (unsigned)(want < (long long)sms * 8 ? want : (long long)sms * 8);
   if (U32) {
     if (smem > 48 * 1024 &&
         (e = cudaFuncSetAttribute(k_prior_transform<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
+                                  max_smem)) != cudaSuccess)
       return e;
     k_prior_transform<float><<<grid, 256, smem, stream>>>(t, U32, M, log_L, X, out);
   } else {
     if (smem > 48 * 1024 &&
         (e = cudaFuncSetAttribute(k_prior_transform<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
+                                  max_smem)) != cudaSuccess)
       return e;
     k_prior_transform<double><<<grid, 256, smem, stream>>>(t, U64, M, log_L, X, out);
   }
