@@ -38,12 +38,12 @@ cudaError_t launch_count_crossed_edges(const int *sender, const float *L, long l
 cudaError_t launch_evidence_stats(const float *L, const int *num_live, long long N, const double *ncoef, int nmax,
                                   gbns_evcalc *final_out, double *lX, double *ldZ, double *lZ, cudaStream_t stream);
 // One block per SM on few runs or one long sample set (gbns_results_team.cu); taken tells whether
-// the batch is small enough.
+// the batch is small enough and the stream has the whole device.
 cudaError_t launch_team_results(const gbns_batch &b, const gbns_results_bufs &res, cudaStream_t stream, bool &taken);
 cudaError_t launch_team_count_edges(const int *sender, const float *L, long long N, int *samples_indices, int *num_live,
-                                    long long *scratch_ll, int *scratch_i, cudaStream_t stream);
+                                    long long *scratch_ll, int *scratch_i, cudaStream_t stream, bool &taken);
 cudaError_t launch_team_evidence(const float *L, const int *num_live, long long N, const double *ncoef, int nmax,
-                                 gbns_evcalc *fin, double *lX, double *ldZ, double *lZ, cudaStream_t stream);
+                                 gbns_evcalc *fin, double *lX, double *ldZ, double *lZ, cudaStream_t stream, bool &taken);
 cudaError_t launch_lg_resid_cc(const gbns_batch &b, const gbns_lg_bufs &lg, cudaStream_t stream);
 cudaError_t launch_lg_step_kernel(const gbns_batch &b, const gbns_lg_bufs &lg, cudaStream_t stream);
 cudaError_t launch_lg_chain_step(const gbns_batch &b, const gbns_lg_bufs &lg, cudaStream_t stream);

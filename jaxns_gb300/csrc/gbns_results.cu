@@ -902,8 +902,11 @@ constexpr long long TEAM_MIN_SAMPLES = 3000;
 
 cudaError_t launch_count_crossed_edges(const int *sender, const float *L, long long N, int *samples_indices,
                                        int *num_live, long long *scratch_ll, int *scratch_i, cudaStream_t stream) {
-  if (N >= TEAM_MIN_SAMPLES)
-    return launch_team_count_edges(sender, L, N, samples_indices, num_live, scratch_ll, scratch_i, stream);
+  if (N >= TEAM_MIN_SAMPLES) {
+    bool taken = false;
+    const cudaError_t e = launch_team_count_edges(sender, L, N, samples_indices, num_live, scratch_ll, scratch_i, stream, taken);
+    if (taken || e != cudaSuccess) return e;
+  }
   k_count_edges<<<1, 1024, 0, stream>>>(sender, L, N, samples_indices, num_live, (unsigned long long *)scratch_ll,
                                         scratch_i);
   return cudaGetLastError();
@@ -911,8 +914,11 @@ cudaError_t launch_count_crossed_edges(const int *sender, const float *L, long l
 
 cudaError_t launch_evidence_stats(const float *L, const int *num_live, long long N, const double *ncoef, int nmax,
                                   gbns_evcalc *final_out, double *lX, double *ldZ, double *lZ, cudaStream_t stream) {
-  if (N >= TEAM_MIN_SAMPLES && (lX || ldZ || lZ))
-    return launch_team_evidence(L, num_live, N, ncoef, nmax, final_out, lX, ldZ, lZ, stream);
+  if (N >= TEAM_MIN_SAMPLES && (lX || ldZ || lZ)) {
+    bool taken = false;
+    const cudaError_t e = launch_team_evidence(L, num_live, N, ncoef, nmax, final_out, lX, ldZ, lZ, stream, taken);
+    if (taken || e != cudaSuccess) return e;
+  }
   if (lZ) k_evidence_stats<true><<<1, RESULTS_EV_THREADS, 0, stream>>>(L, num_live, N, ncoef, nmax, final_out, lX, ldZ, lZ);
   else k_evidence_stats<false><<<1, RESULTS_EV_THREADS, 0, stream>>>(L, num_live, N, ncoef, nmax, final_out, lX, ldZ, lZ);
   return cudaGetLastError();

@@ -22,6 +22,7 @@
 // evidence of 250 k samples with log Z per sample 2,176 -> 54 (52 with the FP64 sums as fp32 pairs), their
 // tree count (five launches) 20 -> 17.
 #include <climits>
+#include <cuda.h>
 #include <cooperative_groups.h>
 #include "gbns_device.cuh"
 #include "gbns_launch.h"
@@ -755,8 +756,33 @@ __global__ void __launch_bounds__(TEAM_T, 1) k_team_results(gbns_batch b, gbns_r
 
 // ------------------------------------------------------------------ launch ----
 
-static cudaError_t team_launch(const void *kernel, int blocks, void **args, cudaStream_t stream) {
-  return cudaLaunchCooperativeKernel(kernel, dim3((unsigned)blocks), dim3(TEAM_T), args, 0, stream);
+// Whether the stream has the whole device.  One of a green context owns some of its SMs only, and a
+// grid of one block per SM of the device, whose blocks wait for one another, has no place there: it
+// gets the kernels of one block per run (gbns_results.cu).
+static bool whole_device(cudaStream_t stream) {
+  using GetCtx = CUresult (*)(CUstream, CUcontext *, CUgreenCtx *);  // cuStreamGetCtx since CUDA 12.5
+  static const GetCtx get = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    const bool ok = cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &p, 12050, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? (GetCtx)p : nullptr;
+  }();
+  CUcontext ctx = nullptr;
+  CUgreenCtx green = nullptr;
+  return !get || get((CUstream)stream, &ctx, &green) != CUDA_SUCCESS || !green;
+}
+
+// taken: whether the launch was made; not on a part of the device, nor where the driver finds the grid
+// too large for what the process may use of it.
+static cudaError_t team_launch(const void *kernel, int blocks, void **args, cudaStream_t stream, bool &taken) {
+  taken = whole_device(stream);
+  if (!taken) return cudaSuccess;
+  const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3((unsigned)blocks), dim3(TEAM_T), args, 0, stream);
+  if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+  cudaGetLastError();
+  taken = false;
+  return cudaSuccess;
 }
 
 static cudaError_t sm_count(int &sms) {
@@ -773,32 +799,34 @@ cudaError_t launch_team_results(const gbns_batch &b, const gbns_results_bufs &re
   if (e != cudaSuccess) return e;
   int per_run = sms / b.num_runs;
   if (per_run < 2) return cudaSuccess;
-  taken = true;
   gbns_batch bb = b;
   gbns_results_bufs rr = res;
   void *args[] = {&bb, &rr, &per_run};
-  return team_launch((const void *)k_team_results, per_run * b.num_runs, args, stream);
+  return team_launch((const void *)k_team_results, per_run * b.num_runs, args, stream, taken);
 }
 
 cudaError_t launch_team_count_edges(const int *sender, const float *L, long long N, int *samples_indices, int *num_live,
-                                    long long *scratch_ll, int *scratch_i, cudaStream_t stream) {
+                                    long long *scratch_ll, int *scratch_i, cudaStream_t stream, bool &taken) {
+  taken = false;
   int sms = 0;
   cudaError_t e = sm_count(sms);
   if (e != cudaSuccess) return e;
   unsigned long long *a = (unsigned long long *)scratch_ll;
   void *args[] = {&sender, &L, &N, &samples_indices, &num_live, &a, &scratch_i};
-  return team_launch((const void *)k_team_count_edges, sms, args, stream);
+  return team_launch((const void *)k_team_count_edges, sms, args, stream, taken);
 }
 
 cudaError_t launch_team_evidence(const float *L, const int *num_live, long long N, const double *ncoef, int nmax,
-                                 gbns_evcalc *fin, double *lX, double *ldZ, double *lZ, cudaStream_t stream) {
+                                 gbns_evcalc *fin, double *lX, double *ldZ, double *lZ, cudaStream_t stream, bool &taken) {
+  taken = false;
   int sms = 0;
   cudaError_t e = sm_count(sms);
   if (e != cudaSuccess) return e;
   // the block sums live in an output until its values are written
   TeamTotals *tot = team_totals(lZ ? lZ : (ldZ ? ldZ : lX));
   void *args[] = {&L, &num_live, &N, &ncoef, &nmax, &fin, &lX, &ldZ, &lZ, &tot};
-  return team_launch(lZ ? (const void *)k_team_evidence<true> : (const void *)k_team_evidence<false>, sms, args, stream);
+  return team_launch(lZ ? (const void *)k_team_evidence<true> : (const void *)k_team_evidence<false>, sms, args, stream,
+                     taken);
 }
 
 }  // namespace gbns
