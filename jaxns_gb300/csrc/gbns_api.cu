@@ -90,25 +90,22 @@ int gbns_forward(const gbns_batch *batch, int run, const float *U_dev, float *lo
 int gbns_batch_init(const gbns_batch *batch, void *stream) {
   int e = check_batch(batch);
   if (e) return e;
-  // total live points = live_off + n of the last run (runs are packed in order)
+  // total live points = live_off + n of the last run (runs are packed in order), and which of the two
+  // initialisations the batch needs: a caller of this ABI can have runs of both kinds in one batch
+  std::unique_ptr<int[]> fam(new (std::nothrow) int[batch->num_runs]);
+  if (!fam) return fail(-1, "gbns_batch_init: out of host memory%s");
   gbns_run_desc last;
   cudaError_t ce = cudaMemcpyAsync(&last, batch->runs + (batch->num_runs - 1), sizeof(last), cudaMemcpyDeviceToHost,
                                    (cudaStream_t)stream);
+  fam[batch->num_runs - 1] = -1;
+  if (ce == cudaSuccess && batch->num_runs > 1)
+    ce = cudaMemcpy2DAsync(fam.get(), sizeof(int), &batch->runs->family, sizeof(gbns_run_desc), sizeof(int),
+                           (size_t)batch->num_runs - 1, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize((cudaStream_t)stream);
   if ((e = check(ce, "gbns_batch_init: reading the run table"))) return e;
-  // which of the two initialisations the batch needs
-  bool lg = last.family == GBNS_LIK_LINGAUSS, fp32 = !lg;
-  for (int k = 0; k < 8; ++k) fp32 = fp32 || batch->bucket_end[k] > batch->bucket_begin[k];
-  if (fp32 && !lg && batch->num_runs > 1) {
-    // (one strided copy: runs of both kinds in one batch are possible for a caller of this ABI)
-    std::unique_ptr<int[]> fam(new (std::nothrow) int[batch->num_runs]);
-    if (!fam) return fail(-1, "gbns_batch_init: out of host memory%s");
-    ce = cudaMemcpy2DAsync(fam.get(), sizeof(int), &batch->runs->family, sizeof(gbns_run_desc), sizeof(int),
-                           (size_t)batch->num_runs, cudaMemcpyDeviceToHost, (cudaStream_t)stream);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize((cudaStream_t)stream);
-    if ((e = check(ce, "gbns_batch_init: reading the run table"))) return e;
-    for (int r = 0; r < batch->num_runs; ++r) lg = lg || fam[r] == GBNS_LIK_LINGAUSS;
-  }
+  fam[batch->num_runs - 1] = last.family;
+  bool lg = false, fp32 = false;
+  for (int r = 0; r < batch->num_runs; ++r) (fam[r] == GBNS_LIK_LINGAUSS ? lg : fp32) = true;
   return check(gbns::launch_init(*batch, last.live_off + last.n, lg, fp32, (cudaStream_t)stream), "gbns_batch_init");
 }
 
