@@ -88,7 +88,7 @@ __device__ float lgp_sum(LgpSmem &sm, float *phi, const float *__restrict__ Phi,
     }
     __syncthreads();  // this pass's residuals are written, the pass before is added
   }
-  if (!compute) add_pass(passes - 1);
+  if (!compute && passes > 0) add_pass(passes - 1);  // (no data rows: the sum is 0)
   return ss;
 }
 

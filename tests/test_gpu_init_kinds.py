@@ -51,3 +51,23 @@ def test_every_run_gets_its_points(gpu_lib, oracle_mod, lg_run, items):
         got = b.live_L[0][r * n:(r + 1) * n].cpu().numpy()
         want = (alone.live_L[0] if r == lg_run else ref.live_L[0][r * n:(r + 1) * n]).cpu().numpy()
         np.testing.assert_array_equal(got, want)
+
+
+def test_no_data_rows(gpu_lib, oracle_mod):
+    """A linear-Gaussian run without data rows, which the C ABI does not refuse: log L is 0 at every
+    point."""
+    from jaxns_gb300 import _ffi
+    from jaxns_gb300.engine import NSBatch, RunSpec
+    D, n = 3, 16
+    spec = RunSpec(D=D, num_live_points=n, shell_size=n // 2, num_slices=2, family=2,
+                   params=np.full(D + 2, 0.5, np.float32), N=1, prior_kind=np.zeros(D, np.int32), prior_a=np.full(D, -1.0),
+                   prior_b=np.full(D, 2.0), max_samples=4 * n, term_cond={"dlogZ": 1e-3}, key=oracle_mod.PRNGKey(7),
+                   store_U=False, log_L_offset=0.0)
+    b = NSBatch([spec], lg_fused=False)
+    b.init()
+    b._descs_host[0].N = 0
+    b.t_runs.copy_(torch.frombuffer(bytearray(bytes(b._descs_host)), dtype=torch.uint8))
+    U = torch.rand(20, D, dtype=torch.float64, device="cuda")
+    np.testing.assert_array_equal(b.forward(0, U).cpu().numpy(), 0.0)
+    _ffi.call("gbns_batch_init", ctypes.byref(b._b), b._stream())
+    np.testing.assert_array_equal(b.live_L[0].cpu().numpy(), 0.0)
