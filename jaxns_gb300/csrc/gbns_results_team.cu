@@ -34,6 +34,11 @@ namespace cg = cooperative_groups;
 constexpr int TEAM_T = 512;
 constexpr int TEAM_W = TEAM_T / 32;
 constexpr long long TEAM_MIN_RANGE = 512;  // positions per block below which a team gets fewer blocks
+// Samples of every run of a batch below which a run gets one block and the launch no barriers between
+// blocks.  us per results pass (two launches of one block per run / a team with barriers / alone): one run
+// of 60 samples 37 / 39 / 34, of 300 37 / 40 / 35, of 1000 41 / 47 / 42, of 1800 45 / 49 / 50; 76 runs of
+// 300 37 / 47 / 37, of 1000 41 / 54 / 43.
+constexpr long long TEAM_SOLO = 1600;
 
 struct TeamTotals {        // one block's sums
   long long edges;         // out-degree - 1 over its positions
@@ -59,6 +64,16 @@ struct TeamSmem {
   FS z_before;
   ScaledSum fin[6];
   double lg[4], h[2];
+};
+
+// The barrier between a launch's blocks; of blocks that work alone, each with a whole run, the
+// block's own.
+struct TeamSync {
+  bool solo;
+  __device__ __forceinline__ void sync() const {
+    if (solo) __syncthreads();
+    else cg::this_grid().sync();
+  }
 };
 
 // This block's part of one run (or sample set).
@@ -101,7 +116,7 @@ __device__ __forceinline__ void team_split(TeamRun &R, int y, int Y) {
 }
 
 // Stable LSD radix sort (4 x 8-bit digits of the keys' upper 32 bits) by the team; result in R.a.
-__device__ void team_radix(cg::grid_group &grid, TeamRun &R, bool work, TeamSmem &sm) {
+__device__ void team_radix(const TeamSync &grid, TeamRun &R, bool work, TeamSmem &sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int *counts = R.si;  // [256][Y] digit counts of the blocks; the indices are written after the sort
   for (int d = 0; d < 4; ++d) {
@@ -177,14 +192,14 @@ __device__ void team_radix(cg::grid_group &grid, TeamRun &R, bool work, TeamSmem
 // count_crossed_edges (internals/tree_structure.py:33-108) by the team; every block of the grid
 // calls it.  visit(pos, k) is called once per sorted position pos with its sample index k.
 template <typename Visit>
-__device__ void team_tree(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, Visit visit) {
+__device__ void team_tree(const TeamSync &grid, TeamRun &R, TeamSmem &sm, Visit visit) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool work = R.Y > 0;
   const long long N = R.N;
   if (work)
     for (long long i = R.lo + tid; i < R.hi; i += TEAM_T) R.deg[i] = 0;
   if (tid == 0) {
-    if (blockIdx.x == 0) *R.any = 0u;
+    if (blockIdx.x == 0 || grid.solo) *R.any = 0u;
     if (work && R.y == 0) *R.mine = 0u;
   }
   grid.sync();
@@ -369,7 +384,7 @@ struct TeamElem {
 // log T and log T2, h the dZ-weighted means of max(L, 0) and max(-L, 0).  out(k, log X pair,
 // log dZ pair, Z through k) is called for every sample of the block's range.
 template <bool OUT_LZ, typename Out>
-__device__ void team_evidence(cg::grid_group &grid, TeamRun &R, TeamSmem &sm, const int *nl, const double *ncoef,
+__device__ void team_evidence(const TeamSync &grid, TeamRun &R, TeamSmem &sm, const int *nl, const double *ncoef,
                               int nmax, double Loff, Out out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool work = R.Y > 0;
@@ -584,7 +599,7 @@ __global__ void __launch_bounds__(TEAM_T, 1) k_team_count_edges(const int *sende
                                                                 int *samples_indices, int *num_live,
                                                                 unsigned long long *scratch, int *deg) {
   __shared__ TeamSmem sm;
-  cg::grid_group grid = cg::this_grid();
+  const TeamSync grid = {false};
   TeamRun R;
   R.N = N;
   R.sender = sender;
@@ -607,7 +622,7 @@ __global__ void __launch_bounds__(TEAM_T, 1)
     k_team_evidence(const float *L, const int *nl, long long N, const double *ncoef, int nmax, gbns_evcalc *fin, double *lX,
                     double *ldZ, double *lZ, TeamTotals *tot) {
   __shared__ TeamSmem sm;
-  cg::grid_group grid = cg::this_grid();
+  const TeamSync grid = {false};
   TeamRun R;
   R.N = N;
   R.L = L;
@@ -637,10 +652,14 @@ __global__ void __launch_bounds__(TEAM_T, 1)
 __global__ void __launch_bounds__(TEAM_T, 1) k_team_results(gbns_batch b, gbns_results_bufs res, int per_run) {
   __shared__ TeamSmem sm;
   __shared__ long long s_evals, s_phantom;
-  cg::grid_group grid = cg::this_grid();
   const int tid = threadIdx.x;
   const int r = blockIdx.x / per_run;
   const bool mine = r < b.num_runs;
+  // short runs: a block each, without barriers between them
+  int longer = 0;
+  for (int q = tid; q < b.num_runs; q += TEAM_T) longer |= min(b.state[q].num_samples, b.runs[q].cap) >= TEAM_SOLO;
+  const TeamSync grid = {!__syncthreads_or(longer)};
+  if (grid.solo && (!mine || blockIdx.x % per_run > 0)) return;
   const gbns_run_desc &rd = b.runs[mine ? r : 0];
   const gbns_run_state &st = b.state[mine ? r : 0];
   const long long N = st.num_samples < rd.cap ? st.num_samples : rd.cap;
@@ -656,10 +675,10 @@ __global__ void __launch_bounds__(TEAM_T, 1) k_team_results(gbns_batch b, gbns_r
   R.deg = res.scratch_i + (so + r);
   R.si = res.samples_indices + so;
   R.nl = res.num_live_points + so;
-  R.any = (unsigned *)res.scalars;  // the scalars are written at the end
-  R.mine = (unsigned *)(sc + 1);
+  R.mine = (unsigned *)(sc + 1);    // the scalars are written at the end
+  R.any = grid.solo ? R.mine : (unsigned *)res.scalars;
   R.tot = team_totals(R.tmp);
-  team_split(R, blockIdx.x - r * per_run, per_run);
+  team_split(R, blockIdx.x - r * per_run, grid.solo ? 1 : per_run);
   if (!mine) R.Y = 0;
   const double off = rd.log_L_offset;
   double *Ls = res.log_L_samples + so, *lX = res.log_X_mean + so, *ldp = res.log_dp_mean + so;
