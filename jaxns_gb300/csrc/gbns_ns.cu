@@ -814,11 +814,18 @@ cudaError_t launch_merge(const gbns_batch &b, bool first, cudaStream_t stream) {
   // run with serial logarithms and a scan per set -> this form: one run of 240 live points 48.6 ->
   // 23, of 720 with 24 phantoms per chain 424 -> 30, of 1024 x 64 words (linear-Gaussian, P = 32)
   // 253 -> 33, twelve linear-Gaussian runs 932 -> 50; 1024 runs of 1000 points 283 -> 171.
+  // Beyond it, where shared memory leaves an SM three or two runs (more than 2048 points) and they do not
+  // all fit at once, 256 threads make up for the missing blocks: 600 runs of 3000 points 409 with 32 KB
+  // and serial logarithms, 478 with 128 threads, 285; 320 of 4096 424 / 551 / 340, 600 of them 496 / 589 /
+  // 362; 320 of 3000, which fit, 301 / 206 / 230.
   const int runs = b.num_runs;
   int threads = 128, blocks = 1;
   if (runs <= 2 * sms) {
     threads = max_n(b) <= 512 ? 256 : 512;
     blocks = sms / runs < 1 ? 1 : (sms / runs > 16 ? 16 : sms / runs);
+  } else if (max_n(b) > 2048) {
+    const long long per_sm = 228 * 1024 / ((long long)smem + 4096);  // (static and reserved shared memory)
+    if (runs > per_sm * sms) threads = 256;
   }
   // A run's blocks count themselves in its state's pad1, whatever a caller left there: zeroed before
   // the first merge of a call, and by every merge after itself.
