@@ -736,8 +736,8 @@ __global__ void __launch_bounds__(32 * PT_WARPS) k_prior_tiles(gbns_prior_table 
   }
 }
 
-// The same for D > 32 PT_E, where a row alone fills a warp's tile: one warp per row, dimensions
-// strided over the lanes.
+// The same for few rows, and for D > 32 PT_E, where a row alone fills a warp's tile: one warp per row,
+// dimensions strided over the lanes.
 template <typename UT>
 __global__ void __launch_bounds__(256) k_prior_transform(gbns_prior_table t, const UT *U, long long M,
                                                          const double *log_L, double *X, double *out) {
@@ -792,7 +792,13 @@ cudaError_t launch_prior_transform(const gbns_prior_table &t, const float *U32, 
   cudaError_t e;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if (t.D <= 32 * PT_E) {
+  // Tiles where there are enough of them: a warp takes its rows' elements one after the other (20 us), so
+  // few rows are done sooner with a warp each.  That kernel's time is flat up to a block of eight rows per
+  // SM and doubles with the second; us, a warp per row / tiles, D = 8 with a map: 100 rows 9.8 / 21, 1000
+  // 10.8 / 24, 2000 18.7 / 24, 4000 35 / 24; D = 20: 500 12 / 29, 2000 21 / 29, 4000 40 / 30; D = 40: 1000
+  // 24 / 34, 2000 42 / 34; D = 64: 1000 29 / 39, 2000 52 / 41; Normals without a map, D = 8: 100 9.3 / 19,
+  // 2000 16.5 / 20; D = 64: 100 16 / 20, 2000 31 / 22.
+  if (t.D <= 32 * PT_E && M > (t.D <= 32 ? 16ll : 8ll) * sms) {
     int GW = 32;
     while (GW / 2 >= t.D) GW /= 2;
     const int rows = t.D <= 32 ? PT_E * 32 / GW : PT_E / ((t.D + 31) / 32);
