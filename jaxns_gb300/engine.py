@@ -399,13 +399,11 @@ class NSBatch:
             Ns = np.array([s.N for s in specs], np.int64)
             row_base = np.concatenate([[0], np.cumsum(Ns)[:-1]]).astype(np.int64)
             rows = int(Ns.sum())
-            # work units (run, 128-chain tile, first 128-row tile, row tiles): row ranges sized so
-            # that there are about four units per CTA, an even number of tiles (the residual kernel
-            # multiplies two at a time); the chain tiles of one row range are adjacent, so the CTAs
-            # that share its Phi tiles run together
+            # work units (run, 128-chain tile, first 128-row tile, row tiles); the chain tiles of one
+            # row range are adjacent, so the CTAs that share its Phi tiles run together
             tiles = [((s.shell_size + 127) // 128, (s.N + 127) // 128) for s in specs]
-            work = sum(ct * rt for ct, rt in tiles)
-            rs = max(2, min(16, (work // (4 * 152) + 1) // 2 * 2))
+            sms = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 152
+            rs = residual_row_tiles(tiles, sms)
             items_tc = [(r, c0, rt0, min(rs, rt - rt0)) for r, (ct, rt) in enumerate(tiles)
                         for rt0 in range(0, rt, rs) for c0 in range(0, ct * 128, 128)]
             self.lg_tc_t = dict(W_hi=z(nc * 64), W_lo=z(nc * 64), Phi_hi=z(rows * 64), Phi_lo=z(rows * 64),
@@ -773,6 +771,21 @@ class NSBatch:
         words = torch.from_numpy(np.ascontiguousarray(np.asarray(U, dt).ravel()).view(np.float32))
         self.live_U[p][uo:uo + n * int(self.ucols[r])].copy_(words)
         self.live_L[p][o:o + n].copy_(torch.from_numpy(np.asarray(log_L, np.float32)))
+
+
+def residual_row_tiles(tiles, sms: int) -> int:
+    """Row tiles per work unit of the tensor-core residual kernel, one CTA per SM, for runs of the given
+    (chain tiles, row tiles).  A CTA's time is its units' (half a pair's for a unit's flags and first copies)
+    plus their pairs of row tiles (256 rows per MMA), so the range is the even one with the least of it on
+    the fullest CTA; single tiles while half of the SMs take them all.  us per step of a lock step, with
+    four units per CTA whatever that left on the fullest one / this rule (the 128-row MMAs of two CTAs
+    per SM before): 10 problems of 4096 x 20, 200 chains 20.3 / 19.1 (18.1); 8 of 8192 x 20, 300 chains 25.7 /
+    22.9 (23.2); 5 of 8192 x 48, 400 chains 29.8 / 26.4 (30.3); 4 of 4096 x 20 14.7 / 14.7 (14.1)."""
+    units = lambda rs: sum(ct * -(-rt // rs) for ct, rt in tiles)
+    if units(1) <= sms // 2:
+        return 1
+    longest = max(rt for _, rt in tiles)
+    return min(range(2, 17, 2), key=lambda rs: (-(-units(rs) // sms) * (0.5 + -(-min(rs, longest) // 2)), rs))
 
 
 def fused_plan(Ns, pmax: int, sizes=(16, 8)):
