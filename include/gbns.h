@@ -154,6 +154,9 @@ typedef struct {
     int num_runs;
     int nmax;                       /* largest n over runs (<= 4096) */
     int ncoef_n;                    /* largest count covered by the ncoef table */
+    int lane_chains;                /* chains that one shell runs at once on the thread-per-chain buckets' items:
+                                       per item its chains, at most chains_per_item, rounded up to 16.  0: not
+                                       known.  Chooses between kernels of the same results, nothing else */
     const gbns_run_desc *runs;      /* [R] */
     gbns_run_state *state;          /* [R] */
     float *live_U[2];               /* [sum n*D] */
@@ -190,6 +193,8 @@ typedef struct {
                                        normalised U-space gradient at its seed point, t in [0, right]
                                        (one extra evaluation per slice; every family, the linear-Gaussian
                                        family on its lock step) */
+    int warp_chains;                /* the same of buckets 2 and 3 (correlated Gaussians by warps): per item its
+                                       chains, at most 512 (bucket 2) or 256 (bucket 3) */
 } gbns_batch;
 
 /* Lock-step chain state of the linear-Gaussian family (device, caller-allocated).  Its

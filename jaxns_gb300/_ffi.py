@@ -52,7 +52,7 @@ class RunState(ctypes.Structure):
 
 
 class Batch(ctypes.Structure):
-    _fields_ = [("num_runs", c_int), ("nmax", c_int), ("ncoef_n", c_int), ("runs", c_void_p), ("state", c_void_p),
+    _fields_ = [("num_runs", c_int), ("nmax", c_int), ("ncoef_n", c_int), ("lane_chains", c_int), ("runs", c_void_p), ("state", c_void_p),
                 ("live_U", c_void_p * 2), ("live_L", c_void_p * 2), ("live_Lc", c_void_p * 2),
                 ("live_E", c_void_p * 2), ("live_S", c_void_p * 2),
                 ("new_U", c_void_p), ("new_L", c_void_p), ("new_E", c_void_p), ("ph_U", c_void_p),
@@ -61,7 +61,7 @@ class Batch(ctypes.Structure):
                 ("prior_a", c_void_p), ("prior_b", c_void_p), ("ncoef", c_void_p), ("items", c_void_p),
                 ("num_items", c_int), ("bucket_begin", c_int * 8), ("bucket_end", c_int * 8),
                 ("chains_per_item", c_int), ("max_evals_per_slice", c_int), ("gradient_guided", c_int),
-                ("gradient_slice", c_int)]
+                ("gradient_slice", c_int), ("warp_chains", c_int)]
 
 
 class LGBufs(ctypes.Structure):

@@ -16,6 +16,17 @@ enum : int {
   LG_HAVE_GRAD = 64      // the gradient launch has written the chain's gradient at its point
 };
 
+// Chains that work items [ib, ie) run at once: their share of what the host counted over the buckets of
+// their kind (wide: 2 and 3), or, without a count, as many as the items hold at the most.
+inline long long bucket_chains(const gbns_batch &b, bool wide, int ib, int ie, int per_item) {
+  const int counted = wide ? b.warp_chains : b.lane_chains;
+  long long items = 0;
+  for (int k = 0; k < 8; ++k)
+    if ((k == 2 || k == 3) == wide && b.bucket_end[k] > b.bucket_begin[k]) items += b.bucket_end[k] - b.bucket_begin[k];
+  if (counted <= 0 || items < ie - ib) return (long long)(ie - ib) * per_item;
+  return (long long)counted * (ie - ib) / items;
+}
+
 cudaError_t launch_slice_shells(const gbns_batch &b, const float *Lstar, const uint32_t *keys, cudaStream_t stream);
 cudaError_t launch_slice_warp(const gbns_batch &b, const float *Lstar, const uint32_t *keys, cudaStream_t stream);
 // The speculative sampler of small batches (gbns_slice_spec.cu) for the thread-per-chain bucket

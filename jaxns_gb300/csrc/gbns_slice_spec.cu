@@ -388,8 +388,9 @@ static cudaError_t launch_spec(const gbns_batch &b, int ib, int ie, const float 
 }
 
 // Lanes per chain for the thread-per-chain bucket [ib, ie), 0 when that kernel is the faster one.
-// An item holds at most chains_per_item chains per lane of its CTA, so items x chains_per_item
-// bounds the chains of the launch.  Measured on one GB300, us per shell of 5 D slices,
+// What counts is the chains at work at once: an item's chains beyond one per lane of its CTA come one
+// after the other on either kernel (80,000 chains of D = 10 shells, four per lane: 2,040 us here, 2,100
+// there; two per lane 1,060 / 1,200).  Measured on one GB300, us per shell of 5 D slices,
 // thread-per-chain against 32 (8 proposals x 4) / 8 / 4 lanes per chain:
 //   chains   MVN D = 8, Normal priors   shells D = 10             MVN D = 16
 //      120   602 | 62  106 137          541 |   66  70 107        1099 |  173 172 222   (150; 240)
@@ -397,15 +398,22 @@ static cudaError_t launch_spec(const gbns_batch &b, int ib, int ie, const float 
 //    5,760   633 | 422 263 205          564 |  431 176 158 (4,800)
 //   12,000   643 | 808 524 390          567 | 1211 469 410 (15,000) 1139 | 2891 842 616  (14,400)
 //   24,000   727 | 1544 989 757         659 |    - 1369 1090 (45,000)
+// and of 2 D slices, thread-per-chain against 8 / 4 lanes:
+//   chains   shells D = 20   D = 32             D = 40             D = 64
+//    5,000   664 | 335 273   1302 |  573  596   2096 | 1168 1000   4427 | 2161 2261
+//   10,000   671 | 591 450   1302 | 1018  983   2125 | 2115 1710   4498 | 3909 3751
+//   20,000   710 | 1107 794  1373 | 1913 1754   2459 | 4064 3137   4985 | 7485 6744
 // The thread-per-chain kernel's time hardly depends on the chain count until it fills the
-// GPU; this kernel's grows with it from the first wave on, so the line lies where they cross.
-constexpr long long SPEC_CHAINS_32 = 704, SPEC_CHAINS_8 = 3584, SPEC_CHAINS_4 = 20000;
-static int spec_lanes(const gbns_batch &b, int ib, int ie) {
-  const long long chains = (long long)(ie - ib) * b.chains_per_item;
+// GPU; this kernel's grows with it from the first wave on, so the line lies where they cross.  Beyond
+// D = 16 its registers (232, and 255 with spills) leave one CTA per SM, and the line lies lower.
+constexpr long long SPEC_CHAINS_32 = 704, SPEC_CHAINS_8 = 3584;
+constexpr long long spec_chains_4(int dmax) { return dmax <= 16 ? 20000 : (dmax == 32 ? 15000 : 12500); }
+static int spec_lanes(const gbns_batch &b, int dmax, int ib, int ie) {
   if (b.gradient_guided || b.gradient_slice) return 0;
+  const long long chains = bucket_chains(b, false, ib, ie, b.chains_per_item);
   if (chains <= SPEC_CHAINS_32) return 32;
   if (chains <= SPEC_CHAINS_8) return 8;
-  if (chains <= SPEC_CHAINS_4) return 4;
+  if (chains <= spec_chains_4(dmax)) return 4;
   return 0;
 }
 
@@ -419,7 +427,7 @@ static cudaError_t launch_lanes(int lanes, const gbns_batch &b, int ib, int ie, 
 
 cudaError_t launch_slice_spec(const gbns_batch &b, int family, int dmax, int ib, int ie, const float *Lstar,
                               const uint32_t *keys, cudaStream_t stream, bool &taken) {
-  const int lanes = spec_lanes(b, ib, ie);
+  const int lanes = spec_lanes(b, dmax, ib, ie);
   taken = lanes != 0;
   if (!taken) return cudaSuccess;
   if (family == GBNS_LIK_MVN) {

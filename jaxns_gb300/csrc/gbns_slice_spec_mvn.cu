@@ -377,24 +377,28 @@ static cudaError_t launch_spec_mvn(const gbns_batch &b, int ib, int ie, int per_
 }
 
 // Proposals per round of a chain for the warp-cooperative bucket [ib, ie), 0 when that kernel is
-// the faster one.  An item holds up to 512 (D <= 32) or 256 chains of one run unless the caller
-// chose another size, which changes neither the results nor this kernel's coverage (it strides
-// over an item's chains).  Measured on one GB300, us per shell of 5 D slices, warp-cooperative
-// against 16 / 8 / 4 proposals per round:
-//   chains   D = 24                          chains   D = 48
-//      360   2719 |  248  275  372              720    7394 |   993 1096  1381
-//    1,440   2875 |  503  304  396            2,880    7439 |  3984 2463  1506
-//    5,760   2993 | 1325  917  844            5,760    7468 |  7126 4507  3196
-//   11,520   3027 | 2598 1623 1330           11,520    7532 | 13018 8183  5755
-//   23,040   3055 | 5041 3192 2348           23,040    7560 | 25624 15084 10204
+// the faster one, by the chains at work at once (an item's size changes neither the results nor this
+// kernel's coverage: it strides over an item's chains).  Measured on one GB300, us per shell of
+// 5 D slices, 16 / 8 / 4 proposals per round:
+//   chains   D = 24                  chains   D = 48
+//      360   248  275  372              720    993 1096  1381
+//    1,440   503  304  396            2,880   3984 2463  1506
+//    5,760  1325  917  844            5,760   7126 4507  3196
+// and of 2 D slices, warp-cooperative against 8 / 4 proposals (runs of 400 live points):
+//   chains   D = 20             D = 32             D = 40             D = 48             D = 64
+//   12,000   747 |  598  449   1592 | 1066  783   2195 | 2573 1871   3025 | 3257 2355   4915 | 4861 3391
+//   15,000   749 |  770  583   1600 | 1389 1032   2183 | 3274 2317   2996 | 4149 2906   4874 | 6192 4210
+//   20,000   766 |  990  740   1571 | 1792 1312   2206 | 4070 2823   3005 | 5200 3560   4874 | 7776 5133
+//   29,000   787 | 1388 1003   1594 | 2513 1746   2215 | 5896 3835   3015 | 7522 4824   4888 | 11255 7078
 // (A trip's loads of the proposals before its stores: 283 -> 248 and 1159 -> 993 us for one run.)
-// The warp-cooperative kernel stays at its latency until its CTAs fill the SMs (~39 k chains at
-// D > 32); this kernel's time grows with the chains beyond one wave of CTAs.
+// The warp-cooperative kernel stays at its latency until its CTAs fill the SMs; this kernel's time
+// grows with the chains beyond one wave of CTAs.  (Many small runs, an item each, fill fewer lanes
+// there: 400 runs of 30 chains, 12,000, D = 24 2203 | 555, D = 48 7058 | 2332.)
 static int spec_mvn_lanes(const gbns_batch &b, int dmax, long long chains) {
   if (b.gradient_guided || b.gradient_slice) return 0;
   if (chains <= 1024) return 16;
   if (chains <= (dmax > 32 ? 1536 : 2048)) return 8;
-  if (chains <= (dmax > 32 ? 15000 : 29000)) return 4;
+  if (chains <= (dmax > 32 ? 14000 : 22000)) return 4;
   return 0;
 }
 
@@ -411,7 +415,7 @@ cudaError_t launch_slice_spec_mvn(const gbns_batch &b, int dmax, int ib, int ie,
   taken = false;
   if (ie <= ib) return cudaSuccess;
   const int per_item = b.nmax < (dmax > 32 ? 256 : 512) ? b.nmax : (dmax > 32 ? 256 : 512);
-  const int lanes = spec_mvn_lanes(b, dmax, (long long)(ie - ib) * per_item);
+  const int lanes = spec_mvn_lanes(b, dmax, bucket_chains(b, true, ib, ie, per_item));
   taken = lanes != 0;
   if (!taken) return cudaSuccess;
   if (dmax == 32) return launch_dmax<32>(lanes, b, ib, ie, per_item, Lstar, keys, stream);

@@ -330,6 +330,9 @@ class NSBatch:
         b.max_evals_per_slice = int(max_evals_per_slice)
         b.gradient_guided = int(self.gradient_guided)
         b.gradient_slice = int(self.gradient_slice)
+        # chains at work at once, from which the launcher chooses the sampler
+        b.lane_chains = sum(-(-min(it[4], CH) // 16) * 16 for it in items if it[0] not in (2, 3))
+        b.warp_chains = sum(min(it[4], 512 if it[0] == 2 else 256) for it in items if it[0] in (2, 3))
         self._b = b
         self._lgb = self._alloc_lg(specs, ss, Ds, shell_off, lg_tensor_cores) if self.lg else None
         self._graphs: Dict[tuple, tuple] = {}
