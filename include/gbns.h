@@ -228,8 +228,7 @@ typedef struct {
     float *Phi_hi, *Phi_lo;                 /* [total_rows * 64] */
     const long long *row_base;              /* [R] first row of each run in Phi_hi / Phi_lo */
     long long total_rows;                   /* sum of N over the runs */
-    int num_ctas_tc;                        /* cap on the persistent grid; 0 = one CTA per SM (two when
-                                               every P <= 32) */
+    int num_ctas_tc;                        /* cap on the persistent grid; 0 = one CTA per SM */
     int num_tiles;                          /* 128-chain tiles over all runs */
     const int *chain_run;                   /* [total_chains] run of each chain */
     const int *tile_base;                   /* [R] first 128-chain tile of each run */

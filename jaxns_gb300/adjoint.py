@@ -109,7 +109,7 @@ def batch_evidence_and_grad(batch, results, thetas, tensor_cores: bool = True, c
             _ffi.call("gbns_evidence_adjoint_tc", *args, p(ws), p(ps), p(status), stream)
         else:
             _ffi.call("gbns_evidence_adjoint", *args, stream)
-        batch.kernel_launches += 5 if tensor_cores else 2
+        batch.kernel_launches += (4 if M >= 256 else 3) if tensor_cores else 2
     if check and tensor_cores and int(status.item()) != 0:
         raise _ffi.GBNSError(f"gbns_evidence_adjoint_tc: device status {int(status.item())} (wait timed out)")
     return out

@@ -201,12 +201,6 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-__device__ __forceinline__ float warp_maxf(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // ------------------------------------------------------- CTA reductions ----
 
 template <typename T>
@@ -230,35 +224,11 @@ __device__ T cta_sum(T v, T *red) {
 __device__ __forceinline__ long long cta_sum_ll(long long v, long long *red) { return cta_sum(v, red); }
 __device__ __forceinline__ double cta_sum_d(double v, double *red) { return cta_sum(v, red); }
 
-__device__ __forceinline__ float cta_max_f(float v, float *red) {
-  v = warp_maxf(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float r = -INFINITY;
-  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) r = fmaxf(r, red[q]);
-  __syncthreads();
-  return r;
-}
-
-__device__ __forceinline__ int cta_and(int v, int *red) {
-  v = __all_sync(0xffffffffu, v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  int r = 1;
-  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) r &= red[q];
-  __syncthreads();
-  return r;
-}
-
 // ----------------------------------------------------- FP64 evidence scan ----
 //
 // The recurrence of _update_evidence_calc_op (internals/shrinkage_statistics.py:43-94),
 // rewritten as prefix sums so that a whole CTA processes blockDim elements per step:
-//   X_k  = X_{k-1} T_k,            X2_k = X2_{k-1} T2_k                 (FP64 log-space prefix sums)
+//   X_k  = X_{k-1} T_k,            X2_k = X2_{k-1} T2_k                 (log-space prefix sums)
 //   dZ_k = X_{k-1} t_k mid_k,      Z_k  = Z_{k-1} + dZ_k
 //   A_k  = ZX_k / X_k = A_{k-1} + X2_{k-1} tT_k mid_k / X_k              (an exclusive prefix sum)
 //   Z2_k = Z2_{k-1} + 2 X_{k-1} A_{k-1} t_k mid_k + X2_{k-1} t2_k mid_k^2
@@ -268,7 +238,7 @@ __device__ __forceinline__ int cta_and(int v, int *red) {
 // others.  Inside a chunk of blockDim elements the terms and their sums are fp32 pairs (FS,
 // below); the accumulators carried from chunk to chunk are FP64 mantissas (ScaledSum), both
 // rescaled exactly by powers of two.  Z, Z2 and dZ2 are accumulated per thread and reduced
-// once at the end; log X and log X2 (FP64) and A are CTA scans with carries between chunks.
+// once at the end; log X, log X2 and A are CTA scans with FP64 carries between chunks.
 // Coefficients per n come from an FP64 table built on the host with the reference formulas.
 
 struct ScaledSum {
@@ -346,14 +316,6 @@ __device__ __forceinline__ EvAcc evacc_from(const gbns_evcalc &e) {
   return a;
 }
 
-// As evacc_from for a register whose log_L is absolute while the scanned values are
-// relative to Loff.
-__device__ __forceinline__ EvAcc evacc_from_shifted(const gbns_evcalc &e, double Loff) {
-  EvAcc a = evacc_from(e);
-  a.Lprev = (float)(e.log_L - Loff);
-  return a;
-}
-
 __device__ __forceinline__ gbns_evcalc evacc_to(const EvAcc &a, double log_L_last) {
   gbns_evcalc e;
   e.log_L = log_L_last;
@@ -379,11 +341,12 @@ __device__ __forceinline__ void ncoef_compute(double n, double *c) {
 }
 
 // ---- fp32-pair scaled sums.  GB300 runs FP64 at about 1/64 of the FP32 rate, so inside a
-// scan only the log-X prefix (which must stay within 1e-12 of the reference's FP64 values) is
-// FP64; every exponential term and every sum of terms is an fp32 pair (h + l) 2^e: TwoSum
-// additions (relative error a few units of 2^-48), exponents aligned by exact powers of two.
-// The terms themselves carry fp32 mantissas (exp2f of a pair-accurate fraction), as the FP64
-// scaled sums do.  Chunk totals are folded into the FP64 accumulators once per chunk.
+// scan everything is an fp32 pair: log X (h + l), and every exponential term and sum of terms
+// (h + l) 2^e, by TwoSum additions (relative error a few units of 2^-48), exponents aligned by exact
+// powers of two.  The terms themselves carry fp32 mantissas (exp2f of a pair-accurate fraction), as the
+// FP64 scaled sums do.  Chunk totals, log X's among them, are folded into FP64 accumulators once per
+// chunk, and log X in a chunk is the carried value plus the sum inside it, so it stays within 1e-12 of
+// the reference's FP64 values.
 struct FS {
   float h, l;
   int e;  // value = (h + l) 2^e, h == 0 means zero
@@ -526,20 +489,6 @@ __device__ __forceinline__ FS shfl_xor_fs(FS v, int o) {
   return r;
 }
 
-// natural log of a (> 0) as an fp32 pair, to fp32 accuracy of the mantissa's log
-__device__ __forceinline__ void fs_log_pair(FS a, float &lh, float &ll) {
-  if (!(a.h > 0.0f)) {
-    lh = -INFINITY;
-    ll = 0.0f;
-    return;
-  }
-  const float ln2_hi = 0.693147182464599609375f, ln2_lo = -1.904654323148236017e-9f;
-  const float ef = (float)a.e;
-  const float ph = ef * ln2_hi;
-  const float pe = fmaf(ef, ln2_hi, -ph) + ef * ln2_lo;
-  pair_sum2(ph, pe, logf(a.h) + a.l / a.h, 0.0f, lh, ll);
-}
-
 __device__ __forceinline__ FS fs_from_ss(ScaledSum s) {
   FS r;
   if (!(s.q > 0.0)) return fs_zero();
@@ -672,8 +621,7 @@ __device__ __forceinline__ void ncoef_pairs(const double *__restrict__ ncoef, in
   }
 }
 
-// Process elements [0, M) of log-likelihoods L (fp32) with live-point counts given by
-// nmode: nconst > 0 -> n_k = nconst; ndesc > 0 -> n_k = ndesc - k; else n_k = narr[k].
+// Process elements [0, M) of log-likelihoods L (fp32) with live-point counts narr.
 // Called by every thread of the CTA (blockDim a multiple of 32), each holding the same acc.
 // Optional per-element outputs (FP64 logs): log X, log dZ and, with OUT_LZ, the running log Z.
 // L values are relative to Loff (added back in FP64); Lidx, when given, gathers L[Lidx[k]].
@@ -686,7 +634,7 @@ __device__ __forceinline__ void ncoef_pairs(const double *__restrict__ ncoef, in
 // scan's samples sum dZ max(L, 0) / sum dZ and sum dZ max(-L, 0) / sum dZ (L relative to
 // Loff), for H.
 template <bool OUT_LZ, int K = 1>
-__device__ void evidence_scan_cta(EvAcc &acc, const float *__restrict__ L, long long M, int nconst, int ndesc,
+__device__ void evidence_scan_cta(EvAcc &acc, const float *__restrict__ L, long long M,
                                   const int *__restrict__ narr, const double *__restrict__ ncoef, int nmax,
                                   double *__restrict__ out_lX, double *__restrict__ out_ldZ,
                                   double *__restrict__ out_lZ, double Loff, const int *__restrict__ Lidx,
@@ -721,8 +669,7 @@ __device__ void evidence_scan_cta(EvAcc &acc, const float *__restrict__ L, long 
       const bool valid = k < M;
       Lk[j] = valid ? L[Lidx ? Lidx[k] : k] : 0.0f;
       if (j == 0) Lfirst_m1 = !valid ? 0.0f : (k == 0 ? acc.Lprev : L[Lidx ? Lidx[k - 1] : k - 1]);
-      int n = 1;
-      if (valid) n = nconst > 0 ? nconst : (ndesc > 0 ? (int)(ndesc - k) : narr[k]);
+      const int n = valid ? narr[k] : 1;
       nk[j] = n < 0 ? 0 : n;
     }
 #pragma unroll

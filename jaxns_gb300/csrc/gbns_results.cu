@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(RESULTS_EV_THREADS)
   e.log_L = -INFINITY; e.log_X_mean = 0.0; e.log_X2_mean = 0.0; e.log_Z_mean = -INFINITY;
   e.log_ZX_mean = -INFINITY; e.log_Z2_mean = -INFINITY; e.log_dZ_mean = -INFINITY; e.log_dZ2_mean = -INFINITY;
   EvAcc acc = evacc_from(e);
-  evidence_scan_cta<OUT_LZ, RESULTS_K>(acc, L, N, 0, 0, nl, ncoef, nmax, lX, ldZ, lZ, 0.0, nullptr, esm);
+  evidence_scan_cta<OUT_LZ, RESULTS_K>(acc, L, N, nl, ncoef, nmax, lX, ldZ, lZ, 0.0, nullptr, esm);
   if (threadIdx.x == 0) *fin = evacc_to(acc, N > 0 ? (double)L[N - 1] : -INFINITY);
 }
 
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(RESULTS_EV_THREADS) k_results_ev(gbns_batch b,
     e.log_L = -INFINITY; e.log_X_mean = 0.0; e.log_X2_mean = 0.0; e.log_Z_mean = -INFINITY;
     e.log_ZX_mean = -INFINITY; e.log_Z2_mean = -INFINITY; e.log_dZ_mean = -INFINITY; e.log_dZ2_mean = -INFINITY;
     EvAcc acc = evacc_from(e);
-    evidence_scan_cta<false, K>(acc, b.store_L + so, N, 0, 0, nl, b.ncoef, b.ncoef_n, lX, ldp, nullptr, off,
+    evidence_scan_cta<false, K>(acc, b.store_L + so, N, nl, b.ncoef, b.ncoef_n, lX, ldp, nullptr, off,
                                 gathered ? si : nullptr, esm, s_h);
     if (threadIdx.x == 0) {
       const gbns_evcalc f = evacc_to(acc, 0.0);
