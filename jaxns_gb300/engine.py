@@ -778,17 +778,21 @@ class NSBatch:
 
 def residual_row_tiles(tiles, sms: int) -> int:
     """Row tiles per work unit of the tensor-core residual kernel, one CTA per SM, for runs of the given
-    (chain tiles, row tiles).  A CTA's time is its units' (half a pair's for a unit's flags and first copies)
-    plus their pairs of row tiles (256 rows per MMA), so the range is the even one with the least of it on
-    the fullest CTA; single tiles while half of the SMs take them all.  us per step of a lock step, with
-    four units per CTA whatever that left on the fullest one / this rule (the 128-row MMAs of two CTAs
-    per SM before): 10 problems of 4096 x 20, 200 chains 20.3 / 19.1 (18.1); 8 of 8192 x 20, 300 chains 25.7 /
-    22.9 (23.2); 5 of 8192 x 48, 400 chains 29.8 / 26.4 (30.3); 4 of 4096 x 20 14.7 / 14.7 (14.1)."""
+    (chain tiles, row tiles): single tiles while half of the SMs take them all; else an even number (256
+    rows per MMA) that leaves about four units per CTA, which still spread when chain tiles finish, unless
+    another leaves a twelfth less on the fullest CTA.  A CTA's time is its units' (half a pair's for a
+    unit's flags and first copies) plus their pairs of row tiles.  us per step of a lock step, with four
+    units per CTA always / this rule (the 128-row MMAs of two CTAs per SM before): 10 problems of 4096 x 20,
+    200 chains 20.3 / 19.1 (18.1); 8 of 8192 x 20, 300 chains 25.7 / 22.9 (23.2); 5 of 8192 x 48, 400 chains
+    29.8 / 26.4 (30.3); one of 1000 x 32 13.9 / 13.3 (13.5); 4 of 4096 x 20 14.7 / 14.7 (14.1)."""
     units = lambda rs: sum(ct * -(-rt // rs) for ct, rt in tiles)
     if units(1) <= sms // 2:
         return 1
     longest = max(rt for _, rt in tiles)
-    return min(range(2, 17, 2), key=lambda rs: (-(-units(rs) // sms) * (0.5 + -(-min(rs, longest) // 2)), rs))
+    load = lambda rs: -(-units(rs) // sms) * (0.5 + -(-min(rs, longest) // 2))
+    four = max(2, min(16, (units(1) // (4 * sms) + 1) // 2 * 2))
+    best = min(range(2, 17, 2), key=lambda rs: (load(rs), rs))
+    return best if 12 * load(best) <= 11 * load(four) else four
 
 
 def fused_plan(Ns, pmax: int, sizes=(16, 8)):
