@@ -964,11 +964,11 @@ __global__ void __launch_bounds__(THREADS, PER_SM) k_lg_shell_fused(const __grid
 // by TMA, warp 1 issues the 3xTF32 MMAs into two 256-column accumulators in turn, warps 2-5 and
 // 6-9 drain a column half each (thread = point): per 32 rows one fp32 chain for each sum, then FP64
 // registers, added to the point's totals when the point tile changes.  (A sum of squares beyond fp32 is
-// infinite and the point's weight zero; fp32 pairs for the four chunks of a tile, 8 us less, made it NaN.)
+// infinite and the point's weight zero; fp32 pairs for the four chunks of a tile, 7 us less, made it NaN.)
 // Bound: the tensor pipe.  256 rows per MMA are what reaches it: 12 MMAs of 128 x 256 x 8 take
 // 1.66 k cycles, of 128 x 128 x 8 2.25 k for half the work (the 128-point operand is read again
 // for every one).  40,000 points x 4096 rows x 32: one tile per CTA (5,008 CTAs, copy, MMAs and
-// epilogue in turn) 119 us, persistent with 128-row MMAs 96 us, this 58 us (the MMAs alone: 29 us).
+// epilogue in turn) 119 us, persistent with 128-row MMAs 96 us, this 65 us (the MMAs alone: 29 us).
 struct AdjStages {
   int nkb;      // K blocks of 32 floats
   int w_bufs;   // W tiles in shared memory (2 at one K block, 1 at two)
