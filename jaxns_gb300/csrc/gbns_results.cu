@@ -903,7 +903,8 @@ cudaError_t launch_results(const gbns_batch &b, const gbns_results_bufs &res, cu
 // the team pays its grid barriers whatever the size, one block its passes.  Live-point counts and
 // evidence through the package, us (one block / team), in order and with phantoms out of order:
 // 1000 samples 67 / 69, 67 / 81; 2000 67 / 70, 80 / 83; 4000 76 / 70, 241 / 156; 8000 115 / 72,
-// 335 / 134; 16000 197 / 70, 720 / 174.
+// 335 / 134; 16000 197 / 70, 720 / 174.  (The count alone, on the device, in order / out of order: 3000
+// samples 6.1 / 39 and 9.9 / 34, 6000 9.6 / 66 and 10.4 / 35, 8000 11.1 / 84 and 10.2 / 36.)
 constexpr long long TEAM_MIN_SAMPLES = 3000;
 
 cudaError_t launch_count_crossed_edges(const int *sender, const float *L, long long N, int *samples_indices,
