@@ -408,8 +408,16 @@ __device__ void team_evidence(const TeamSync &grid, TeamRun &R, TeamSmem &sm, co
     ah = sh; al = sl; bh = s2h; bl = s2l;
     float4 t;  // (the total as a pair is not used)
     cta_scan_p2(ah, al, bh, bl, t, sm.ev.pair);
-    pair_sum2(ah, al, -sh, -sl, ah, al);
-    pair_sum2(bh, bl, -s2h, -s2l, bh, bl);
+    // the sums of the threads before, not this one's taken off again: a count of 0 (log T = -inf) leaves
+    // the samples before it in its thread alone
+    ah = __shfl_up_sync(0xffffffffu, ah, 1);
+    al = __shfl_up_sync(0xffffffffu, al, 1);
+    bh = __shfl_up_sync(0xffffffffu, bh, 1);
+    bl = __shfl_up_sync(0xffffffffu, bl, 1);
+    if (lane == 0) {
+      const float4 w = warp > 0 ? sm.ev.pair.w[warp - 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+      ah = w.x; al = w.y; bh = w.z; bl = w.w;
+    }
     if (warp == 0) {
       // the block's total in FP64 from the warps' sums: log T in even lanes, log T2 in odd ones
       const float2 *w = reinterpret_cast<const float2 *>(sm.ev.pair.own);

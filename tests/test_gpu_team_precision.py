@@ -32,3 +32,21 @@ def test_register_log_X_is_fp64(gpu_lib, live):
     for got, k in ((final[1], 0), (final[2], 4)):  # log X, log X2
         exact = N * (Fraction(float(pairs[k])) + Fraction(float(pairs[k + 1])))
         assert abs((Fraction(float(got)) - exact) / exact) <= 22 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("N,at", [(3000, 2999), (3001, 3000), (3001, 1500), (20000, 19999), (300001, 300000), (300001, 77777)])
+def test_a_count_of_zero_leaves_the_samples_before_it(gpu_lib, N, at):
+    """X is 0 after a sample with no live point; log X before it is what it is without it."""
+    from jaxns_gb300 import _ffi
+    from jaxns_gb300.engine import ncoef_table
+    dev = lambda x: torch.as_tensor(x, device="cuda")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    n = np.random.default_rng(N).integers(1, 60, N).astype(np.int32)
+    n[at] = 0
+    tL, tn, tab = dev(np.sort(np.random.default_rng(at).standard_normal(N)).astype(np.float32)), dev(n), dev(ncoef_table(64))
+    fin, lX, ldZ = (torch.empty(k, dtype=torch.float64, device="cuda") for k in (8, N, N))
+    _ffi.call("gbns_evidence_stats", p(tL), p(tn), ctypes.c_longlong(N), p(tab), ctypes.c_int(64), p(fin), p(lX), p(ldZ),
+              ctypes.c_void_p(0), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    ref = np.cumsum(-np.log1p(1.0 / n[:at].astype(np.longdouble))).astype(np.float64)
+    np.testing.assert_allclose(lX.cpu().numpy()[:at], ref, rtol=1e-12, atol=1e-12)
+    assert np.isfinite(ldZ.cpu().numpy()[:at]).all()
